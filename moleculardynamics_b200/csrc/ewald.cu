@@ -8,14 +8,13 @@
 //   self         -C alpha/sqrt(pi) sum q^2;
 //   intra        -C q_i q_j erf(alpha r)/r over same-molecule pairs (min image),
 //                from per-atom partner lists built once from the molecule ids;
-//   reciprocal   S(k) = sum_j q_j exp(i k.r_j) over the half space of k vectors
-//                (S(-k) = conj S(k), so energy and force sums double), with the
-//                per-axis factors exp(i n a x) built by complex recurrence.
+//   reciprocal   sum_j q_j of the eight cos/sin products per k vector of one octant,
+//                which together hold S(k) = sum_j q_j exp(i k.r_j) for every sign of
+//                k's components, with the per-axis factors built by recurrence.
 // The SPC/E force field adds O-O Lennard-Jones (oxygens = atoms with original
 // index divisible by 3, as SpceForceField::gatherOxygens takes them) in the same
 // pass over the real-space list.
 #include <algorithm>
-#include <climits>
 #include <cmath>
 #include <new>
 #include <unordered_map>
@@ -262,199 +261,245 @@ __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
+// Reciprocal sums in separable real form.  With a, b, c each cos or sin,
+//   A_abc(nx, ny, nz) = sum_j q_j a(nx kx0 x_j) b(ny ky0 y_j) c(nz kz0 z_j),  n >= 0,
+// the eight sums of an octant vector carry every sign combination of (nx, ny, nz) at
+// once: the coefficient f depends on |k| alone, and summing cos(k.(r_i - r_j)) over the
+// signs leaves g(nx) g(ny) g(nz) times a product of three cosines (g(0) = 1, else 2), so
+//   E = sum_octant f g g g sum_abc A_abc^2,
+//   dE/dq(r) = U(r) = sum_octant 2 f g g g sum_abc A_abc a(x) b(y) c(z),  F = -q grad U.
+// That is two multiply-adds per site and k vector for A and four for grad U, against
+// about ten and sixteen with one complex exponential per vector.  A task is one (nx, ny)
+// column of kColZ consecutive nz: a thread's register tile.
+constexpr int kColZ = 4;            // nz per task
+constexpr int kColSums = 8 * kColZ; // sums A_abc per task
+constexpr int kTaskChunk = 32;      // tasks with one nz0, padded to whole warps
+constexpr int kSumBlock = 128;
+
 struct KArgs {
-    const double4* kvec;  // kx, ky, kz, factor
-    const int4* kn;       // nx, ny, nz
-    int nk, kmax;
-    double a, b, c;       // 2 pi / L per axis
+    const int4* task;   // nx, ny, nz0, 1 (0: padding)
+    const double2* fac; // per task and nz: f g g g (0 outside the sphere), k^2
+    int ntask, kmax;
+    double a, b, c;     // 2 pi / L per axis
 };
 
 constexpr int kSiteTile = 32;
 
-// S(k) partial sums: block (kb, sb) handles k vectors [kb*256, +256) against the
-// sites of slice sb; per-site factor tables X[nx], Y[ny], Z[nz] of a tile of sites
-// are built in shared memory by complex recurrence.
-__global__ void __launch_bounds__(kBlock)
+// Entries per axis of a site's factor table: nz0 + kColZ may pass kmax.
+__host__ __device__ constexpr int table_axis(int kmax) { return (kmax / kColZ + 1) * kColZ; }
+
+// Partial sums A_abc: block (tb, sb) takes tasks [tb * 128, +128) over the sites of slice
+// sb, one task per thread, 32 sums in registers.  Per tile of 32 sites the factors
+// e^{i m theta} of each axis (the charge folded into x) are built in shared memory by
+// complex recurrence; a site then costs a thread four products, 32 multiply-adds and six
+// 16-byte shared loads, four of them broadcasts (one nz0 per warp), so the FP64 pipe
+// bounds the kernel (a register-operand outer product of this shape reaches 47 of its 64
+// multiply-adds per clock and SM here).  12,288 sites, kmax 18 (12.2k half-space
+// vectors): 268 us with one complex product chain per vector, 48 us in this form.
+__global__ void __launch_bounds__(kSumBlock)
 k_structure_factor(const double4* __restrict__ pos, const double* __restrict__ q, int64_t n,
-                   KArgs ka, int64_t sites_per_slice, double2* part) {
-    extern __shared__ double2 tab[];  // kSiteTile * (kmax+1 + 2*(2kmax+1))
-    const int nX = ka.kmax + 1, nY = 2 * ka.kmax + 1;
-    const int per = nX + 2 * nY;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int4 kn = k < ka.nk ? ka.kn[k] : make_int4(0, 0, 0, 0);
+                   KArgs ka, int64_t sites_per_slice, double* __restrict__ part) {
+    extern __shared__ double2 tab[];  // 3 axes x table_axis(kmax) x (kSiteTile + 1)
+    constexpr int kPad = kSiteTile + 1;  // consecutive m on different banks
+    const int nT = table_axis(ka.kmax);
+    const int t = blockIdx.x * kSumBlock + threadIdx.x;
+    const int4 tk = t < ka.ntask ? __ldg(ka.task + t) : make_int4(0, 0, 0, 0);
+    const double2* X = tab + tk.x * kPad;
+    const double2* Y = tab + (nT + tk.y) * kPad;
+    const double2* Z = tab + (2 * nT + tk.z) * kPad;
     const int64_t s0 = blockIdx.y * sites_per_slice;
     const int64_t s1 = min(n, s0 + sites_per_slice);
-    double re = 0.0, im = 0.0;
+    double acc[kColZ][8];
+#pragma unroll
+    for (int z = 0; z < kColZ; ++z)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[z][j] = 0.0;
     for (int64_t base = s0; base < s1; base += kSiteTile) {
         __syncthreads();
-        // build tables: thread t builds site (t % tile), one axis per 3 groups
-        for (int w = threadIdx.x; w < 3 * kSiteTile; w += blockDim.x) {
+        for (int w = threadIdx.x; w < 3 * kSiteTile; w += kSumBlock) {
             const int site = w % kSiteTile, axis = w / kSiteTile;
-            const int64_t sidx = base + site;
-            double2* T = tab + site * per;
-            if (sidx < s1) {
-                const double4 p = pos[sidx];
+            const int64_t s = base + site;
+            double2* T = tab + axis * nT * kPad + site;
+            double2 v = make_double2(0.0, 0.0), e1 = v;
+            if (s < s1) {
+                const double4 p = pos[s];
                 const double coord = axis == 0 ? p.x : (axis == 1 ? p.y : p.z);
-                const double kk = axis == 0 ? ka.a : (axis == 1 ? ka.b : ka.c);
-                double sn, cs;
-                sincos(kk * coord, &sn, &cs);
-                const double2 e1 = make_double2(cs, sn);
-                if (axis == 0) {
-                    double2 x = make_double2(1.0, 0.0);
-                    for (int m = 0; m < nX; ++m) {
-                        T[m] = x;
-                        x = cmul(x, e1);
-                    }
-                } else {
-                    double2* Y = T + nX + (axis - 1) * nY;
-                    double2 y = make_double2(1.0, 0.0);
-                    for (int m = 0; m <= ka.kmax; ++m) {
-                        Y[ka.kmax + m] = y;
-                        Y[ka.kmax - m] = make_double2(y.x, -y.y);
-                        y = cmul(y, e1);
-                    }
-                }
-            } else {
-                for (int m = 0; m < (axis == 0 ? nX : nY); ++m)
-                    (axis == 0 ? T : T + nX + (axis - 1) * nY)[m] = make_double2(0.0, 0.0);
+                sincos((axis == 0 ? ka.a : (axis == 1 ? ka.b : ka.c)) * coord, &e1.y, &e1.x);
+                v.x = axis == 0 ? q[s] : 1.0;
+            }
+            for (int m = 0; m < nT; ++m) {
+                T[m * kPad] = v;
+                v = cmul(v, e1);
             }
         }
         __syncthreads();
-        const int lim = static_cast<int>(s1 - base < kSiteTile ? s1 - base : kSiteTile);
-        if (k < ka.nk) {
-            for (int site = 0; site < lim; ++site) {
-                const double2* T = tab + site * per;
-                const double2 e = cmul(cmul(T[kn.x], T[nX + ka.kmax + kn.y]),
-                                       T[nX + nY + ka.kmax + kn.z]);
-                const double qs = q[base + site];
-                re = fma(qs, e.x, re);
-                im = fma(qs, e.y, im);
+#pragma unroll 2
+        for (int site = 0; site < kSiteTile; ++site) {
+            const double2 x = X[site], y = Y[site];
+            const double xy[4] = {x.x * y.x, x.x * y.y, x.y * y.x, x.y * y.y};
+#pragma unroll
+            for (int z = 0; z < kColZ; ++z) {
+                const double2 zz = Z[z * kPad + site];
+#pragma unroll
+                for (int ab = 0; ab < 4; ++ab) {
+                    acc[z][2 * ab] = fma(xy[ab], zz.x, acc[z][2 * ab]);
+                    acc[z][2 * ab + 1] = fma(xy[ab], zz.y, acc[z][2 * ab + 1]);
+                }
             }
         }
     }
-    if (k < ka.nk) part[static_cast<int64_t>(blockIdx.y) * ka.nk + k] = make_double2(re, im);
+    if (t >= ka.ntask) return;
+    double* o = part + static_cast<int64_t>(blockIdx.y) * kColSums * ka.ntask + t;
+#pragma unroll
+    for (int z = 0; z < kColZ; ++z)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[static_cast<int64_t>(8 * z + j) * ka.ntask] = acc[z][j];
 }
 
-// Sums the partials (slice order), stores S(k) and reduces the reciprocal energy
-// and virial: E = sum_half 2 factor |S|^2, W = sum_half 2 factor |S|^2 (1 - k^2/(2 a^2)).
-__global__ void k_structure_final(const double2* __restrict__ part, int slices, KArgs ka,
-                                  double inv_2alpha2, double2* sk, double* rpart,
-                                  unsigned* ticket, double* out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Adds the slices (eight groups of lanes, group g slices g, g + 8, ... in order, then the
+// groups in order), reduces the reciprocal energy and virial, W = sum E(k)
+// (1 - k^2 / (2 a^2)), and leaves the coefficients 2 f g g g A_abc of U, eight per
+// octant vector.
+constexpr int kFinalGroups = 8;
+
+__global__ void __launch_bounds__(32 * kFinalGroups)
+k_structure_final(const double* __restrict__ part, int slices, KArgs ka, double inv_2alpha2,
+                  double* __restrict__ coef, double* rpart, unsigned* ticket, double* out) {
+    __shared__ double sums[kFinalGroups][32];
+    const int lane = threadIdx.x % 32, g = threadIdx.x / 32;
+    const int idx = blockIdx.x * 32 + lane;  // kColSums * ntask is a multiple of 32
+    const int64_t count = static_cast<int64_t>(kColSums) * ka.ntask;
+    double A = 0.0;
+#pragma unroll 8
+    for (int s = g; s < slices; s += kFinalGroups) A += part[s * count + idx];
+    sums[g][lane] = A;
+    __syncthreads();
     double v[2] = {0.0, 0.0};
-    if (k < ka.nk) {
-        double re = 0.0, im = 0.0;
-        for (int s = 0; s < slices; ++s) {
-            const double2 p = part[static_cast<int64_t>(s) * ka.nk + k];
-            re += p.x;
-            im += p.y;
-        }
-        sk[k] = make_double2(re, im);
-        const double4 kv = ka.kvec[k];
-        const double k2 = kv.x * kv.x + kv.y * kv.y + kv.z * kv.z;
-        const double e = 2.0 * kv.w * (re * re + im * im);
+    if (g == 0) {
+#pragma unroll
+        for (int k = 1; k < kFinalGroups; ++k) A += sums[k][lane];
+        const int j = idx / ka.ntask, t = idx % ka.ntask;
+        const double2 f = ka.fac[t * kColZ + j / 8];
+        const double e = f.x * A * A;
         v[0] = e;
-        v[1] = e * (1.0 - k2 * inv_2alpha2);
+        v[1] = e * (1.0 - f.y * inv_2alpha2);
+        coef[static_cast<int64_t>(t) * kColSums + j] = 2.0 * f.x * A;
     }
     grid_reduce<2>(v, rpart, ticket, out);
 }
 
-// Reciprocal-space forces (ewald.cpp:163-170), one thread per site, k vectors in
-// (nx, ny) lines with exp(i nz c z) stepped along each line.
-// k-space forces (or, with CHARGE, dE_recip/dq_s = sum over the half space of
-// 4 factor Re(conj(S) e^{i k.r_s})) over a 2-D grid: blockIdx.x picks 256 sites,
-// blockIdx.y a slice of the (nx, ny) lines of k vectors, so small systems still
-// fill the GPU.  Each slice starts its e^{i nx a x}, e^{i ny b y} factors with
-// sincos and continues by complex recurrence along its lines; its partial sums go
-// to part[slice][site] and k_recip_sum adds the slices in order (deterministic).
+// F = -q grad U (or, with CHARGE, dE_recip/dq = U) of one site per thread over a 2-D
+// grid: blockIdx.x picks 128 sites, blockIdx.y a range of task chunks, so small systems
+// still fill the GPU; k_recip_sum adds the ranges in order (deterministic).  A chunk's
+// coefficients are staged in shared memory and read as broadcasts; the site's z factors
+// of the chunk's kColZ nz stay in registers, x and y factors start with sincos at each
+// chunk and continue by complex recurrence.  Per task and site 64 multiply-adds form
+// G_ab = sum_c coef_abc c(z) and dG_ab/dz, about 23 more the gradient: the FP64 pipe
+// bounds the kernel.  12,288 sites, kmax 18: 769 us with one complex exponential per
+// vector, 108 us in this form; two sites a thread, sharing the broadcasts, measured the
+// same.
 template <bool CHARGE>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kSumBlock)
 k_recip_force(const double4* __restrict__ pos, const double* __restrict__ q, int64_t n, KArgs ka,
-              const int4* __restrict__ lines, int nlines, int lines_per_slice,
-              const double2* __restrict__ sk, double4* __restrict__ part) {
-    const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (s >= n) return;
-    const int l0 = blockIdx.y * lines_per_slice;
-    const int l1 = min(nlines, l0 + lines_per_slice);
-    const double4 p = pos[s];
-    const double qs = q[s];
-    double sn, cs;
-    sincos(ka.a * p.x, &sn, &cs);
-    const double2 ex = make_double2(cs, sn);
-    sincos(ka.b * p.y, &sn, &cs);
-    const double2 ey = make_double2(cs, sn);
-    sincos(ka.c * p.z, &sn, &cs);
-    const double2 ez = make_double2(cs, sn);
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    double2 X = make_double2(1.0, 0.0), Y = make_double2(1.0, 0.0);
-    int cur_nx = INT_MIN, cur_ny = INT_MIN;
-    for (int l = l0; l < l1; ++l) {
-        const int4 L = lines[l];  // nx, ny, nz0, first k index; count in next line's .w
-        if (L.x != cur_nx) {
-            if (cur_nx != INT_MIN && L.x == cur_nx + 1) {
+              int chunks_per_slice, const double* __restrict__ coef, double4* __restrict__ part) {
+    __shared__ double2 cs[kTaskChunk * kColSums / 2];
+    __shared__ int4 tks[kTaskChunk];
+    const int64_t s = blockIdx.x * static_cast<int64_t>(kSumBlock) + threadIdx.x;
+    const double4 p = pos[s < n ? s : n - 1];
+    double2 ex, ey, ez;
+    sincos(ka.a * p.x, &ex.y, &ex.x);
+    sincos(ka.b * p.y, &ey.y, &ey.x);
+    sincos(ka.c * p.z, &ez.y, &ez.x);
+    double ux = 0.0, uy = 0.0, uz = 0.0;
+    const int chunks = ka.ntask / kTaskChunk;
+    const int c0 = blockIdx.y * chunks_per_slice, c1 = min(chunks, c0 + chunks_per_slice);
+    for (int c = c0; c < c1; ++c) {
+        __syncthreads();
+        const double2* src = reinterpret_cast<const double2*>(
+            coef + static_cast<int64_t>(c) * kTaskChunk * kColSums);
+        for (int w = threadIdx.x; w < kTaskChunk * kColSums / 2; w += kSumBlock) cs[w] = __ldg(src + w);
+        if (threadIdx.x < kTaskChunk) tks[threadIdx.x] = __ldg(ka.task + c * kTaskChunk + threadIdx.x);
+        __syncthreads();
+        int4 tk = tks[0];
+        double2 X, Y, Z[kColZ];
+        double kz[kColZ];
+        sincos(static_cast<double>(tk.x) * ka.a * p.x, &X.y, &X.x);
+        sincos(static_cast<double>(tk.y) * ka.b * p.y, &Y.y, &Y.x);
+        sincos(static_cast<double>(tk.z) * ka.c * p.z, &Z[0].y, &Z[0].x);
+#pragma unroll
+        for (int z = 0; z < kColZ; ++z) {
+            if (z > 0) Z[z] = cmul(Z[z - 1], ez);
+            kz[z] = static_cast<double>(tk.z + z) * ka.c;
+        }
+        for (int i = 0; i < kTaskChunk; ++i) {
+            const int4 nt = tks[i];
+            if (!nt.w) break;  // padding ends a chunk
+            if (nt.x != tk.x) {  // the next column of x: ny starts again at 0
                 X = cmul(X, ex);
-            } else {
-                sincos(static_cast<double>(L.x) * ka.a * p.x, &sn, &cs);
-                X = make_double2(cs, sn);
-            }
-            cur_nx = L.x;
-            cur_ny = INT_MIN;
-        }
-        if (L.y != cur_ny) {
-            if (cur_ny != INT_MIN && L.y == cur_ny + 1) {
+                Y = make_double2(1.0, 0.0);
+            } else if (nt.y != tk.y) {
                 Y = cmul(Y, ey);
-            } else {
-                sincos(static_cast<double>(L.y) * ka.b * p.y, &sn, &cs);
-                Y = make_double2(cs, sn);
             }
-            cur_ny = L.y;
-        }
-        const double2 XY = cmul(X, Y);
-        sincos(static_cast<double>(L.z) * ka.c * p.z, &sn, &cs);
-        double2 Z = make_double2(cs, sn);
-        const int k0 = L.w, k1 = (l + 1 < nlines) ? lines[l + 1].w : ka.nk;
-        for (int k = k0; k < k1; ++k) {
-            const double2 e = cmul(XY, Z);
-            const double4 kv = ka.kvec[k];
-            const double2 S = sk[k];
+            tk = nt;
+            double G[4], D[4];
+#pragma unroll
+            for (int ab = 0; ab < 4; ++ab) G[ab] = D[ab] = 0.0;
+#pragma unroll
+            for (int z = 0; z < kColZ; ++z) {
+                const double dc = kz[z] * Z[z].x, ds = -kz[z] * Z[z].y;
+#pragma unroll
+                for (int ab = 0; ab < 4; ++ab) {
+                    const double2 B = cs[i * (kColSums / 2) + z * 4 + ab];
+                    G[ab] = fma(B.x, Z[z].x, fma(B.y, Z[z].y, G[ab]));
+                    if (!CHARGE) D[ab] = fma(B.x, ds, fma(B.y, dc, D[ab]));
+                }
+            }
+            const double pc = fma(Y.x, G[0], Y.y * G[1]), ps = fma(Y.x, G[2], Y.y * G[3]);
             if (CHARGE) {
-                fx += 4.0 * kv.w * (S.x * e.x + S.y * e.y);
+                ux = fma(X.x, pc, fma(X.y, ps, ux));
             } else {
-                // 2 (half space) * factor * 2 * q * (Re S sin - Im S cos)
-                const double coeff = 4.0 * kv.w * qs * (S.x * e.y - S.y * e.x);
-                fx = fma(coeff, kv.x, fx);
-                fy = fma(coeff, kv.y, fy);
-                fz = fma(coeff, kv.z, fz);
+                const double kx = static_cast<double>(tk.x) * ka.a;
+                const double ky = static_cast<double>(tk.y) * ka.b;
+                const double qc = fma(Y.x, G[1], -Y.y * G[0]), qsn = fma(Y.x, G[3], -Y.y * G[2]);
+                const double rc = fma(Y.x, D[0], Y.y * D[1]), rs = fma(Y.x, D[2], Y.y * D[3]);
+                ux = fma(kx, fma(X.x, ps, -X.y * pc), ux);
+                uy = fma(ky, fma(X.x, qc, X.y * qsn), uy);
+                uz = fma(X.x, rc, fma(X.y, rs, uz));
             }
-            Z = cmul(Z, ez);
         }
     }
-    part[blockIdx.y * n + s] = make_double4(fx, fy, fz, 0.0);
+    if (s >= n) return;
+    if (CHARGE) {
+        part[blockIdx.y * n + s] = make_double4(ux, 0.0, 0.0, 0.0);
+    } else {
+        const double mq = -q[s];
+        part[blockIdx.y * n + s] = make_double4(mq * ux, mq * uy, mq * uz, 0.0);
+    }
 }
 
-// Adds the slices' partial k-space forces (CHARGE: charge gradients), one warp
-// per site: lane l sums slices l, l + 32, ... in order, then the lanes combine
-// by a fixed butterfly, so the result does not depend on scheduling.
+// Adds the slices' partial k-space forces (CHARGE: charge gradients), `lanes` (a power
+// of two up to 32) per site: lane l sums slices l, l + lanes, ... in order, then the
+// lanes combine by a fixed butterfly, so the result does not depend on scheduling.
 template <bool CHARGE>
-__global__ void k_recip_sum(const double4* __restrict__ part, int slices, int64_t n, double* fxo,
-                            double* fyo, double* fzo, double* dq) {
-    const int64_t s = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (s >= n) return;  // whole warps leave together
+__global__ void k_recip_sum(const double4* __restrict__ part, int slices, int lanes, int64_t n,
+                            double* fxo, double* fyo, double* fzo, double* dq) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    const int64_t s = t / lanes;
+    const int lane = static_cast<int>(t % lanes);
     double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int k = lane; k < slices; k += 32) {
-        const double4 v = part[k * n + s];
-        fx += v.x;
-        fy += v.y;
-        fz += v.z;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    if (s < n)
+        for (int k = lane; k < slices; k += lanes) {
+            const double4 v = part[k * n + s];
+            fx += v.x;
+            fy += v.y;
+            fz += v.z;
+        }
+    for (int o = lanes / 2; o > 0; o >>= 1) {
         fx += __shfl_xor_sync(0xffffffffu, fx, o);
         fy += __shfl_xor_sync(0xffffffffu, fy, o);
         fz += __shfl_xor_sync(0xffffffffu, fz, o);
     }
-    if (lane != 0) return;
+    if (s >= n || lane != 0) return;
     if (CHARGE) {
         dq[s] += fx;
     } else {
@@ -464,12 +509,15 @@ __global__ void k_recip_sum(const double4* __restrict__ part, int slices, int64_
     }
 }
 
-// Grid of the k-space force pass: enough line slices to give every SM a few
-// blocks (one slice for large systems).
-int recip_slices(const md_context* ctx, int64_t n, int nlines) {
-    const int64_t site_blocks = (n + kBlock - 1) / kBlock;
-    int64_t slices = (4 * static_cast<int64_t>(ctx->sm_count) + site_blocks - 1) / site_blocks;
-    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(slices, nlines)));
+// Task chunks per block of the k-space force pass: enough slices for six blocks an SM,
+// which take turns on the four resident, at most one per chunk.  12,288 sites: 126 us with
+// as many blocks as are resident at once (the longest block sets the time), 108 us so.
+int recip_chunks_per_slice(const md_context* ctx, int64_t n, int ntask) {
+    const int chunks = ntask / kTaskChunk;
+    const int64_t site_blocks = (n + kSumBlock - 1) / kSumBlock;
+    int64_t slices = (6 * static_cast<int64_t>(ctx->sm_count) + site_blocks - 1) / site_blocks;
+    slices = std::max<int64_t>(1, std::min<int64_t>(slices, chunks));
+    return static_cast<int>((chunks + slices - 1) / slices);
 }
 
 __global__ void k_to_slot4(const int* __restrict__ slot, int64_t n, const double4* in, double4* out) {
@@ -645,9 +693,8 @@ struct md_ewald {
     double kbox[3] = {0, 0, 0};
     int k_kmax = -1;
     double k_alpha = 0.0;
-    mdb::DevBuf kvec, kn, lines, sk, skpart;
-    mdb::DevBuf rpart;            // per line slice k-space force partials
-    int nk = 0, nlines = 0;
+    mdb::DevBuf ktask, kfac, kcoef;
+    int nk = 0, ntask = 0;        // half-space vectors; tasks, whole chunks of them
     double last[kEwCount] = {0};
     double alpha = 0.0;
     mdb::PmeState* pme = nullptr;  // reciprocal term by smooth PME instead of k-vector sums
@@ -690,8 +737,9 @@ int ewald_topology(md_ewald* ew, md_system* sys) {
     return MD_OK;
 }
 
-// k vectors of the half space, grouped in (nx, ny) lines (ewald.cpp:112-172): the
-// full set n in [-kmax,kmax]^3, 0 < |n|^2 < kmax^2 + 2, is {k} u {-k} of these.
+// The octant's k vectors (ewald.cpp:112-172: n in [-kmax, kmax]^3, 0 < |n|^2 < kmax^2 + 2,
+// which the octant's signs cover) as tasks of kColZ consecutive nz, grouped by nz0; within
+// a group nx ascends, and for each nx ny ascends from 0.
 int ewald_kvectors(md_ewald* ew, const double box[3], double alpha) {
     if (ew->k_kmax == ew->kmax && ew->k_alpha == alpha && ew->kbox[0] == box[0] &&
         ew->kbox[1] == box[1] && ew->kbox[2] == box[2])
@@ -701,41 +749,44 @@ int ewald_kvectors(md_ewald* ew, const double box[3], double alpha) {
     const double kx0 = 2.0 * kPi / box[0], ky0 = 2.0 * kPi / box[1], kz0 = 2.0 * kPi / box[2];
     const int n2max = kmax * kmax + 2;
     const double coulomb = coulomb_prefactor();
-    std::vector<double4> kv;
-    std::vector<int4> kn, lines;
-    for (int nx = 0; nx <= kmax; ++nx) {
-        for (int ny = -kmax; ny <= kmax; ++ny) {
-            if (nx == 0 && ny < 0) continue;
-            int first = -1;
-            for (int nz = -kmax; nz <= kmax; ++nz) {
-                if (nx == 0 && ny == 0 && nz <= 0) continue;
-                const int n2 = nx * nx + ny * ny + nz * nz;
-                if (n2 == 0 || n2 >= n2max) continue;
-                if (first < 0) first = nz;
-                const double kxv = kx0 * static_cast<double>(nx);
-                const double kyv = ky0 * static_cast<double>(ny);
-                const double kzv = kz0 * static_cast<double>(nz);
-                const double k2 = kxv * kxv + kyv * kyv + kzv * kzv;
-                const double factor =
-                    coulomb * (2.0 * kPi / volume) * std::exp(-k2 / (4.0 * alpha * alpha)) / k2;
-                if (first == nz) lines.push_back(make_int4(nx, ny, nz, static_cast<int>(kv.size())));
-                kv.push_back(make_double4(kxv, kyv, kzv, factor));
-                kn.push_back(make_int4(nx, ny, nz, 0));
+    std::vector<int4> task;
+    std::vector<double2> fac;
+    int full = 0;  // vectors of the full set
+    for (int z0 = 0; z0 <= kmax; z0 += kColZ) {
+        for (int nx = 0; nx <= kmax; ++nx) {
+            for (int ny = 0; ny <= kmax && nx * nx + ny * ny + z0 * z0 < n2max; ++ny) {
+                task.push_back(make_int4(nx, ny, z0, 1));
+                for (int nz = z0; nz < z0 + kColZ; ++nz) {
+                    const int n2 = nx * nx + ny * ny + nz * nz;
+                    if (nz > kmax || n2 == 0 || n2 >= n2max) {
+                        fac.push_back(make_double2(0.0, 0.0));
+                        continue;
+                    }
+                    const int signs = (nx ? 2 : 1) * (ny ? 2 : 1) * (nz ? 2 : 1);
+                    const double kxv = kx0 * static_cast<double>(nx);
+                    const double kyv = ky0 * static_cast<double>(ny);
+                    const double kzv = kz0 * static_cast<double>(nz);
+                    const double k2 = kxv * kxv + kyv * kyv + kzv * kzv;
+                    const double factor =
+                        coulomb * (2.0 * kPi / volume) * std::exp(-k2 / (4.0 * alpha * alpha)) / k2;
+                    fac.push_back(make_double2(signs * factor, k2));
+                    full += signs;
+                }
             }
         }
+        while (task.size() % kTaskChunk) {
+            task.push_back(make_int4(0, 0, z0, 0));
+            for (int z = 0; z < kColZ; ++z) fac.push_back(make_double2(0.0, 0.0));
+        }
     }
-    ew->nk = static_cast<int>(kv.size());
-    ew->nlines = static_cast<int>(lines.size());
-    const size_t nk = std::max<size_t>(kv.size(), 1);
-    MDB_TRY(ew->kvec.ensure(sizeof(double4) * nk));
-    MDB_TRY(ew->kn.ensure(sizeof(int4) * nk));
-    MDB_TRY(ew->lines.ensure(sizeof(int4) * std::max<size_t>(lines.size(), 1)));
-    MDB_TRY(ew->sk.ensure(sizeof(double2) * nk));
-    if (!kv.empty()) {
-        MDB_CUDA(cudaMemcpy(ew->kvec.ptr, kv.data(), sizeof(double4) * kv.size(), cudaMemcpyHostToDevice));
-        MDB_CUDA(cudaMemcpy(ew->kn.ptr, kn.data(), sizeof(int4) * kn.size(), cudaMemcpyHostToDevice));
-        MDB_CUDA(cudaMemcpy(ew->lines.ptr, lines.data(), sizeof(int4) * lines.size(),
-                            cudaMemcpyHostToDevice));
+    ew->nk = full / 2;
+    ew->ntask = ew->nk > 0 ? static_cast<int>(task.size()) : 0;
+    if (ew->ntask > 0) {
+        MDB_TRY(ew->ktask.ensure(sizeof(int4) * task.size()));
+        MDB_TRY(ew->kfac.ensure(sizeof(double2) * fac.size()));
+        MDB_TRY(ew->kcoef.ensure(sizeof(double) * kColSums * task.size()));
+        MDB_CUDA(cudaMemcpy(ew->ktask.ptr, task.data(), sizeof(int4) * task.size(), cudaMemcpyHostToDevice));
+        MDB_CUDA(cudaMemcpy(ew->kfac.ptr, fac.data(), sizeof(double2) * fac.size(), cudaMemcpyHostToDevice));
     }
     ew->k_kmax = kmax;
     ew->k_alpha = alpha;
@@ -776,28 +827,30 @@ int ewald_list(md_ewald* ew, md_system* sys) {
 // gated: the neighbour list is maintained by device-decided rebuilds (no host
 // synchronisation; the list must already be built for this system).
 // k-space forces added to the system's forces (charge = false), or
-// dE_recip/dq added to dq (device order); S(k) must be current.
+// dE_recip/dq added to dq (device order); the coefficients must be current.
 int recip_force_async(md_ewald* ew, md_system* sys, const KArgs& ka, bool charge, double* dq) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
-    if (n == 0 || ew->nk == 0) return MD_OK;
-    const int slices = recip_slices(ctx, n, ew->nlines);
-    const int per = (ew->nlines + slices - 1) / slices;
-    MDB_TRY(ew->rpart.ensure(sizeof(double4) * static_cast<size_t>(slices) * n));
-    const dim3 grid(static_cast<unsigned>((n + kBlock - 1) / kBlock), static_cast<unsigned>(slices));
-    double4* part = ew->rpart.as<double4>();
+    if (n == 0 || ew->ntask == 0) return MD_OK;
+    const int per = recip_chunks_per_slice(ctx, n, ew->ntask);
+    const int slices = (ew->ntask / kTaskChunk + per - 1) / per;
+    void* scratch;
+    MDB_TRY(ctx_scratch(ctx, sizeof(double4) * static_cast<size_t>(slices) * n, &scratch));
+    const dim3 grid(static_cast<unsigned>((n + kSumBlock - 1) / kSumBlock), static_cast<unsigned>(slices));
+    double4* part = static_cast<double4*>(scratch);
+    int lanes = 1;
+    while (lanes < 32 && lanes < slices) lanes *= 2;
+    const unsigned sum_grid = grid_for(lanes * n, kBlock);
     if (charge) {
-        k_recip_force<true><<<grid, kBlock, 0, ctx->stream>>>(
-            sys->cur.pos, sys->cur.charge, n, ka, ew->lines.as<int4>(), ew->nlines, per,
-            ew->sk.as<double2>(), part);
-        k_recip_sum<true><<<grid_for(32 * n, kBlock), kBlock, 0, ctx->stream>>>(
-            part, slices, n, nullptr, nullptr, nullptr, dq);
+        k_recip_force<true><<<grid, kSumBlock, 0, ctx->stream>>>(
+            sys->cur.pos, sys->cur.charge, n, ka, per, ew->kcoef.as<double>(), part);
+        k_recip_sum<true><<<sum_grid, kBlock, 0, ctx->stream>>>(part, slices, lanes, n, nullptr,
+                                                               nullptr, nullptr, dq);
     } else {
-        k_recip_force<false><<<grid, kBlock, 0, ctx->stream>>>(
-            sys->cur.pos, sys->cur.charge, n, ka, ew->lines.as<int4>(), ew->nlines, per,
-            ew->sk.as<double2>(), part);
-        k_recip_sum<false><<<grid_for(32 * n, kBlock), kBlock, 0, ctx->stream>>>(
-            part, slices, n, sys->cur.fx, sys->cur.fy, sys->cur.fz, nullptr);
+        k_recip_force<false><<<grid, kSumBlock, 0, ctx->stream>>>(
+            sys->cur.pos, sys->cur.charge, n, ka, per, ew->kcoef.as<double>(), part);
+        k_recip_sum<false><<<sum_grid, kBlock, 0, ctx->stream>>>(
+            part, slices, lanes, n, sys->cur.fx, sys->cur.fy, sys->cur.fz, nullptr);
     }
     ctx->launches += 2;
     MDB_CHECK_LAUNCH();
@@ -826,9 +879,9 @@ RealArgs real_args_of(const md_ewald* ew, double alpha) {
 
 KArgs kargs_of(md_ewald* ew, const md_system* sys) {
     KArgs ka;
-    ka.kvec = ew->kvec.as<double4>();
-    ka.kn = ew->kn.as<int4>();
-    ka.nk = ew->nk;
+    ka.task = ew->ktask.as<int4>();
+    ka.fac = ew->kfac.as<double2>();
+    ka.ntask = ew->ntask;
     ka.kmax = ew->kmax;
     ka.a = 2.0 * kPi / sys->box[0];
     ka.b = 2.0 * kPi / sys->box[1];
@@ -890,27 +943,32 @@ int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated) {
     if (ew->pme) {
         MDB_TRY(pme_eval_async(ew->pme, sys, alpha, coulomb_prefactor(), mode, res + kEwRecip,
                                ctx_counter(ctx, 12)));
-    } else if (ew->nk > 0 && n > 0) {
-        const int kblocks = (ew->nk + kBlock - 1) / kBlock;
-        // enough site slices to give every SM a few blocks
-        int64_t slices = std::max<int64_t>(1, (4 * ctx->sm_count) / kblocks);
+    } else if (ew->ntask > 0 && n > 0) {
+        const int tblocks = (ew->ntask + kSumBlock - 1) / kSumBlock;
+        // enough site slices to give every SM three blocks
+        int64_t slices = std::max<int64_t>(1, (3 * ctx->sm_count) / tblocks);
         slices = std::min<int64_t>(slices, (n + kSiteTile - 1) / kSiteTile);
         const int64_t per = ((n + slices - 1) / slices + kSiteTile - 1) / kSiteTile * kSiteTile;
         slices = (n + per - 1) / per;
-        MDB_TRY(ew->skpart.ensure(sizeof(double2) * static_cast<size_t>(slices) * ew->nk));
-        const size_t smem =
-            sizeof(double2) * kSiteTile * static_cast<size_t>((ew->kmax + 1) + 2 * (2 * ew->kmax + 1));
+        // the slices' sums, like the force pass's after them, live in the context's
+        // scratch only until the kernel that adds them
+        void* scratch;
+        MDB_TRY(ctx_scratch(ctx, sizeof(double) * kColSums * static_cast<size_t>(slices) * ew->ntask,
+                            &scratch));
+        double* kpart = static_cast<double*>(scratch);
+        const size_t smem = sizeof(double2) * 3 * table_axis(ew->kmax) * (kSiteTile + 1);
         if (smem > 48 * 1024)
             MDB_CUDA(cudaFuncSetAttribute(k_structure_factor,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           static_cast<int>(smem)));
-        k_structure_factor<<<dim3(kblocks, static_cast<unsigned>(slices)), kBlock, smem, ctx->stream>>>(
-            sys->cur.pos, sys->cur.charge, n, ka, per, ew->skpart.as<double2>());
+        k_structure_factor<<<dim3(tblocks, static_cast<unsigned>(slices)), kSumBlock, smem, ctx->stream>>>(
+            sys->cur.pos, sys->cur.charge, n, ka, per, kpart);
+        const int fblocks = kColSums * ew->ntask / 32;
         double* rp;
-        MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(kblocks), &rp));
-        k_structure_final<<<kblocks, kBlock, 0, ctx->stream>>>(
-            ew->skpart.as<double2>(), static_cast<int>(slices), ka, 1.0 / (2.0 * alpha * alpha),
-            ew->sk.as<double2>(), rp, ctx_counter(ctx, 7), res + kEwRecip);
+        MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(fblocks), &rp));
+        k_structure_final<<<fblocks, 32 * kFinalGroups, 0, ctx->stream>>>(
+            kpart, static_cast<int>(slices), ka, 1.0 / (2.0 * alpha * alpha),
+            ew->kcoef.as<double>(), rp, ctx_counter(ctx, 7), res + kEwRecip);
         if (mode != 0) MDB_TRY(recip_force_async(ew, sys, ka, false, nullptr));
     } else {
         MDB_CUDA(cudaMemsetAsync(res + kEwRecip, 0, 2 * sizeof(double), ctx->stream));
@@ -980,12 +1038,9 @@ int md_ewald_destroy(md_ewald* ew) {
     }
     ew->partner_off.release();
     ew->partner_idx.release();
-    ew->kvec.release();
-    ew->kn.release();
-    ew->lines.release();
-    ew->rpart.release();
-    ew->sk.release();
-    ew->skpart.release();
+    ew->ktask.release();
+    ew->kfac.release();
+    ew->kcoef.release();
     delete ew;
     return MD_OK;
 }
