@@ -52,51 +52,75 @@ LJArgs make_lj_args(const md_lj* lj) {
     return a;
 }
 
-// lennard_jones.cpp:62-79 with exact operation order.  Returns false outside rc.
-template <bool LFS>
-__device__ __forceinline__ bool pair_exact(const LJArgs& a, double r2, double& u, double& w,
-                                           double& s) {
-    if (!(r2 < a.rc2)) return false;
-    const double s2 = __ddiv_rn(a.sig2, r2);
+// lennard_jones.cpp:62-79 with exact operation order, for a pair inside rc; DIV divides by
+// r2.
+struct PairTerms {
+    double u, w, s;
+};
+
+template <bool LFS, class Div>
+__device__ __forceinline__ PairTerms pair_terms(const LJArgs& a, double r2, Div div) {
+    PairTerms t;
+    const double s2 = div(a.sig2);
     const double s6 = __dmul_rn(__dmul_rn(s2, s2), s2);
-    const double uLJ = __dmul_rn(a.four_eps, __dsub_rn(__dmul_rn(s6, s6), s6));
-    const double wLJ = __dmul_rn(a.tf_eps, __dsub_rn(__dmul_rn(__dmul_rn(2.0, s6), s6), s6));
+    const double s12 = __dmul_rn(s6, s6);
+    t.u = __dmul_rn(a.four_eps, __dsub_rn(s12, s6));
+    t.w = __dmul_rn(a.tf_eps, __dsub_rn(__dmul_rn(2.0, s12), s6));  // (2 s6) s6 = 2 s12 exactly
     if (LFS) {
         const double r = __dsqrt_rn(r2);
-        u = __dsub_rn(__dsub_rn(uLJ, a.uc), __dmul_rn(__dsub_rn(r, a.rc), a.dudrc));
-        w = __dadd_rn(wLJ, __dmul_rn(r, a.dudrc));
-    } else {
-        u = uLJ;
-        w = wLJ;
+        t.u = __dsub_rn(__dsub_rn(t.u, a.uc), __dmul_rn(__dsub_rn(r, a.rc), a.dudrc));
+        t.w = __dadd_rn(t.w, __dmul_rn(r, a.dudrc));
     }
-    s = __ddiv_rn(w, r2);
+    t.s = div(t.w);
+    return t;
+}
+
+// Separations so small (or large) that the fast quotients could under- or overflow.
+template <bool LFS>
+__device__ __noinline__ PairTerms pair_terms_ieee(double sig2, double four_eps, double tf_eps,
+                                                  double rc, double uc, double dudrc, double r2) {
+    LJArgs a;
+    a.sig2 = sig2;
+    a.four_eps = four_eps;
+    a.tf_eps = tf_eps;
+    a.rc = rc;
+    a.uc = uc;
+    a.dudrc = dudrc;
+    return pair_terms<LFS>(a, r2, [r2](double x) { return __ddiv_rn(x, r2); });
+}
+
+// Both divisions of a pair share one reciprocal (bit-identical quotients).  Returns false
+// outside rc.
+template <bool LFS>
+__device__ __forceinline__ bool pair_exact(const LJArgs& a, double r2, PairTerms& t) {
+    if (!(r2 < a.rc2)) return false;
+    if (divides_fast(r2)) {
+        const double y = reciprocal(r2);
+        t = pair_terms<LFS>(a, r2, [r2, y](double x) { return quotient(x, r2, y); });
+    } else {
+        t = pair_terms_ieee<LFS>(a.sig2, a.four_eps, a.tf_eps, a.rc, a.uc, a.dudrc, r2);
+    }
     return true;
 }
 
 // Accumulates the pair (i, j) into atom i's force (FP64 reference arithmetic).
-// The displacement is always r_lo - r_hi by original index, as the reference's
-// i<j pair sources produce it; atom lo gains +f, atom hi gains -f.
+// The displacement has the rounding of r_lo - r_hi by original index, as the reference's
+// i<j pair sources produce it, and atom i's sign; the lower atom counts the energy.
 template <bool LFS>
 __device__ __forceinline__ void accumulate_exact(const LJArgs& a, const Fold3& f3, double4 pi,
                                                  double4 pj, double& fx, double& fy, double& fz,
                                                  double& e, double& vir) {
     const bool lo = pi.w < pj.w;
     double dx, dy, dz;
-    if (lo) min_image_wrapped(f3, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, dx, dy, dz);
-    else min_image_wrapped(f3, pj.x, pj.y, pj.z, pi.x, pi.y, pi.z, dx, dy, dz);
-    double u, w, s;
-    if (!pair_exact<LFS>(a, norm2_exact(dx, dy, dz), u, w, s)) return;
-    const double gx = __dmul_rn(dx, s), gy = __dmul_rn(dy, s), gz = __dmul_rn(dz, s);
+    min_image_pair(f3, pi, pj, lo, dx, dy, dz);
+    PairTerms t;
+    if (!pair_exact<LFS>(a, norm2_exact(dx, dy, dz), t)) return;
+    fx = __dadd_rn(fx, __dmul_rn(dx, t.s));
+    fy = __dadd_rn(fy, __dmul_rn(dy, t.s));
+    fz = __dadd_rn(fz, __dmul_rn(dz, t.s));
     if (lo) {
-        fx = __dadd_rn(fx, gx);
-        fy = __dadd_rn(fy, gy);
-        fz = __dadd_rn(fz, gz);
-        e = __dadd_rn(e, u);
-        vir = __dadd_rn(vir, w);
-    } else {
-        fx = __dsub_rn(fx, gx);
-        fy = __dsub_rn(fy, gy);
-        fz = __dsub_rn(fz, gz);
+        e = __dadd_rn(e, t.u);
+        vir = __dadd_rn(vir, t.w);
     }
 }
 
@@ -376,6 +400,103 @@ k_lj_verlet(const typename PosOf<MIXED>::T* __restrict__ pos, const double4* __r
 // The gathered kernel shape that also takes the closing half-kick (the default
 // shape; other shapes leave the kick to the integrator's own pass).
 constexpr bool verlet_kicks(int tpa, int unroll) { return tpa == 2 && unroll == 2; }
+
+// The FP64 pass of systems too small to fill the machine two threads an atom: kWide lanes
+// per atom each form the terms of one list entry, and the sums are then taken in the
+// two-thread kernel's order -- lane 2 c + p adds component c (fx, fy, fz, energy, virial)
+// of the entries of parity p one after another, from shared memory -- and with its
+// reduction tree (a block of 16 atoms is one warp of that kernel's), so forces, energy,
+// virial and kinetic energy are the two-thread kernel's bit for bit.  That kernel's time
+// is a row's chain of dependent pair terms when few warps share an SM; here the chain is
+// the additions alone.  Force pass of the liquid, two threads an atom against this (us,
+// events and launch included): 864 atoms 32 / 14, 4,000 atoms 32 / 17, 8,788 atoms 31 /
+// 22, 13,500 atoms 31 / 31, 32,000 atoms 36 / 54.
+constexpr int kWide = 16;
+constexpr int kWideAtoms = kBlock / kWide;
+
+template <bool LFS, bool KICK>
+__global__ void __launch_bounds__(kBlock, 4)
+k_lj_wide(const double4* __restrict__ pos, const int* __restrict__ nbr,
+          const int* __restrict__ count, int stride, int64_t n, Box3 box, LJArgs a,
+          double* __restrict__ fxo, double* __restrict__ fyo, double* __restrict__ fzo,
+          double* part, unsigned* ticket, double* out, KickArgs kick) {
+    constexpr int kTerms = 5;  // force, energy, virial
+    constexpr int K = KICK ? 3 : 2;
+    __shared__ double s_t[kWideAtoms][kTerms][kWide];
+    __shared__ double s_red[K][2 * kWideAtoms];
+    const int ai = threadIdx.x / kWide, g = threadIdx.x % kWide;
+    const int64_t i = blockIdx.x * static_cast<int64_t>(kWideAtoms) + ai;
+    const Fold3 f3 = fold3_of(box);
+    const int cnt = i < n ? min(count[i], stride) : 0;
+    const double4 pi = ldg4(pos + (i < n ? i : 0));
+    const int* row = nbr + (i < n ? i : 0) * static_cast<int64_t>(stride);
+    const int comp = g >> 1, par = g & 1;  // this lane's sum (comp < kTerms)
+    double acc = 0.0;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);  // of the warp's two atoms
+    int j = g < cnt ? __ldg(row + g) : -1;
+    double4 pj = ldg4(pos + (j >= 0 ? j : 0));
+    for (int k0 = 0; k0 < most; k0 += kWide) {
+        const int kn = k0 + kWide + g;
+        const int jn = kn < cnt ? __ldg(row + kn) : -1;
+        double v[kTerms] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (j >= 0) accumulate_exact<LFS>(a, f3, pi, pj, v[0], v[1], v[2], v[3], v[4]);
+#pragma unroll
+        for (int c = 0; c < kTerms; ++c) s_t[ai][c][g] = v[c];
+        j = jn;
+        pj = ldg4(pos + (j >= 0 ? j : 0));
+        __syncwarp();
+        if (comp < kTerms) {  // a term that is zero leaves the sum as it is
+#pragma unroll
+            for (int s = 0; s < kWide / 2; ++s) acc = __dadd_rn(acc, s_t[ai][comp][2 * s + par]);
+        }
+        __syncwarp();
+    }
+    const double f = acc + __shfl_xor_sync(0xffffffffu, acc, 1);  // both parities of a component
+    const double fy = __shfl_sync(0xffffffffu, f, 2, kWide), fz = __shfl_sync(0xffffffffu, f, 4, kWide);
+    double ke = 0.0;
+    if (i < n && g == 0) {
+        const double fx = f;
+        fxo[i] = fx;
+        fyo[i] = fy;
+        fzo[i] = fz;
+        if constexpr (KICK) {  // the closing half-kick, as the separate kick kernel does it
+            const double c = __dmul_rn(kick.half_dt, kick.inv_mass[i]);
+            const double vx = fma(c, fx, kick.vx[i]);
+            const double vy = fma(c, fy, kick.vy[i]);
+            const double vz = fma(c, fz, kick.vz[i]);
+            kick.vx[i] = vx;
+            kick.vy[i] = vy;
+            kick.vz[i] = vz;
+            ke = 0.5 * kick.mass[i] * (vx * vx + vy * vy + vz * vz);
+        }
+    }
+    if (comp == 3 || comp == 4) s_red[comp - 3][2 * ai + par] = acc;
+    if (KICK && g < 2) s_red[K - 1][2 * ai + g] = ke;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < K) {
+        const double s = warp_sum(s_red[warp][lane]);
+        if (lane == 0) {
+            part[static_cast<size_t>(blockIdx.x) * K + warp] = s;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    // eight of these blocks are one block of the two-thread kernel: its eight warps' sums,
+    // added by the tree of a warp whose other lanes are zero
+    __shared__ double sm[K][32];
+    const unsigned nb = gridDim.x;
+    grid_reduce_tail<K>(sm, (nb + 7) / 8, ticket, out, KICK ? kick.status : nullptr, nb,
+                        [=](unsigned p, int k) {
+                            double v[8];
+#pragma unroll
+                            for (unsigned w = 0; w < 8; ++w)
+                                v[w] = 8 * p + w < nb
+                                           ? __ldcg(part + static_cast<size_t>(8 * p + w) * K + k)
+                                           : 0.0;
+                            return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+                        });
+}
 
 // One system's arguments of the batched force pass.
 struct BatchForceRep {
@@ -1245,6 +1366,22 @@ bool launch_verlet(md_system* sys, md_verlet* v, const LJArgs& a, double* part, 
     return kicks;
 }
 
+// FP64 systems of up to 64 atoms per SM take kWide lanes an atom (see k_lj_wide); the mixed
+// pass, whose pair terms are a few FP32 operations, gains too little to leave two threads.
+bool verlet_wide(const md_context* ctx, int64_t n, bool mixed, int tpa, int unroll) {
+    return !mixed && tpa == 2 && unroll == 2 && n > 0 &&
+           n < 64 * static_cast<int64_t>(ctx->sm_count);
+}
+
+template <bool LFS>
+void launch_wide(md_system* sys, md_verlet* v, const LJArgs& a, double* part, unsigned* ticket,
+                 double* out, const KickArgs* kick) {
+    auto kernel = kick ? k_lj_wide<LFS, true> : k_lj_wide<LFS, false>;
+    kernel<<<grid_for(sys->n, kWideAtoms), kBlock, 0, sys->ctx->stream>>>(
+        sys->cur.pos, v->nbr.as<int>(), v->count.as<int>(), v->stride, sys->n, box_of(sys), a,
+        sys->cur.fx, sys->cur.fy, sys->cur.fz, part, ticket, out, kick ? *kick : KickArgs{});
+}
+
 // Fixed-point positions for the mixed pair kernels (quantize_position), skipped
 // when `flag` is given and zero: the step's kick/drift already wrote them and no
 // rebuild re-sorted the atoms since.
@@ -1406,14 +1543,15 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
     md_context* ctx = sys->ctx;
     const LJArgs a = verlet_lj_args(lj, sys);
     const int tpa = lj->tpa ? lj->tpa : g_lj_tpa, unroll = lj->unroll ? lj->unroll : g_lj_unroll;
-    const int64_t threads = std::max<int64_t>(sys->n * tpa, 1);
+    const bool mixed = lj->precision == MD_PRECISION_MIXED;
+    const bool wide = verlet_wide(ctx, sys->n, mixed, tpa, unroll);
+    const int64_t threads = std::max<int64_t>(sys->n * (wide ? kWide : tpa), 1);
     const int64_t blocks = std::max<int64_t>(grid_for(threads, kBlock), halo_blocks(sys->n));
     double* part;
     MDB_TRY(ctx_partials(ctx, 3 * static_cast<size_t>(blocks), &part));
     unsigned* ticket = ctx_counter(ctx, 2);
     double* out = ctx_result(ctx, kResEnergy);
     const bool lfs = lj->truncation == MD_LINEAR_FORCE_SHIFT;
-    const bool mixed = lj->precision == MD_PRECISION_MIXED;
     if (!q_current) MDB_TRY(lj_quantize_async(lj, sys, q_gate));
     // halo tiles, when the list keeps them (fused runs of large systems turn them on,
     // or md_verlet_set_halo)
@@ -1430,6 +1568,10 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
         // the default halo kernel also takes the closing half-kick when asked
         if (lfs) launch_halo_u<true>(unroll, sys, v, a, part, ticket, out, kick);
         else launch_halo_u<false>(unroll, sys, v, a, part, ticket, out, kick);
+        if (kick && kicked) *kicked = true;
+    } else if (wide) {
+        if (lfs) launch_wide<true>(sys, v, a, part, ticket, out, kick);
+        else launch_wide<false>(sys, v, a, part, ticket, out, kick);
         if (kick && kicked) *kicked = true;
     } else {
         // the default gathered shape also takes the closing half-kick when asked

@@ -76,6 +76,52 @@ __device__ __forceinline__ void min_image_wrapped(const Fold3& f, double ax, dou
     dz = fold_wrapped(__dsub_rn(az, bz), f.b[2]);
 }
 
+// The same displacement for a pair in either order: a - b folded with the rounding of the
+// reference's order (lower index first; lo: a is the lower), as seen from a.  Away from
+// half a box length folding is odd in v bit for bit, so only the general fold needs the
+// order; a high-word compare settles the usual case off the FP64 pipe.
+static __device__ __noinline__ double fold_exact_call(double v, double L, double invL) {
+    return fold_exact(v, L, invL);
+}
+
+__device__ __forceinline__ double fold_pair(double v, const FoldBounds& b, bool lo) {
+    if ((__double2hiint(v) & 0x7fffffff) < __double2hiint(b.lo)) return v;
+    const double a = fabs(v);
+    if (a >= b.hi && a <= b.top) return v > 0.0 ? __dsub_rn(v, b.L) : __dadd_rn(v, b.L);
+    return lo ? fold_exact_call(v, b.L, b.invL) : -fold_exact_call(-v, b.L, b.invL);
+}
+
+__device__ __forceinline__ void min_image_pair(const Fold3& f, const double4& a, const double4& b,
+                                               bool lo, double& dx, double& dy, double& dz) {
+    dx = fold_pair(__dsub_rn(a.x, b.x), f.b[0], lo);
+    dy = fold_pair(__dsub_rn(a.y, b.y), f.b[1], lo);
+    dz = fold_pair(__dsub_rn(a.z, b.z), f.b[2], lo);
+}
+
+// Quotients that share a divisor.  reciprocal() is Newton's iteration y += y (1 - b y) from
+// the hardware's approximation (PTX rcp.approx.ftz.f64, about 20 bits), twice; quotient()
+// is Markstein's division (P. Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): q = a y, then q + y (a - b q)
+// with the remainder exact in one fused multiply-add, the correctly rounded a / b.  An
+// IEEE division has a latency of 126 clocks and costs 12 multiply-adds of throughput
+// here, a shared reciprocal 4 and each quotient 3.  For divisors with divides_fast().
+__device__ __forceinline__ double reciprocal(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = fma(y, fma(-b, y, 1.0), y);
+    return fma(y, fma(-b, y, 1.0), y);
+}
+
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return fma(y, fma(-b, q, a), q);
+}
+
+// 2^-100 <= b < 2^400: nothing on the way under- or overflows for ordinary a.
+__device__ __forceinline__ bool divides_fast(double b) {
+    return static_cast<unsigned>(__double2hiint(b)) - 0x39b00000u < 0x58f00000u - 0x39b00000u;
+}
+
 // Minimum-image displacement r_a - r_b with the reference's operation order.
 __device__ __forceinline__ void min_image_exact(const Box3& b, double ax, double ay, double az,
                                                 double bx, double by, double bz, double& dx,
@@ -110,34 +156,16 @@ __device__ __forceinline__ int4 quantize_position(const double4& p, double sx, d
                      static_cast<int>(p.w));
 }
 
-// Deterministic grid reduction of K doubles per thread.  Each block reduces its
-// values with a fixed shuffle tree and writes part[block*K + k]; the last block
-// to arrive (atomic ticket) re-reduces all partials in block order and writes
-// out[k], then resets the ticket.  With `status`, a non-finite sum (an atom that
-// blew up) also sets MD_STATUS_NONFINITE there.  Must be called by every thread
-// of the block; blockDim.x must be a multiple of 32 and <= 1024.  Returns true in
-// the last block.  The block index and count are explicit: a batched launch that
-// runs many systems gives each system's blocks their own rank and count.
-template <int K>
-__device__ bool grid_reduce_at(double (&v)[K], double* part, unsigned* ticket, double* out,
-                               uint32_t* status, unsigned block, unsigned nblocks) {
-    __shared__ double sm[K][32];
+// The end of a grid reduction: the last block to arrive (atomic ticket) sums
+// partial(p, k) over p < parts in a fixed order -- thread t the partials t, t +
+// blockDim.x, ..., then a shuffle tree -- writes out[k] and resets the ticket.  sm is
+// shared memory free since the block's last barrier.
+template <int K, class Partial>
+__device__ __forceinline__ bool grid_reduce_tail(double (&sm)[K][32], unsigned parts,
+                                                 unsigned* ticket, double* out, uint32_t* status,
+                                                 unsigned nblocks, Partial partial) {
     __shared__ bool is_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        const double s = warp_sum(v[k]);
-        if (lane == 0) sm[k][warp] = s;
-    }
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            double s = lane < nw ? sm[k][lane] : 0.0;
-            s = warp_sum(s);
-            if (lane == 0) part[static_cast<size_t>(block) * K + k] = s;
-        }
-    }
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned t = atomicAdd(ticket, 1u);
@@ -149,9 +177,9 @@ __device__ bool grid_reduce_at(double (&v)[K], double* part, unsigned* ticket, d
     double acc[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0;
-    for (unsigned b = threadIdx.x; b < nblocks; b += blockDim.x) {
+    for (unsigned p = threadIdx.x; p < parts; p += blockDim.x) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) acc[k] += __ldcg(part + static_cast<size_t>(b) * K + k);
+        for (int k = 0; k < K; ++k) acc[k] += partial(p, k);
     }
     __syncthreads();
 #pragma unroll
@@ -173,6 +201,38 @@ __device__ bool grid_reduce_at(double (&v)[K], double* part, unsigned* ticket, d
     }
     if (threadIdx.x == 0) *ticket = 0u;
     return true;  // this was the last block: `out` holds the sums
+}
+
+// Deterministic grid reduction of K doubles per thread.  Each block reduces its
+// values with a fixed shuffle tree and writes part[block*K + k]; the last block
+// to arrive re-reduces all partials in block order and writes out[k].  With
+// `status`, a non-finite sum (an atom that blew up) also sets MD_STATUS_NONFINITE
+// there.  Must be called by every thread
+// of the block; blockDim.x must be a multiple of 32 and <= 1024.  Returns true in
+// the last block.  The block index and count are explicit: a batched launch that
+// runs many systems gives each system's blocks their own rank and count.
+template <int K>
+__device__ bool grid_reduce_at(double (&v)[K], double* part, unsigned* ticket, double* out,
+                               uint32_t* status, unsigned block, unsigned nblocks) {
+    __shared__ double sm[K][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double s = warp_sum(v[k]);
+        if (lane == 0) sm[k][warp] = s;
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            double s = lane < nw ? sm[k][lane] : 0.0;
+            s = warp_sum(s);
+            if (lane == 0) part[static_cast<size_t>(block) * K + k] = s;
+        }
+    }
+    return grid_reduce_tail<K>(sm, nblocks, ticket, out, status, nblocks, [=](unsigned p, int k) {
+        return __ldcg(part + static_cast<size_t>(p) * K + k);
+    });
 }
 
 template <int K>
