@@ -411,7 +411,8 @@ int md_adjoint_backward(md_adjoint* a, const double* grad_rows, double grad_thet
         const int64_t k0 = sg * every, k1 = std::min(steps, k0 + every), len = k1 - k0;
         // recompute the segment from its checkpoint, keeping every state
         const double4* ckp = a->ck.as<double4>() + 2 * n * sg;
-        k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
+        sys->wrapped = false;
+    k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
         MDB_TRY(segment_start(a));
         double4* snap = a->snap.as<double4>();
         k_snapshot<<<g, kBlock, 0, ctx->stream>>>(sys->cur, n, snap, snap + n);
@@ -453,7 +454,8 @@ int md_adjoint_backward(md_adjoint* a, const double* grad_rows, double grad_thet
     {
         // leave the system where the forward left it (forces too)
         const double4* ckp = a->ck.as<double4>() + 2 * n * nseg;
-        k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
+        sys->wrapped = false;
+    k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
         ++ctx->launches;
         MDB_TRY(verlet_build(a->list, sys, false));
         MDB_TRY(lj_forces_verlet_async(&a->lj, sys, a->list));

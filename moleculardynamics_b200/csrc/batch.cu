@@ -245,7 +245,7 @@ int md_batch_run(md_batch* b, int64_t steps, double* thermo) {
     for (auto& r : b->reps) {
         MDB_TRY(verlet_ensure_ready(r.list, r.sys, "md_batch_run"));
         if (r.sys->n == 0) return fail(MD_ERR_INVALID_ARGUMENT, "md_batch_run: empty replica");
-        verlet_halo_for_run(r.list, r.sys, r.lj);
+        verlet_halo_for_run(r.list, r.sys, r.lj, true);
     }
     MDB_CUDA(cudaSetDevice(b->device));
     if (b->runs.size() != nr) {

@@ -600,6 +600,7 @@ int spce_step_async(SpceLoop& L, bool first, double* row) {
     md_context* ctx = sys->ctx;
     if (L.nhc) MDB_TRY(nhc_pre_async(it, ctx, first ? ctx_result(ctx, kResKE) : nullptr));
     if (L.nmol > 0) {
+        sys->wrapped = false;  // molecules keep their own image
         k_cvv_pre<<<grid_for(L.nmol, kBlock), kBlock, 0, ctx->stream>>>(
             sys->cur, sys->slot, L.nmol, cvv_args(it, sys), L.nhc, it->counters.as<int>(),
             ctx->d_status);
@@ -676,6 +677,7 @@ int constrained_pre_force(md_integrator* it, md_system* sys) {
         MDB_TRY(nhc_pre_async(it, ctx, ctx_result(ctx, kResKE)));
     }
     if (nmol > 0) {
+        sys->wrapped = false;  // molecules keep their own image
         k_cvv_pre<<<grid_for(nmol, kBlock), kBlock, 0, ctx->stream>>>(
             sys->cur, sys->slot, nmol, cvv_args(it, sys), nhc, it->counters.as<int>(), ctx->d_status);
         ++ctx->launches;
@@ -774,6 +776,7 @@ int md_rigid_constrain_positions(md_rigid* rw, md_system* sys, const double* rx,
     MDB_CUDA(cudaMemcpyAsync(d + 2 * n, rz, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
     MDB_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(int), ctx->stream));
     if (nmol > 0) {
+        sys->wrapped = false;
         k_shake<<<grid_for(nmol, kBlock), kBlock, 0, ctx->stream>>>(
             sys->cur, sys->slot, nmol, d, d + n, d + 2 * n, rigid_args(*rw), box_of(sys),
             cnt.as<int>(), ctx->d_status);

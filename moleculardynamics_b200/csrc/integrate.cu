@@ -415,6 +415,7 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         else k_kick_drift<false><<<kd, kBlock, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
         ctx_time_end(ctx, MD_KERNEL_INTEGRATE);
     }
+    sys->wrapped = true;
     ++ctx->launches;
     MDB_CHECK_LAUNCH();
     return MD_OK;
@@ -1084,7 +1085,7 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
     if (it->kind >= 3)
         return fail(MD_ERR_INVALID_ARGUMENT, "md_run_lj: constrained integrators run with md_run_spce");
     md_context* ctx = sys->ctx;
-    verlet_halo_for_run(v, sys, lj);
+    verlet_halo_for_run(v, sys, lj, false);
     // Thermo rows persist on the integrator (a captured step graph writes them at a
     // device-held index), grown in powers of two so that calls of similar length
     // keep the same buffer.

@@ -65,7 +65,7 @@ __device__ __forceinline__ PairTerms pair_terms(const LJArgs& a, double r2, Div 
     const double s6 = __dmul_rn(__dmul_rn(s2, s2), s2);
     const double s12 = __dmul_rn(s6, s6);
     t.u = __dmul_rn(a.four_eps, __dsub_rn(s12, s6));
-    t.w = __dmul_rn(a.tf_eps, __dsub_rn(__dmul_rn(2.0, s12), s6));  // (2 s6) s6 = 2 s12 exactly
+    t.w = __dmul_rn(a.tf_eps, fma(2.0, s12, -s6));  // (2 s6) s6 = 2 s12 exactly
     if (LFS) {
         const double r = __dsqrt_rn(r2);
         t.u = __dsub_rn(__dsub_rn(t.u, a.uc), __dmul_rn(__dsub_rn(r, a.rc), a.dudrc));
@@ -747,6 +747,166 @@ k_lj_halo(const int4* __restrict__ q, const double4* __restrict__ pd, const int*
     }
 }
 
+__device__ __forceinline__ unsigned smem_u32(const void* p) {
+    return static_cast<unsigned>(__cvta_generic_to_shared(p));
+}
+
+// A row of a tile that was not staged, walked as k_lj_verlet's FP64 path walks it.
+struct ExactSums {
+    double fx, fy, fz, e, vir;
+};
+
+template <bool LFS>
+__device__ __noinline__ ExactSums gathered_row_exact(LJArgs a, Box3 box,
+                                                     const double4* __restrict__ pos,
+                                                     const int* __restrict__ row, int cnt, int g,
+                                                     double4 pi) {
+    ExactSums acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+    const Fold3 f3 = fold3_of(box);
+    for (int k = g; k < cnt; k += kBlock / kHaloAtoms)
+        accumulate_exact<LFS>(a, f3, pi, ldg4(pos + __ldg(row + k)), acc.fx, acc.fy, acc.fz, acc.e,
+                              acc.vir);
+    return acc;
+}
+
+// FP64 forces over halo tiles: k_lj_halo's staging (here whole double4 positions, x and y,
+// then z and the original index, in two arrays that a row's byte offsets of 16-byte slots
+// address) and its walk of the row, with the reference arithmetic of k_lj_verlet in the
+// same order, so forces, energy and virial are that kernel's bit for bit.  The gathered
+// kernel is bound by its two 16-byte gathers an entry through L1/TEX; from shared memory an
+// entry costs some 20 wavefronts a warp instead of 64.  The terms of an entry are formed
+// without a branch on the cutoff (a warp nearly always holds a pair inside it), so entries
+// overlap.  1,048,576-atom liquid, kick included: 606 us with two IEEE divisions a pair,
+// 525 us with the shared reciprocal, 397 us from tiles (two entries side by side, or their
+// loads ahead of the arithmetic of four, spill past 80 registers: 467 to 530 us).
+// Wrapped coordinates only.  A list with cells has three of them a side, so a pair near
+// half a box length is beyond the cutoff whichever way it folds.
+constexpr int kHalo64Cap = 2304;  // slots: three blocks per SM; tiles with more gather
+
+template <bool LFS, bool KICK>
+__global__ void __launch_bounds__(kBlock, 3)
+k_lj_halo64(const double4* __restrict__ pos, const int* __restrict__ nbr,
+            const uint16_t* __restrict__ nbr16, const int* __restrict__ count, int stride, int64_t n,
+            const int2* __restrict__ runs, const int2* __restrict__ meta, Box3 box, LJArgs a,
+            double* __restrict__ fxo, double* __restrict__ fyo, double* __restrict__ fzo,
+            double* part, unsigned* ticket, double* out, KickArgs kick) {
+    constexpr int TPA = kBlock / kHaloAtoms;
+    extern __shared__ char s_xyzw[];  // double2 (x, y)[kHalo64Cap], double2 (z, w)[kHalo64Cap]
+    constexpr unsigned kZW = kHalo64Cap * sizeof(double2);
+    __shared__ int s_beg[kHaloRuns + 1], s_base[kHaloRuns + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int2 m = meta[blockIdx.x];
+    const bool staged = m.x > 0 && m.y <= kHalo64Cap;
+    if (staged) {
+        if (tid < m.x) {
+            const int2 r = runs[static_cast<int64_t>(blockIdx.x) * kHaloRuns + tid];
+            s_beg[tid] = r.x;
+            s_base[tid] = r.y;
+        }
+        if (tid == 0) s_base[m.x] = m.y;
+        __syncthreads();
+        const unsigned tile = smem_u32(s_xyzw);
+        for (int t = warp; t < m.x; t += kBlock / 32) {
+            const double4* src = pos + s_beg[t];
+            const int base = s_base[t], len = s_base[t + 1] - base;
+            for (int k = lane; k < len; k += 32) {
+                const unsigned slot = tile + 16u * static_cast<unsigned>(base + k);
+                const char* s = reinterpret_cast<const char*>(src + k);
+                asm volatile(
+                    "cp.async.cg.shared.global [%0], [%2], 16;\n"
+                    "cp.async.cg.shared.global [%1], [%3], 16;\n" ::"r"(slot),
+                    "r"(slot + kZW), "l"(s), "l"(s + 16)
+                    : "memory");
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+    }
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * kHaloAtoms + tid / TPA;
+    const int g = tid % TPA;
+    ExactSums acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (i < n) {
+        const double4 pi = ldg4(pos + i);
+        const int cnt = min(count[i], stride);  // an overflowed row is flagged, never over-read
+        if (staged) {
+            const uint4* rowv = reinterpret_cast<const uint4*>(nbr16 + i * stride);
+            const unsigned sel = g ? 0x4432u : 0x4410u;  // this thread's 16-bit halves
+            const Fold3 f3 = fold3_of(box);
+            const auto fold = [](double v, const FoldBounds& b) {
+                if ((__double2hiint(v) & 0x7fffffff) < __double2hiint(b.lo)) return v;
+                return v > 0.0 ? __dsub_rn(v, b.L) : __dadd_rn(v, b.L);
+            };
+            const auto pair = [&](unsigned word, bool live) {
+                const unsigned off = __byte_perm(word, 0u, sel);
+                const double2 xy = *reinterpret_cast<const double2*>(s_xyzw + off);
+                const double2 zw = *reinterpret_cast<const double2*>(s_xyzw + kZW + off);
+                const double dx = fold(__dsub_rn(pi.x, xy.x), f3.b[0]);
+                const double dy = fold(__dsub_rn(pi.y, xy.y), f3.b[1]);
+                const double dz = fold(__dsub_rn(pi.z, zw.x), f3.b[2]);
+                const double r2 = norm2_exact(dx, dy, dz);
+                const bool in = r2 < a.rc2 && live;
+                const double y = reciprocal(r2);
+                PairTerms p = pair_terms<LFS>(a, r2, [r2, y](double x) { return quotient(x, r2, y); });
+                // below 2^-100 (rc^2 is below 2^400 on this path): as pair_exact
+                if (in && __double2hiint(r2) < 0x39b00000)
+                    p = pair_terms_ieee<LFS>(a.sig2, a.four_eps, a.tf_eps, a.rc, a.uc, a.dudrc, r2);
+                if (in) {
+                    acc.fx = __dadd_rn(acc.fx, __dmul_rn(dx, p.s));
+                    acc.fy = __dadd_rn(acc.fy, __dmul_rn(dy, p.s));
+                    acc.fz = __dadd_rn(acc.fz, __dmul_rn(dz, p.s));
+                }
+                if (in && pi.w < zw.y) {
+                    acc.e = __dadd_rn(acc.e, p.u);
+                    acc.vir = __dadd_rn(acc.vir, p.w);
+                }
+            };
+            const int nch = (cnt + 7) >> 3;
+            uint4 cur = nch > 0 ? __ldg(rowv) : make_uint4(0u, 0u, 0u, 0u);
+            for (int c = 0; c < nch; ++c) {  // a last chunk's padding is the atom's own slot
+                const uint4 nxt = c + 1 < nch ? __ldg(rowv + c + 1) : cur;
+                const int left = cnt - 8 * c - g;
+                pair(cur.x, left > 0);
+                pair(cur.y, left > 2);
+                pair(cur.z, left > 4);
+                pair(cur.w, left > 6);
+                cur = nxt;
+            }
+        } else {
+            acc = gathered_row_exact<LFS>(a, box, pos, nbr + i * stride, cnt, g, pi);
+        }
+    }
+    double fx = acc.fx, fy = acc.fy, fz = acc.fz;
+#pragma unroll
+    for (int o = TPA / 2; o > 0; o >>= 1) {
+        fx += __shfl_xor_sync(0xffffffffu, fx, o);
+        fy += __shfl_xor_sync(0xffffffffu, fy, o);
+        fz += __shfl_xor_sync(0xffffffffu, fz, o);
+    }
+    double ke = 0.0;
+    if (i < n && g == 0) {
+        fxo[i] = fx;
+        fyo[i] = fy;
+        fzo[i] = fz;
+        if constexpr (KICK) {  // the closing half-kick, as the separate kick kernel does it
+            const double c = __dmul_rn(kick.half_dt, kick.inv_mass[i]);
+            const double vx = fma(c, fx, kick.vx[i]);
+            const double vy = fma(c, fy, kick.vy[i]);
+            const double vz = fma(c, fz, kick.vz[i]);
+            kick.vx[i] = vx;
+            kick.vy[i] = vy;
+            kick.vz[i] = vz;
+            ke = 0.5 * kick.mass[i] * (vx * vx + vy * vy + vz * vz);
+        }
+    }
+    if constexpr (KICK) {
+        double v[3] = {acc.e, acc.vir, ke};
+        grid_reduce<3>(v, part, ticket, out, kick.status);
+    } else {
+        double v[2] = {acc.e, acc.vir};
+        grid_reduce<2>(v, part, ticket, out);
+    }
+}
+
 // ------------------------------------------------------------ k_lj_tile
 // Mixed-precision forces over halo tiles, persistent and double-buffered (cubic
 // boxes).  Each CTA walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ...: while
@@ -765,10 +925,6 @@ k_lj_halo(const int4* __restrict__ q, const double4* __restrict__ pd, const int*
 // read without a count test.  Pairs within the cutoff band are settled by the
 // reference arithmetic on the FP64 positions, as in the gathered kernel.
 constexpr long long kTileWaitCycles = 2000000000LL;  // ~1 s bound on a tile's copies
-
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
@@ -1407,6 +1563,19 @@ void launch_halo(md_system* sys, md_verlet* v, const LJArgs& a, double* part, un
         kick ? *kick : KickArgs{});
 }
 
+template <bool LFS>
+int launch_halo64(md_system* sys, md_verlet* v, const LJArgs& a, double* part, unsigned* ticket,
+                  double* out, const KickArgs* kick) {
+    auto kernel = kick ? k_lj_halo64<LFS, true> : k_lj_halo64<LFS, false>;
+    constexpr int kBytes = 2 * kHalo64Cap * sizeof(double2);
+    MDB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes));
+    kernel<<<static_cast<unsigned>(halo_blocks(sys->n)), kBlock, kBytes, sys->ctx->stream>>>(
+        sys->cur.pos, v->nbr.as<int>(), v->nbr16.as<uint16_t>(), v->count.as<int>(), v->stride,
+        sys->n, v->halo_runs.as<int2>(), v->halo_meta.as<int2>(), box_of(sys), a, sys->cur.fx,
+        sys->cur.fy, sys->cur.fz, part, ticket, out, kick ? *kick : KickArgs{});
+    return MD_OK;
+}
+
 UnitConst unit_const(const LJArgs& a) {
     UnitConst c;
     const double res2 = a.res2;
@@ -1555,10 +1724,15 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
     if (!q_current) MDB_TRY(lj_quantize_async(lj, sys, q_gate));
     // halo tiles, when the list keeps them (fused runs of large systems turn them on,
     // or md_verlet_set_halo)
-    const bool halo = mixed && lj->halo && sys->n > 0 && v->halo_on && v->stride % 8 == 0;
+    const bool halo = lj->halo && sys->n > 0 && v->halo_on && v->stride % 8 == 0 &&
+                      (mixed || (sys->wrapped && a.rc2 < 0x1p400));
     ctx_time_begin(ctx, MD_KERNEL_LJ_FORCE);
     const bool cubic = a.res[0] == a.res[1] && a.res[0] == a.res[2];
-    if (halo && cubic && lj->tile_tpa > 1) {
+    if (halo && !mixed) {
+        if (lfs) MDB_TRY(launch_halo64<true>(sys, v, a, part, ticket, out, kick));
+        else MDB_TRY(launch_halo64<false>(sys, v, a, part, ticket, out, kick));
+        if (kick && kicked) *kicked = true;
+    } else if (halo && cubic && lj->tile_tpa > 1) {
         if (lfs) launch_tile<true>(lj->tile_tpa, sys, v, a, part, ticket, out);
         else launch_tile<false>(lj->tile_tpa, sys, v, a, part, ticket, out);
     } else if (halo && cubic && lj->tile_tpa == 1) {

@@ -156,6 +156,9 @@ struct md_system {
     bool has_molecules = false;  // molecule ids differ from the atom's own index
     uint64_t mol_version = 1;    // bumped whenever molecule ids are set
     double last_energy = 0.0, last_virial = 0.0;
+    // Every coordinate lies in the box: the last kernel to write positions wrapped them (the
+    // unconstrained integrators), nothing set them since.
+    bool wrapped = false;
     // Fixed-point copy of the positions for the mixed-precision pair kernel: per
     // axis the box length maps to 2^32, so x, y, z are int32 (w = original index)
     // and one 16-byte load fetches a neighbour; written before each mixed launch.
@@ -320,12 +323,17 @@ constexpr int kHaloSpan = 16;
 // The choice depends on the list and the force field only, never on the length of
 // one call, so short and long runs of the same system step with the same kernels.
 constexpr int64_t kHaloMinAtoms = 65536;
+// FP64: at 108,000 atoms tiles save 3 of 83 us a step and cost 50 us a rebuild, at 256,000
+// atoms 19 of 154 us against 65, at 1,048,576 atoms 125 of 523 us against 257 (a rebuild
+// every seven steps or so).
+constexpr int64_t kHaloMinAtoms64 = 196608;
 inline int64_t halo_blocks(int64_t n) { return (n + kHaloAtoms - 1) / kHaloAtoms; }
 // Turns the halo tiles on for this list (built right away from the current list
 // unless the stream is capturing); false when they cannot be used.
 bool verlet_halo_ready(md_verlet* v, md_system* sys);
-// The fused-run policy above, for a mixed-precision LJ force field.
-void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj);
+// The fused-run policy above, for an LJ force field (batch: of a batch's replica, whose FP64
+// pass gathers with all the others').
+void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj, bool batch);
 int verlet_build(md_verlet* v, md_system* sys, bool conditional);
 int verlet_check(md_verlet* v, md_system* sys);  // device flag <- needs rebuild
 int verlet_ensure_capacity(md_verlet* v, md_system* sys);

@@ -1224,8 +1224,9 @@ bool verlet_halo_ready(md_verlet* v, md_system* sys) {
     return true;
 }
 
-void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj) {
-    if (lj->precision == MD_PRECISION_MIXED && lj->halo && sys->n >= kHaloMinAtoms)
+void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj, bool batch) {
+    const bool mixed = lj->precision == MD_PRECISION_MIXED;
+    if (lj->halo && (mixed ? sys->n >= kHaloMinAtoms : !batch && sys->n >= kHaloMinAtoms64))
         verlet_halo_ready(v, sys);
 }
 

@@ -296,6 +296,7 @@ int md_system_set(md_system* sys, int field, const double* src) {
     if (field < MD_FIELD_X || field > MD_FIELD_CHARGE)
         return fail(MD_ERR_INVALID_ARGUMENT, "md_system_set: unknown field %d", field);
     if (sys->n == 0) return MD_OK;
+    if (field <= MD_FIELD_Z) sys->wrapped = false;
     md_context* ctx = sys->ctx;
     void* staging;
     MDB_TRY(ctx_scratch(ctx, static_cast<size_t>(sys->n) * sizeof(double), &staging));
@@ -335,6 +336,8 @@ int md_system_set_fields(md_system* sys, int count, const int* fields, const dou
         if (fields[k] < MD_FIELD_X || fields[k] > MD_FIELD_CHARGE || !src[k])
             return fail(MD_ERR_INVALID_ARGUMENT, "md_system_set_fields: bad field %d", k);
     if (sys->n == 0 || count == 0) return MD_OK;
+    for (int k = 0; k < count; ++k)
+        if (fields[k] <= MD_FIELD_Z) sys->wrapped = false;
     md_context* ctx = sys->ctx;
     const size_t col = static_cast<size_t>(sys->n);
     void* staging;
