@@ -25,6 +25,13 @@ namespace {
 
 constexpr int kBlock = 256;
 
+// Where a fused run stands, on the device: a captured step cannot carry a step number.
+struct RunCursor {
+    int done;  // steps recorded (the next thermo row)
+    int pad;
+    uint64_t first;  // the integrator's step counter when the run began
+};
+
 struct StepArgs {
     Box3 box;
     double dt, half_dt;
@@ -32,6 +39,7 @@ struct StepArgs {
     double c1, c2, temperature;
     uint32_t key0, key1;
     uint64_t step;
+    const RunCursor* run;  // a replayed graph's step: run->first + run->done instead of step
     const double* noise;  // replayed normals for this step (original order), or null
     uint32_t* status;     // MD_STATUS_NONFINITE when a position stops being finite
     int4* q;              // fixed-point copy of the new positions for the mixed force, or null
@@ -138,11 +146,12 @@ __global__ void k_baoab_pre(md_atoms a, int64_t n, StepArgs s, DispArgs d) {
             x1 = s.noise[3 * static_cast<int64_t>(o) + 1];
             x2 = s.noise[3 * static_cast<int64_t>(o) + 2];
         } else {
-            const U4 r0 = philox4x32_10(U4{static_cast<uint32_t>(o), 0u, static_cast<uint32_t>(s.step),
-                                           static_cast<uint32_t>(s.step >> 32)},
+            const uint64_t step = s.run ? s.run->first + static_cast<uint64_t>(s.run->done) : s.step;
+            const U4 r0 = philox4x32_10(U4{static_cast<uint32_t>(o), 0u, static_cast<uint32_t>(step),
+                                           static_cast<uint32_t>(step >> 32)},
                                         s.key0, s.key1);
-            const U4 r1 = philox4x32_10(U4{static_cast<uint32_t>(o), 1u, static_cast<uint32_t>(s.step),
-                                           static_cast<uint32_t>(s.step >> 32)},
+            const U4 r1 = philox4x32_10(U4{static_cast<uint32_t>(o), 1u, static_cast<uint32_t>(step),
+                                           static_cast<uint32_t>(step >> 32)},
                                         s.key0, s.key1);
             double x3;
             normal2(r0, x0, x1);
@@ -161,6 +170,7 @@ __global__ void k_baoab_pre(md_atoms a, int64_t n, StepArgs s, DispArgs d) {
         a.vx[k] = vx;
         a.vy[k] = vy;
         a.vz[k] = vz;
+        if (s.q) s.q[k] = quantize_position(p, s.qs[0], s.qs[1], s.qs[2]);
         if (CHECK) a1 = disp2(f3, p, d.ref[k]);
     }
     if (CHECK) top2_grid(a1, 0.0, d);
@@ -348,6 +358,7 @@ StepArgs step_args(const md_integrator* it, const md_system* sys) {
     s.key0 = static_cast<uint32_t>(it->seed);
     s.key1 = static_cast<uint32_t>(it->seed >> 32);
     s.step = it->step;
+    s.run = nullptr;
     s.noise = nullptr;
     s.status = sys->ctx->d_status;
     s.q = nullptr;
@@ -369,17 +380,16 @@ NhcState* nhc_of(md_integrator* it) {
 // fresh_ke: the chain half of a Nose-Hoover step sums the kinetic energy of the
 // current velocities; otherwise it uses the value the chain tracked through the
 // previous step's rescalings (fused loops, after their first step).
-// q: also write the fixed-point positions for a mixed-precision force (kick/drift
-// integrators only; pre_force_quantizes says whether it does).
-bool pre_force_quantizes(const md_integrator* it) { return it->kind != 1; }
-
+// q: also write the fixed-point positions for a mixed-precision force.  run: a captured
+// step takes its step number from there (a Langevin step's noise depends on it).
 int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke = true,
-              int4* q = nullptr) {
+              int4* q = nullptr, const RunCursor* run = nullptr) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
     if (n == 0) return MD_OK;
     StepArgs s = step_args(it, sys);
-    if (q && pre_force_quantizes(it)) {
+    s.run = run;
+    if (q) {
         s.q = q;
         for (int d = 0; d < 3; ++d) s.qs[d] = 4294967296.0 / sys->box[d];
     }
@@ -399,7 +409,7 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         }
         if (check) k_baoab_pre<true><<<blocks, kBlock, 0, ctx->stream>>>(sys->cur, n, s, d);
         else k_baoab_pre<false><<<blocks, kBlock, 0, ctx->stream>>>(sys->cur, n, s, d);
-        ++it->step;
+        if (!run) ++it->step;  // a replay's steps are counted by the run
     } else {
         NhcState* nhc = nhc_of(it);
         if (nhc) {
@@ -537,12 +547,11 @@ int record_at_async(md_context* ctx, const NhcState* nhc, double* rows, int* idx
     return MD_OK;
 }
 
-// The fixed-point position buffer the step's kick/drift fills for a mixed force
-// (null when the force is FP64 or the integrator has no kick/drift kernel).
+// The fixed-point position buffer the step's first kernel fills for a mixed force (null
+// when the force is FP64).
 int step_quantize_target(md_integrator* it, md_system* sys, const md_lj* lj, int4** q) {
     *q = nullptr;
-    if (lj->precision != MD_PRECISION_MIXED || !pre_force_quantizes(it) || sys->n <= 0)
-        return MD_OK;
+    if (lj->precision != MD_PRECISION_MIXED || sys->n <= 0) return MD_OK;
     MDB_TRY(sys->qpos.ensure(sizeof(int4) * static_cast<size_t>(sys->n)));
     *q = sys->qpos.as<int4>();
     return MD_OK;
@@ -589,7 +598,7 @@ int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj*
     int4* q = nullptr;
     MDB_TRY(step_quantize_target(it, sys, lj, &q));  // allocated by the first, eager step
     rc = capture_into(ctx, graph, nullptr, 0, [&]() -> int {
-        MDB_TRY(pre_force(it, sys, v, false, q));
+        MDB_TRY(pre_force(it, sys, v, false, q, reinterpret_cast<const RunCursor*>(idx)));
         k_set_rebuild<<<1, 1, 0, ctx->stream>>>(h, v->d_rebuild_flag);
         ++ctx->launches;
         MDB_CHECK_LAUNCH();
@@ -1093,22 +1102,27 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
         size_t cap = 1024;
         while (cap < static_cast<size_t>(steps)) cap *= 2;
         MDB_TRY(it->run_rows.ensure(sizeof(double) * 4 * cap));
-        MDB_TRY(it->run_idx.ensure(sizeof(int)));
-        MDB_CUDA(cudaMemsetAsync(it->run_idx.ptr, 0, sizeof(int), ctx->stream));
-        if (!it->h_rebuilt) MDB_CUDA(cudaMallocHost(&it->h_rebuilt, 2 * sizeof(int)));
+        MDB_TRY(it->run_idx.ensure(sizeof(RunCursor)));
+        if (!it->h_rebuilt)
+            MDB_CUDA(cudaMallocHost(&it->h_rebuilt, sizeof(RunCursor) + 2 * sizeof(int)));
+        RunCursor* cursor = reinterpret_cast<RunCursor*>(it->h_rebuilt + 2);
+        *cursor = RunCursor{0, 0, it->step};
+        MDB_CUDA(cudaMemcpyAsync(it->run_idx.ptr, cursor, sizeof(RunCursor), cudaMemcpyHostToDevice,
+                                 ctx->stream));
     }
     double* rows = it->run_rows.as<double>();
     int* idx = it->run_idx.as<int>();
     NhcState* nhc = nhc_of(it);
-    // Steps replay one captured step graph when that is possible (BAOAB's noise
-    // counter is a host-side launch argument, so it never is).  The graph of an
+    // Steps replay one captured step graph when that is possible (replayed noise advances
+    // through a host-side pointer, so with it it is not).  The graph of an
     // earlier call is replayed while the system, list and force field are the same
     // handles and nothing has been allocated, freed, permuted or reconfigured since
     // (the graph epoch).  Otherwise the first step runs from the host -- it sizes
     // every buffer -- and the step is captured afterwards.  A chain's first step
     // always runs from the host: it sums the entry kinetic energy instead of using
     // the tracked value, which the caller may have changed between calls.
-    const bool want_graph = ctx->graphs && !ctx->timing && it->kind != 1 && steps >= 1 && sys->n > 0;
+    const bool want_graph = ctx->graphs && !ctx->timing && !(it->kind == 1 && it->noise.ptr) &&
+                            steps >= 1 && sys->n > 0;
     StepGraph* sg = static_cast<StepGraph*>(it->run_graph);
     const void* key[3] = {sys, v, lj};
     bool cached = want_graph && sg && sg->exec && it->run_epoch == graph_epoch() &&
@@ -1143,6 +1157,7 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
         MDB_CUDA(cudaMemcpyAsync(it->h_rebuilt + 1, v->d_rebuild_total, sizeof(int),
                                  cudaMemcpyDeviceToHost, ctx->stream));
         MDB_CUDA(cudaStreamSynchronize(ctx->stream));
+        if (it->kind == 1) it->step += static_cast<uint64_t>(graph_steps);
         ctx->launches += graph_steps * sg->main_launches +
                          static_cast<int64_t>(it->h_rebuilt[1] - it->h_rebuilt[0]) * sg->body_launches;
         k = steps;
