@@ -89,19 +89,33 @@ struct Mol {
     double x[3], y[3], z[3];
 };
 
+// min_image_wrapped of a bond: shorter than half the box, so only a molecule that straddles
+// its edge folds; one high-word compare per component finds that out.
+__device__ __forceinline__ void min_image_bond(const Fold3& f, const Mol& r, int i, int j, double& dx,
+                                               double& dy, double& dz) {
+    dx = fold_pair(__dsub_rn(r.x[i], r.x[j]), f.b[0], true);
+    dy = fold_pair(__dsub_rn(r.y[i], r.y[j]), f.b[1], true);
+    dz = fold_pair(__dsub_rn(r.z[i], r.z[j]), f.b[2], true);
+}
+
 // rigid_water.cpp:61-116 for one molecule.  Returns iterations, -1 (no
 // convergence) or -2 (singular denominator).
-// The reference bond vectors and the inverse-mass sums do not change during the
-// iterations; they are formed once, with the same operations, before the sweeps.
+// The reference bond vectors, the inverse-mass sums and the masses' reciprocals do not
+// change during the iterations; they are formed once before the sweeps.  A sweep is a chain
+// of dependent FP64 operations, three constraints one after another: its divisions (126
+// clocks each, two of the three in the chain) are quotients by shared or precomputed
+// reciprocals, correctly rounded like the divisions they replace.  1,029 sites at tolerance
+// 1e-12: 65 us with IEEE divisions and 256-thread blocks, 40 us so.
 __device__ int shake_molecule(Mol& r, const Mol& ref, const double m[3], const RigidArgs& a,
                               const Fold3& f3) {
     double b[3][3], two_inv_mass[3];
+    const double im[3] = {__ddiv_rn(1.0, m[0]), __ddiv_rn(1.0, m[1]), __ddiv_rn(1.0, m[2])};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const int i = cons_i(c), j = cons_j(c);
         min_image_wrapped(f3, ref.x[i], ref.y[i], ref.z[i], ref.x[j], ref.y[j], ref.z[j], b[c][0],
                           b[c][1], b[c][2]);
-        two_inv_mass[c] = __dmul_rn(2.0, __dadd_rn(__ddiv_rn(1.0, m[i]), __ddiv_rn(1.0, m[j])));
+        two_inv_mass[c] = __dmul_rn(2.0, __dadd_rn(im[i], im[j]));
     }
     for (int it = 0; it < a.max_iterations; ++it) {
         bool open = false;  // some violation above the tolerance (worst > tolerance)
@@ -110,15 +124,15 @@ __device__ int shake_molecule(Mol& r, const Mol& ref, const double m[3], const R
             const int i = cons_i(c), j = cons_j(c);
             const double d2 = a.target2[c];
             double ax, ay, az;
-            min_image_wrapped(f3, r.x[i], r.y[i], r.z[i], r.x[j], r.y[j], r.z[j], ax, ay, az);
+            min_image_bond(f3, r, i, j, ax, ay, az);
             const double s = __dsub_rn(norm2_exact(ax, ay, az), d2);
             if (fabs(s) > a.within[c]) open = true;
             if (fabs(s) <= a.within[c]) continue;
             const double bx = b[c][0], by = b[c][1], bz = b[c][2];
             const double denom = __dmul_rn(two_inv_mass[c], dot_exact(ax, ay, az, bx, by, bz));
             if (fabs(denom) < 1e-30) return -2;
-            const double g = __ddiv_rn(s, denom);
-            const double gi = __ddiv_rn(g, m[i]), gj = __ddiv_rn(g, m[j]);
+            const double g = quotient(s, denom, reciprocal(denom));
+            const double gi = quotient(g, m[i], im[i]), gj = quotient(g, m[j], im[j]);
             r.x[i] = __dsub_rn(r.x[i], __dmul_rn(bx, gi));
             r.y[i] = __dsub_rn(r.y[i], __dmul_rn(by, gi));
             r.z[i] = __dsub_rn(r.z[i], __dmul_rn(bz, gi));
@@ -279,17 +293,21 @@ __device__ __forceinline__ int constrain_positions(Mol& r, const Mol& ref, const
 
 // rigid_water.cpp:118-161 for one molecule.
 // Positions are fixed during the iterations: the bond vectors, their squared
-// lengths times the inverse-mass sums, are formed once before the sweeps.
+// lengths times the inverse-mass sums and the reciprocals the sweeps divide with are
+// formed once before them.  1,029 sites: 54 us with IEEE divisions (two in each
+// constraint's chain) and 256-thread blocks, 22 us so.
 __device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const RigidArgs& a,
                                const Fold3& f3) {
-    double b[3][3], mass_norm[3];
+    double b[3][3], mass_norm[3], inv_norm[3];
+    const double im[3] = {__ddiv_rn(1.0, m[0]), __ddiv_rn(1.0, m[1]), __ddiv_rn(1.0, m[2])};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const int i = cons_i(c), j = cons_j(c);
         min_image_wrapped(f3, r.x[i], r.y[i], r.z[i], r.x[j], r.y[j], r.z[j], b[c][0], b[c][1],
                           b[c][2]);
-        const double inv_mass_sum = __dadd_rn(__ddiv_rn(1.0, m[i]), __ddiv_rn(1.0, m[j]));
+        const double inv_mass_sum = __dadd_rn(im[i], im[j]);
         mass_norm[c] = __dmul_rn(inv_mass_sum, norm2_exact(b[c][0], b[c][1], b[c][2]));
+        inv_norm[c] = reciprocal(mass_norm[c]);
     }
     for (int it = 0; it < a.max_iterations; ++it) {
         bool open = false;  // some |r.v| / d2 above the tolerance
@@ -302,8 +320,8 @@ __device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const Ri
             const double rv = dot_exact(ax, ay, az, ux, uy, uz);
             if (fabs(rv) > a.within[c]) open = true;
             if (fabs(rv) <= a.within[c]) continue;
-            const double k = __ddiv_rn(rv, mass_norm[c]);
-            const double ki = __ddiv_rn(k, m[i]), kj = __ddiv_rn(k, m[j]);
+            const double k = quotient(rv, mass_norm[c], inv_norm[c]);
+            const double ki = quotient(k, m[i], im[i]), kj = quotient(k, m[j], im[j]);
             v.x[i] = __dsub_rn(v.x[i], __dmul_rn(ax, ki));
             v.y[i] = __dsub_rn(v.y[i], __dmul_rn(ay, ki));
             v.z[i] = __dsub_rn(v.z[i], __dmul_rn(az, ki));
@@ -462,6 +480,37 @@ __global__ void k_cvv_pre(md_atoms a, const int* __restrict__ slot, int64_t nmol
     store_vel(a, ms, v);
 }
 
+// The kinetic-energy sum of a launch of one-warp blocks, in the order and tree of a launch
+// of kBlock threads a block (grid_reduce there): four consecutive blocks are its four warps.
+__device__ __forceinline__ void warp_blocks_reduce(double v, double* part, unsigned* ticket,
+                                                   double* out) {
+    static_assert(kBlock == 128, "four warps a block");
+    const unsigned lane = threadIdx.x, nb = gridDim.x;
+    v = warp_sum(v);
+    unsigned t = 0;
+    if (lane == 0) {
+        part[blockIdx.x] = v;
+        __threadfence();
+        t = atomicAdd(ticket, 1u);
+    }
+    if (__shfl_sync(0xffffffffu, t, 0) != nb - 1) return;
+    __threadfence();
+    const auto at = [=](unsigned b) { return b < nb ? __ldcg(part + b) : 0.0; };
+    const unsigned parts = (nb + 3) / 4;
+    double s[4];
+#pragma unroll
+    for (unsigned w = 0; w < 4; ++w) {
+        double acc = 0.0;
+        for (unsigned p = 32 * w + lane; p < parts; p += kBlock)
+            acc += (at(4 * p) + at(4 * p + 2)) + (at(4 * p + 1) + at(4 * p + 3));
+        s[w] = warp_sum(acc);
+    }
+    if (lane == 0) {
+        *out = (s[0] + s[2]) + (s[1] + s[3]);
+        *ticket = 0u;
+    }
+}
+
 // constrained_velocity_verlet.hpp:54-56: kick; RATTLE; kinetic-energy sum.
 __global__ void __launch_bounds__(kBlock)
 k_cvv_post(md_atoms a, const int* __restrict__ slot, int64_t nmol, CvvArgs c, int* max_it,
@@ -491,7 +540,8 @@ k_cvv_post(md_atoms a, const int* __restrict__ slot, int64_t nmol, CvvArgs c, in
         for (int k = 0; k < 3; ++k)
             ke[0] += 0.5 * mass[k] * (v.x[k] * v.x[k] + v.y[k] * v.y[k] + v.z[k] * v.z[k]);
     }
-    grid_reduce<1>(ke, part, ticket, ke_out);
+    if (blockDim.x == 32) warp_blocks_reduce(ke[0], part, ticket, ke_out);
+    else grid_reduce<1>(ke, part, ticket, ke_out);
 }
 
 // SPC/E potential energy from the Ewald result slots (spce_forcefield.cpp:40):
@@ -520,6 +570,12 @@ CvvArgs cvv_args(const md_integrator* it, const md_system* sys) {
     c.ra = rigid_args(it->rigid);
     c.box = box_of(sys);
     return c;
+}
+
+// Threads per block of the molecule kernels: single warps while that spreads them over more
+// SMs (a warp's chain of FP64 operations leaves little for others to share), else kBlock.
+int mol_block(const md_context* ctx, int64_t nmol) {
+    return nmol <= 128 * static_cast<int64_t>(ctx->sm_count) ? 32 : kBlock;
 }
 
 int check_triples(const md_system* sys, const char* who) {
@@ -565,7 +621,7 @@ struct SpceLoop {
     md_ewald* ff = nullptr;
     NhcState* nhc = nullptr;
     int64_t nmol = 0;
-    int g = 1;
+    int g = 1, block = kBlock;  // grid and block of the molecule kernels
     double elrc = 0.0, self_coef = 0.0;
 };
 
@@ -586,7 +642,8 @@ int spce_loop_begin(md_integrator* it, md_system* sys, md_ewald* ff, const char*
     L.self_coef = -md_coulomb_prefactor() * alpha / std::sqrt(kPi);
     L.nhc = it->kind == 4 ? it->chain_state.as<NhcState>() : nullptr;
     L.nmol = sys->n / 3;
-    L.g = grid_for(std::max<int64_t>(L.nmol, 1), kBlock);
+    L.block = mol_block(sys->ctx, L.nmol);
+    L.g = grid_for(std::max<int64_t>(L.nmol, 1), L.block);
     if (L.nhc) MDB_TRY(system_kinetic_async(sys, kResKE));
     return MD_OK;
 }
@@ -601,7 +658,7 @@ int spce_step_async(SpceLoop& L, bool first, double* row) {
     if (L.nhc) MDB_TRY(nhc_pre_async(it, ctx, first ? ctx_result(ctx, kResKE) : nullptr));
     if (L.nmol > 0) {
         sys->wrapped = false;  // molecules keep their own image
-        k_cvv_pre<<<grid_for(L.nmol, kBlock), kBlock, 0, ctx->stream>>>(
+        k_cvv_pre<<<grid_for(L.nmol, L.block), L.block, 0, ctx->stream>>>(
             sys->cur, sys->slot, L.nmol, cvv_args(it, sys), L.nhc, it->counters.as<int>(),
             ctx->d_status);
         ++ctx->launches;
@@ -611,7 +668,7 @@ int spce_step_async(SpceLoop& L, bool first, double* row) {
                                            ctx_result(ctx, kResEnergy));
     double* part;  // fetched after the Ewald sum, which may grow the partials
     MDB_TRY(ctx_partials(ctx, static_cast<size_t>(L.g), &part));
-    k_cvv_post<<<L.g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, L.nmol, cvv_args(it, sys),
+    k_cvv_post<<<L.g, L.block, 0, ctx->stream>>>(sys->cur, sys->slot, L.nmol, cvv_args(it, sys),
                                                it->counters.as<int>() + 1, ctx->d_status, part,
                                                ctx_counter(ctx, 8), ctx_result(ctx, kResKE));
     ctx->launches += 2;
@@ -677,8 +734,9 @@ int constrained_pre_force(md_integrator* it, md_system* sys) {
         MDB_TRY(nhc_pre_async(it, ctx, ctx_result(ctx, kResKE)));
     }
     if (nmol > 0) {
+        const int block = mol_block(ctx, nmol);
         sys->wrapped = false;  // molecules keep their own image
-        k_cvv_pre<<<grid_for(nmol, kBlock), kBlock, 0, ctx->stream>>>(
+        k_cvv_pre<<<grid_for(nmol, block), block, 0, ctx->stream>>>(
             sys->cur, sys->slot, nmol, cvv_args(it, sys), nhc, it->counters.as<int>(), ctx->d_status);
         ++ctx->launches;
         MDB_CHECK_LAUNCH();
@@ -690,10 +748,10 @@ int constrained_post_force(md_integrator* it, md_system* sys, bool apply_scale) 
     MDB_TRY(ensure_counters(it));
     md_context* ctx = sys->ctx;
     const int64_t nmol = sys->n / 3;
-    const int g = grid_for(std::max<int64_t>(nmol, 1), kBlock);
+    const int block = mol_block(ctx, nmol), g = grid_for(std::max<int64_t>(nmol, 1), block);
     double* part;
     MDB_TRY(ctx_partials(ctx, static_cast<size_t>(g), &part));
-    k_cvv_post<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, nmol, cvv_args(it, sys),
+    k_cvv_post<<<g, block, 0, ctx->stream>>>(sys->cur, sys->slot, nmol, cvv_args(it, sys),
                                              it->counters.as<int>() + 1, ctx->d_status, part,
                                              ctx_counter(ctx, 8), ctx_result(ctx, kResKE));
     ++ctx->launches;
@@ -776,8 +834,9 @@ int md_rigid_constrain_positions(md_rigid* rw, md_system* sys, const double* rx,
     MDB_CUDA(cudaMemcpyAsync(d + 2 * n, rz, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
     MDB_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(int), ctx->stream));
     if (nmol > 0) {
+        const int block = mol_block(ctx, nmol);
         sys->wrapped = false;
-        k_shake<<<grid_for(nmol, kBlock), kBlock, 0, ctx->stream>>>(
+        k_shake<<<grid_for(nmol, block), block, 0, ctx->stream>>>(
             sys->cur, sys->slot, nmol, d, d + n, d + 2 * n, rigid_args(*rw), box_of(sys),
             cnt.as<int>(), ctx->d_status);
         ++ctx->launches;
@@ -802,7 +861,8 @@ int md_rigid_constrain_velocities(md_rigid* rw, md_system* sys, int* iterations)
     MDB_TRY(cnt.ensure(sizeof(int)));
     MDB_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(int), ctx->stream));
     if (nmol > 0) {
-        k_rattle<<<grid_for(nmol, kBlock), kBlock, 0, ctx->stream>>>(
+        const int block = mol_block(ctx, nmol);
+        k_rattle<<<grid_for(nmol, block), block, 0, ctx->stream>>>(
             sys->cur, sys->slot, nmol, rigid_args(*rw), box_of(sys), cnt.as<int>(), ctx->d_status);
         ++ctx->launches;
         MDB_CHECK_LAUNCH();
@@ -914,7 +974,7 @@ int md_water_rdf_run(md_integrator* it, md_system* sys, md_ewald* ff, md_rdf* rd
         if (!rescale) return MD_OK;
         MDB_TRY(md_system_rescale_temperature(sys, dof, temperature));
         if (L.nmol > 0) {
-            k_rattle<<<grid_for(L.nmol, kBlock), kBlock, 0, ctx->stream>>>(
+            k_rattle<<<grid_for(L.nmol, L.block), L.block, 0, ctx->stream>>>(
                 sys->cur, sys->slot, L.nmol, rigid_args(it->rigid), box_of(sys),
                 it->counters.as<int>() + 1, ctx->d_status);
             ++ctx->launches;
