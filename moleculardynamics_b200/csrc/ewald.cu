@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <new>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -35,6 +36,7 @@ namespace {
 
 constexpr double kPi = 3.14159265358979323846;
 constexpr int kBlock = 256;
+constexpr int kRealBlock = 64;  // the real-space pass
 
 // ewald.hpp:10-13, ewald.cpp:17-21
 double coulomb_prefactor() {
@@ -50,52 +52,82 @@ struct RealArgs {
     double rc, uc, dudrc;
 };
 
-// The real-space Coulomb (ewald.cpp:60-68) and O-O LJ (lennard_jones.cpp:62-77)
-// terms of one pair at r2, in FP32 (MD_PRECISION_MIXED): returns the force
-// coefficient s (F = s d) and adds the energies and virials of the pair.
-__device__ __forceinline__ float real_pair_mixed(float r2, float cqq, bool coulomb, bool lj,
-                                                 const RealArgs& a, float& er, float& wr,
-                                                 float& el, float& wl) {
-    float s = 0.0f;
+// Terms of one pair inside the cutoff: force coefficient (F = s d), real-space energy and
+// virial, LJ energy and virial (zero where the pair has no such term).
+template <class T>
+struct RealTerms {
+    T s, er, wr, el, wl;
+};
+
+// The real-space Coulomb (ewald.cpp:60-68) and O-O LJ (lennard_jones.cpp:62-77) terms of a
+// pair at r2 in arithmetic T (FP32: MD_PRECISION_MIXED); div2 divides by r2, div1 by r.
+template <class T, class Div2, class Div1>
+__device__ __forceinline__ RealTerms<T> real_terms(T r2, T r, T cqq, bool coulomb, bool lj,
+                                                   const RealArgs& a, Div2 div2, Div1 div1) {
+    RealTerms<T> t = {T(0), T(0), T(0), T(0), T(0)};
     if (coulomb) {
-        const float r = sqrtf(r2);
-        const float erfc_ar = erfcf(static_cast<float>(a.alpha) * r);
-        const float w = cqq * (static_cast<float>(a.two_alpha_over_sqrt_pi) *
-                                   expf(static_cast<float>(a.neg_alpha2) * r2) +
-                               erfc_ar / r);
-        s = w / r2;
-        er = cqq * erfc_ar / r;
-        wr = w;
+        T erfc_ar, gauss;
+        if constexpr (sizeof(T) == 4) {
+            erfc_ar = erfcf(static_cast<T>(a.alpha) * r);
+            gauss = expf(static_cast<T>(a.neg_alpha2) * r2);
+        } else {
+            erfc_ar = erfc(a.alpha * r);
+            gauss = exp(a.neg_alpha2 * r2);
+        }
+        t.wr = cqq * (static_cast<T>(a.two_alpha_over_sqrt_pi) * gauss + div1(erfc_ar));
+        t.s = div2(t.wr);
+        t.er = div1(cqq * erfc_ar);
     }
     if (lj) {
-        const float s2 = static_cast<float>(a.sig2) / r2;
-        const float s6 = s2 * s2 * s2;
-        float w = static_cast<float>(a.tf_eps) * (2.0f * s6 * s6 - s6);
-        float u = static_cast<float>(a.four_eps) * (s6 * s6 - s6);
+        const T s2 = div2(static_cast<T>(a.sig2));
+        const T s6 = s2 * s2 * s2;
+        t.wl = static_cast<T>(a.tf_eps) * (T(2) * s6 * s6 - s6);
+        t.el = static_cast<T>(a.four_eps) * (s6 * s6 - s6);
         if (a.lj_lfs) {
-            const float r = sqrtf(r2);
-            u = u - static_cast<float>(a.uc) - (r - static_cast<float>(a.rc)) * static_cast<float>(a.dudrc);
-            w = w + r * static_cast<float>(a.dudrc);
+            t.el = t.el - static_cast<T>(a.uc) - (r - static_cast<T>(a.rc)) * static_cast<T>(a.dudrc);
+            t.wl = t.wl + r * static_cast<T>(a.dudrc);
         }
-        s += w / r2;
-        el = u;
-        wl = w;
+        t.s += div2(t.wl);
     }
-    return s;
+    return t;
+}
+
+// Separations whose quotients could leave the normal range divide in IEEE arithmetic.
+template <class T>
+__device__ __noinline__ RealTerms<T> real_terms_ieee(T r2, T cqq, bool coulomb, bool lj,
+                                                     const RealArgs* a) {
+    const T r = sqrt(r2);
+    return real_terms<T>(r2, r, cqq, coulomb, lj, *a, [r2](T x) { return x / r2; },
+                         [r](T x) { return x / r; });
+}
+
+template <class T>
+__device__ __forceinline__ RealTerms<T> real_pair(T r2, T cqq, bool coulomb, bool lj,
+                                                  const RealArgs& a) {
+    if (!(r2 > T(1e-15))) return real_terms_ieee<T>(r2, cqq, coulomb, lj, &a);
+    T r;
+    if constexpr (sizeof(T) == 4) r = __fsqrt_rn(r2);
+    else r = __dsqrt_rn(r2);
+    const T y2 = reciprocal(r2), y1 = reciprocal(r);
+    return real_terms<T>(r2, r, cqq, coulomb, lj, a, [r2, y2](T x) { return quotient(x, r2, y2); },
+                         [r, y1](T x) { return quotient(x, r, y1); });
 }
 
 // Real-space (and SPC/E O-O LJ) pair terms over the Verlet list.  out[0..3]:
 // E_real, W_real, E_lj, W_lj.  mode 1 writes forces, mode 2 adds to them.
 // MIXED: the displacement, the cutoff test and every sum stay FP64; the pair
 // terms (erfc, exp, the LJ powers) are evaluated in FP32.
-// 128-thread blocks (kRealBlock); the FP64 variant fits six per SM in 78
-// registers without spilling, the FP32 one five.
+// A pair's five divisions are by r and r^2 alone and share two reciprocals; the next
+// entry's index and site are requested while the current pair is evaluated.  Blocks of
+// kRealBlock threads: small, so that the last wave of a few thousand sites is short.
+// 12,288 sites, 16 threads a site: FP32 terms 120 us with five
+// IEEE divisions, no prefetch and 128-thread blocks, 85 us so; FP64 terms 157 and 122 us.
 template <int TPA, bool MIXED>
-__global__ void __launch_bounds__(128, MIXED ? 5 : 6)
+__global__ void __launch_bounds__(kRealBlock, MIXED ? 14 : 10)
 k_ewald_real(const double4* __restrict__ pos, const double* __restrict__ q,
              const int64_t* __restrict__ mol, const int* __restrict__ nbr,
-             const int* __restrict__ count, int stride, int64_t n, Box3 box, RealArgs a,
-             int mode, double* fxo, double* fyo, double* fzo, double* part, unsigned* ticket,
+             const int* __restrict__ count, int stride, int64_t n, Box3 box,
+             const __grid_constant__ RealArgs a, int mode, double* fxo, double* fyo, double* fzo, double* part, unsigned* ticket,
              double* out) {
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     const int64_t i = t / TPA;
@@ -106,78 +138,44 @@ k_ewald_real(const double4* __restrict__ pos, const double* __restrict__ q,
         const double4 pi = pos[i];
         const double qi = q[i];
         const int64_t mi = mol[i];
-        const bool oxy_i = (static_cast<int64_t>(pi.w) % 3) == 0;
+        const bool oxy_i = a.spce_lj && (static_cast<int>(pi.w) % 3) == 0;
         const int cnt = min(count[i], stride);
         const int* row = nbr + i * static_cast<int64_t>(stride);
-        // the neighbour's position, charge and molecule are requested together, so
-        // one L2 round trip serves the cutoff test and the pair terms
-#pragma unroll 2
-        for (int k = g; k < cnt; k += TPA) {
-            const int j = __ldg(row + k);
-            const double4 pj = ldg4(pos + j);
-            const double qj = __ldg(q + j);
-            const int64_t mj = __ldg(mol + j);
-            const bool lo = pi.w < pj.w;
-            // r_lower - r_higher by original index, the reference's pair order; the
-            // operands are selected rather than branched on, so a warp runs one fold
+        int k = g;
+        int j = k < cnt ? __ldg(row + k) : static_cast<int>(i);
+        int jn = k + TPA < cnt ? __ldg(row + k + TPA) : static_cast<int>(i);
+        double4 pj = ldg4(pos + j);
+        double qj = __ldg(q + j);
+        int64_t mj = __ldg(mol + j);
+        for (; k < cnt; k += TPA) {
+            const double4 pc = pj;
+            const double qc = qj;
+            const bool coul = mj != mi;
+            // the next entry
+            pj = ldg4(pos + jn);
+            qj = __ldg(q + jn);
+            mj = __ldg(mol + jn);
+            jn = k + 2 * TPA < cnt ? __ldg(row + k + 2 * TPA) : jn;
+            // r_lower - r_higher by original index has the reference's rounding
+            const bool lo = pi.w < pc.w;
             double dx, dy, dz;
-            min_image_wrapped(f3, lo ? pi.x : pj.x, lo ? pi.y : pj.y, lo ? pi.z : pj.z,
-                              lo ? pj.x : pi.x, lo ? pj.y : pi.y, lo ? pj.z : pi.z, dx, dy, dz);
+            min_image_pair(f3, pi, pc, lo, dx, dy, dz);
             const double r2 = norm2_exact(dx, dy, dz);
             if (!(r2 < a.rc2)) continue;
-            double s = 0.0;
-            if (MIXED) {
-                const bool coul = mj != mi;
-                const bool lj = a.spce_lj && oxy_i && (static_cast<int>(pj.w) % 3) == 0;
-                float per = 0.0f, pwr = 0.0f, pel = 0.0f, pwl = 0.0f;
-                s = real_pair_mixed(static_cast<float>(r2),
-                                    coul ? static_cast<float>(a.coulomb * (qi * qj)) : 0.0f, coul,
-                                    lj, a, per, pwr, pel, pwl);
-                if (lo) {
-                    er += per;
-                    wr += pwr;
-                    el += pel;
-                    wl += pwl;
-                }
-                const double sg = lo ? s : -s;
-                fx = fma(dx, sg, fx);
-                fy = fma(dy, sg, fy);
-                fz = fma(dz, sg, fz);
-                continue;
+            const bool lj = oxy_i && (static_cast<int>(pc.w) % 3) == 0;
+            using T = typename std::conditional<MIXED, float, double>::type;
+            const RealTerms<T> p = real_pair<T>(static_cast<T>(r2), static_cast<T>(a.coulomb * (qi * qc)),
+                                                coul, lj, a);
+            if (lo) {
+                er += p.er;
+                wr += p.wr;
+                el += p.el;
+                wl += p.wl;
             }
-            if (mol[j] != mi) {
-                // ewald.cpp:60-68
-                const double r = __dsqrt_rn(r2);
-                const double cqq = a.coulomb * (qi * q[j]);
-                const double erfc_ar = erfc(a.alpha * r);
-                const double w = cqq * (a.two_alpha_over_sqrt_pi * exp(a.neg_alpha2 * r2) + erfc_ar / r);
-                s = w / r2;
-                if (lo) {
-                    er += cqq * erfc_ar / r;
-                    wr += w;
-                }
-            }
-            if (a.spce_lj && oxy_i && (static_cast<int>(pj.w) % 3) == 0) {
-                // lennard_jones.cpp:62-70 (Truncated)
-                const double s2 = a.sig2 / r2;
-                const double s6 = s2 * s2 * s2;
-                double w = a.tf_eps * (2.0 * s6 * s6 - s6);
-                double u = a.four_eps * (s6 * s6 - s6);
-                if (a.lj_lfs) {  // lennard_jones.cpp:73-77
-                    const double r = sqrt(r2);
-                    u = u - a.uc - (r - a.rc) * a.dudrc;
-                    w = w + r * a.dudrc;
-                }
-                s += w / r2;
-                if (lo) {
-                    el += u;
-                    wl += w;
-                }
-            }
-            const double sg = lo ? s : -s;
-            fx = fma(dx, sg, fx);
-            fy = fma(dy, sg, fy);
-            fz = fma(dz, sg, fz);
+            const double s = p.s;
+            fx = fma(dx, s, fx);
+            fy = fma(dy, s, fy);
+            fz = fma(dz, s, fz);
         }
     }
 #pragma unroll
@@ -628,10 +626,6 @@ int real_tpa(const md_context* ctx, int64_t n) {
     while (tpa < 32 && n * tpa < want) tpa *= 2;
     return tpa;
 }
-
-// 128-thread blocks: six (FP64) or five (FP32 pair terms) fit on an SM, 24 or 20
-// warps, where two 256-thread blocks at ~96 registers would give 16.
-constexpr int kRealBlock = 128;
 
 template <int TPA, bool MIXED>
 void launch_real_t(md_system* sys, md_verlet* v, const RealArgs& a, int mode, double* fx,

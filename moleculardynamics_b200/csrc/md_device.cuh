@@ -122,6 +122,21 @@ __device__ __forceinline__ bool divides_fast(double b) {
     return static_cast<unsigned>(__double2hiint(b)) - 0x39b00000u < 0x58f00000u - 0x39b00000u;
 }
 
+// The same in FP32: one Newton step from rcp.approx gives the correctly rounded reciprocal
+// of every normal divisor (all 2^23 significands tested) but one whose significand is all
+// ones, and quotient() then the IEEE quotient, branch-free.  For 2^-60 <= b < 2^60 and
+// quotients in the normal range.
+__device__ __forceinline__ float reciprocal(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return fmaf(y, fmaf(-b, y, 1.0f), y);
+}
+
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+    const float q = __fmul_rn(a, y);
+    return fmaf(y, fmaf(-b, q, a), q);
+}
+
 // Minimum-image displacement r_a - r_b with the reference's operation order.
 __device__ __forceinline__ void min_image_exact(const Box3& b, double ax, double ay, double az,
                                                 double bx, double by, double bz, double& dx,
