@@ -401,6 +401,54 @@ k_lj_verlet(const typename PosOf<MIXED>::T* __restrict__ pos, const double4* __r
 // shape; other shapes leave the kick to the integrator's own pass).
 constexpr bool verlet_kicks(int tpa, int unroll) { return tpa == 2 && unroll == 2; }
 
+// An atom's force written and, with KICK, the closing half-kick applied as the separate
+// kick kernel does it; its kinetic energy (0 without).
+template <bool KICK>
+__device__ __forceinline__ double finish_atom(int64_t i, double fx, double fy, double fz, double* fxo,
+                                              double* fyo, double* fzo, const KickArgs& kick) {
+    fxo[i] = fx;
+    fyo[i] = fy;
+    fzo[i] = fz;
+    if constexpr (!KICK) return 0.0;
+    const double c = __dmul_rn(kick.half_dt, kick.inv_mass[i]);
+    const double vx = fma(c, fx, kick.vx[i]);
+    const double vy = fma(c, fy, kick.vy[i]);
+    const double vz = fma(c, fz, kick.vz[i]);
+    kick.vx[i] = vx;
+    kick.vy[i] = vy;
+    kick.vz[i] = vz;
+    return 0.5 * kick.mass[i] * (vx * vx + vy * vy + vz * vz);
+}
+
+// grid_reduce of the two-thread kernel, from a block that holds the values of W of its
+// warps (K values per thread of theirs): each warp's tree, then eight warps by the tree of
+// a warp whose other lanes are zero, then its blocks.
+template <int K, int W>
+__device__ __forceinline__ void reduce_as_two_thread(const double (&s_red)[K][W][32], double* part,
+                                                     unsigned* ticket, double* out,
+                                                     uint32_t* status) {
+    __shared__ double sm[K][32];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x >> 5; t < K * W; t += blockDim.x >> 5) {
+        const int k = t / W, w = t % W;
+        const double s = warp_sum(s_red[k][w][lane]);
+        if (lane == 0) {
+            part[(static_cast<size_t>(blockIdx.x) * W + w) * K + k] = s;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    const unsigned warps = gridDim.x * W;
+    grid_reduce_tail<K>(sm, (warps + 7) / 8, ticket, out, status, gridDim.x, [=](unsigned p, int k) {
+        double v[8];
+#pragma unroll
+        for (unsigned w = 0; w < 8; ++w)
+            v[w] = 8 * p + w < warps ? __ldcg(part + static_cast<size_t>(8 * p + w) * K + k) : 0.0;
+        return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
+    });
+}
+
 // The FP64 pass of systems too small to fill the machine two threads an atom: kWide lanes
 // per atom each form the terms of one list entry, and the sums are then taken in the
 // two-thread kernel's order -- lane 2 c + p adds component c (fx, fy, fz, energy, virial)
@@ -423,7 +471,7 @@ k_lj_wide(const double4* __restrict__ pos, const int* __restrict__ nbr,
     constexpr int kTerms = 5;  // force, energy, virial
     constexpr int K = KICK ? 3 : 2;
     __shared__ double s_t[kWideAtoms][kTerms][kWide];
-    __shared__ double s_red[K][2 * kWideAtoms];
+    __shared__ double s_red[K][1][2 * kWideAtoms];
     const int ai = threadIdx.x / kWide, g = threadIdx.x % kWide;
     const int64_t i = blockIdx.x * static_cast<int64_t>(kWideAtoms) + ai;
     const Fold3 f3 = fold3_of(box);
@@ -454,48 +502,74 @@ k_lj_wide(const double4* __restrict__ pos, const int* __restrict__ nbr,
     const double f = acc + __shfl_xor_sync(0xffffffffu, acc, 1);  // both parities of a component
     const double fy = __shfl_sync(0xffffffffu, f, 2, kWide), fz = __shfl_sync(0xffffffffu, f, 4, kWide);
     double ke = 0.0;
-    if (i < n && g == 0) {
-        const double fx = f;
-        fxo[i] = fx;
-        fyo[i] = fy;
-        fzo[i] = fz;
-        if constexpr (KICK) {  // the closing half-kick, as the separate kick kernel does it
-            const double c = __dmul_rn(kick.half_dt, kick.inv_mass[i]);
-            const double vx = fma(c, fx, kick.vx[i]);
-            const double vy = fma(c, fy, kick.vy[i]);
-            const double vz = fma(c, fz, kick.vz[i]);
-            kick.vx[i] = vx;
-            kick.vy[i] = vy;
-            kick.vz[i] = vz;
-            ke = 0.5 * kick.mass[i] * (vx * vx + vy * vy + vz * vz);
-        }
-    }
-    if (comp == 3 || comp == 4) s_red[comp - 3][2 * ai + par] = acc;
-    if (KICK && g < 2) s_red[K - 1][2 * ai + g] = ke;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp < K) {
-        const double s = warp_sum(s_red[warp][lane]);
-        if (lane == 0) {
-            part[static_cast<size_t>(blockIdx.x) * K + warp] = s;
-            __threadfence();
-        }
-    }
-    __syncthreads();
-    // eight of these blocks are one block of the two-thread kernel: its eight warps' sums,
-    // added by the tree of a warp whose other lanes are zero
-    __shared__ double sm[K][32];
-    const unsigned nb = gridDim.x;
-    grid_reduce_tail<K>(sm, (nb + 7) / 8, ticket, out, KICK ? kick.status : nullptr, nb,
-                        [=](unsigned p, int k) {
-                            double v[8];
+    if (i < n && g == 0) ke = finish_atom<KICK>(i, f, fy, fz, fxo, fyo, fzo, kick);
+    if (comp == 3 || comp == 4) s_red[comp - 3][0][2 * ai + par] = acc;
+    if (KICK && g < 2) s_red[K - 1][0][2 * ai + g] = ke;
+    reduce_as_two_thread<K, 1>(s_red, part, ticket, out, KICK ? kick.status : nullptr);
+}
+
+// The same for systems of 64 to 256 atoms per SM, four lanes an atom: lanes p and
+// p + 2 form two entries of parity p; lane p adds both to the forces, lane p + 2 both to
+// energy and virial, each receiving the other's terms by shuffle, so the additions are
+// shared out and none is waited for in shared memory.  Force pass of the liquid, two lanes
+// against four (us, events and launch included): 13,500 atoms 32 / 23, 23,328 atoms 35 /
+// 29, 32,000 atoms 36 / 33 (59 / 50 with a skin of 1), 55,296 atoms 45 / 48.
+constexpr int kQuad = 4;
+constexpr int kQuadAtoms = kBlock / kQuad;
+
+template <bool LFS, bool KICK>
+__global__ void __launch_bounds__(kBlock, 4)
+k_lj_quad(const double4* __restrict__ pos, const int* __restrict__ nbr,
+          const int* __restrict__ count, int stride, int64_t n, Box3 box, LJArgs a,
+          double* __restrict__ fxo, double* __restrict__ fyo, double* __restrict__ fzo,
+          double* part, unsigned* ticket, double* out, KickArgs kick) {
+    constexpr int K = KICK ? 3 : 2;
+    constexpr int kTwoWarps = kQuadAtoms / 16;  // warps of the two-thread kernel in this block
+    __shared__ double s_red[K][kTwoWarps][32];
+    const int ai = threadIdx.x / kQuad, g = threadIdx.x % kQuad;
+    const int64_t i = blockIdx.x * static_cast<int64_t>(kQuadAtoms) + ai;
+    const Fold3 f3 = fold3_of(box);
+    const int cnt = i < n ? min(count[i], stride) : 0;
+    const double4 pi = ldg4(pos + (i < n ? i : 0));
+    const int* row = nbr + (i < n ? i : 0) * static_cast<int64_t>(stride);
+    const bool forces = g < 2;  // lanes 0 and 1 own the forces, 2 and 3 energy and virial
+    double acc[3] = {0.0, 0.0, 0.0};
+    const int most = __reduce_max_sync(0xffffffffu, cnt);  // of the warp's eight atoms
+    int j = g < cnt ? __ldg(row + g) : -1;
+    int jn = g + kQuad < cnt ? __ldg(row + g + kQuad) : -1;
+    double4 pj = ldg4(pos + max(j, 0));
+    for (int k0 = 0; k0 < most; k0 += kQuad) {
+        const double4 pc = pj;
+        const bool live = j >= 0;
+        pj = ldg4(pos + max(jn, 0));
+        j = jn;
+        const int kn = k0 + 2 * kQuad + g;
+        jn = kn < cnt ? __ldg(row + kn) : -1;
+        double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (live) accumulate_exact<LFS>(a, f3, pi, pc, v[0], v[1], v[2], v[3], v[4]);
+        // entry order within a parity: lane p's, then lane p + 2's; a zero leaves a sum alone
+        const double own[3] = {forces ? v[0] : v[3], forces ? v[1] : v[4], v[2]};
+        const double other[3] = {__shfl_xor_sync(0xffffffffu, forces ? v[3] : v[0], 2),
+                                 __shfl_xor_sync(0xffffffffu, forces ? v[4] : v[1], 2),
+                                 __shfl_xor_sync(0xffffffffu, v[2], 2)};
 #pragma unroll
-                            for (unsigned w = 0; w < 8; ++w)
-                                v[w] = 8 * p + w < nb
-                                           ? __ldcg(part + static_cast<size_t>(8 * p + w) * K + k)
-                                           : 0.0;
-                            return ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
-                        });
+        for (int c = 0; c < 3; ++c)
+            acc[c] = __dadd_rn(__dadd_rn(acc[c], forces ? own[c] : other[c]), forces ? other[c] : own[c]);
+    }
+    // both parities of a force component meet on lane 0
+    const double fx = acc[0] + __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    const double fy = acc[1] + __shfl_xor_sync(0xffffffffu, acc[1], 1);
+    const double fz = acc[2] + __shfl_xor_sync(0xffffffffu, acc[2], 1);
+    double ke = 0.0;
+    if (i < n && g == 0) ke = finish_atom<KICK>(i, fx, fy, fz, fxo, fyo, fzo, kick);
+    const int tw = ai / 16, tl = 2 * (ai % 16);
+    if (!forces) {
+        s_red[0][tw][tl + g - 2] = acc[0];
+        s_red[1][tw][tl + g - 2] = acc[1];
+    } else if (KICK) {
+        s_red[K - 1][tw][tl + g] = ke;
+    }
+    reduce_as_two_thread<K, kTwoWarps>(s_red, part, ticket, out, KICK ? kick.status : nullptr);
 }
 
 // One system's arguments of the batched force pass.
@@ -1522,18 +1596,21 @@ bool launch_verlet(md_system* sys, md_verlet* v, const LJArgs& a, double* part, 
     return kicks;
 }
 
-// FP64 systems of up to 64 atoms per SM take kWide lanes an atom (see k_lj_wide); the mixed
-// pass, whose pair terms are a few FP32 operations, gains too little to leave two threads.
-bool verlet_wide(const md_context* ctx, int64_t n, bool mixed, int tpa, int unroll) {
-    return !mixed && tpa == 2 && unroll == 2 && n > 0 &&
-           n < 64 * static_cast<int64_t>(ctx->sm_count);
+// Lanes per atom of the FP64 gathered pass where its shape is the default (or asked to be):
+// kWide up to 64 atoms per SM, kQuad up to 256, two beyond.  The mixed pass, whose pair
+// terms are a few FP32 operations, gains too little to leave two threads.
+int verlet_lanes(const md_context* ctx, int64_t n, bool mixed, int tpa, int unroll) {
+    if (mixed || tpa != 2 || unroll != 2 || n <= 0) return tpa;
+    if (n < 64 * static_cast<int64_t>(ctx->sm_count)) return kWide;
+    return n < 256 * static_cast<int64_t>(ctx->sm_count) ? kQuad : tpa;
 }
 
 template <bool LFS>
-void launch_wide(md_system* sys, md_verlet* v, const LJArgs& a, double* part, unsigned* ticket,
-                 double* out, const KickArgs* kick) {
-    auto kernel = kick ? k_lj_wide<LFS, true> : k_lj_wide<LFS, false>;
-    kernel<<<grid_for(sys->n, kWideAtoms), kBlock, 0, sys->ctx->stream>>>(
+void launch_wide(int lanes, md_system* sys, md_verlet* v, const LJArgs& a, double* part,
+                 unsigned* ticket, double* out, const KickArgs* kick) {
+    auto kernel = lanes == kQuad ? (kick ? k_lj_quad<LFS, true> : k_lj_quad<LFS, false>)
+                                 : (kick ? k_lj_wide<LFS, true> : k_lj_wide<LFS, false>);
+    kernel<<<grid_for(sys->n, kBlock / lanes), kBlock, 0, sys->ctx->stream>>>(
         sys->cur.pos, v->nbr.as<int>(), v->count.as<int>(), v->stride, sys->n, box_of(sys), a,
         sys->cur.fx, sys->cur.fy, sys->cur.fz, part, ticket, out, kick ? *kick : KickArgs{});
 }
@@ -1713,9 +1790,11 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
     const LJArgs a = verlet_lj_args(lj, sys);
     const int tpa = lj->tpa ? lj->tpa : g_lj_tpa, unroll = lj->unroll ? lj->unroll : g_lj_unroll;
     const bool mixed = lj->precision == MD_PRECISION_MIXED;
-    const bool wide = verlet_wide(ctx, sys->n, mixed, tpa, unroll);
-    const int64_t threads = std::max<int64_t>(sys->n * (wide ? kWide : tpa), 1);
-    const int64_t blocks = std::max<int64_t>(grid_for(threads, kBlock), halo_blocks(sys->n));
+    const int lanes = verlet_lanes(ctx, sys->n, mixed, tpa, unroll);
+    const int64_t threads = std::max<int64_t>(sys->n * lanes, 1);
+    int64_t blocks = std::max<int64_t>(grid_for(threads, kBlock), halo_blocks(sys->n));
+    // these leave a partial sum per 16 atoms (reduce_as_two_thread), in whole blocks
+    if (lanes != tpa) blocks *= kBlock / lanes / 16;
     double* part;
     MDB_TRY(ctx_partials(ctx, 3 * static_cast<size_t>(blocks), &part));
     unsigned* ticket = ctx_counter(ctx, 2);
@@ -1743,9 +1822,9 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
         if (lfs) launch_halo_u<true>(unroll, sys, v, a, part, ticket, out, kick);
         else launch_halo_u<false>(unroll, sys, v, a, part, ticket, out, kick);
         if (kick && kicked) *kicked = true;
-    } else if (wide) {
-        if (lfs) launch_wide<true>(sys, v, a, part, ticket, out, kick);
-        else launch_wide<false>(sys, v, a, part, ticket, out, kick);
+    } else if (lanes != tpa) {
+        if (lfs) launch_wide<true>(lanes, sys, v, a, part, ticket, out, kick);
+        else launch_wide<false>(lanes, sys, v, a, part, ticket, out, kick);
         if (kick && kicked) *kicked = true;
     } else {
         // the default gathered shape also takes the closing half-kick when asked

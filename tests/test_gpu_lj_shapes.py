@@ -79,3 +79,31 @@ def test_small_systems_equal_their_batch(md, mixed, cubic, trunc):
         assert np.array_equal(it.run(s, v, lj, 12, thermo=True), rows[k]), n
         assert np.array_equal(parts[k][1].positions, s.positions), n
         assert np.array_equal(parts[k][1].velocities, s.velocities), n
+
+
+@pytest.mark.parametrize("trunc", [0, 1])
+def test_middle_systems_equal_their_batch(md, trunc):
+    """From 64 to 256 atoms per SM four lanes take an atom, again with the two-lane sums:
+    10,976 atoms (a part of the last block), 23,328 and, back at two lanes, 39,303."""
+    def make(cells, missing, ctx):
+        st = md.fcc_lattice(cells, 0.75, 1.3, cells)
+        keep = slice(missing, None)
+        s = md.System.from_arrays(st["pos"][keep], st["box"], vel=st["vel"][keep],
+                                  mass=st["mass"][keep], ctx=ctx)
+        lj = md.LennardJones(1.0, 1.0, 2.5, trunc)
+        v = md.VerletList(st["box"], 2.5, 0.3, ctx=ctx)
+        v.build(s)
+        lj.compute_forces(s, v)
+        return md.NoseHooverChain(0.005, 1.3, 0.5, 3, 3 * s.n - 3), s, v, lj
+
+    sizes = [(14, 0), (14, 41), (18, 0), (22, 3289)]
+    batch = md.Batch()
+    parts = [make(c, m, md.Context(0)) for c, m in sizes]
+    for p in parts:
+        batch.add(*p)
+    rows = batch.run(15, thermo=True)
+    for k, (c, m) in enumerate(sizes):
+        it, s, v, lj = make(c, m, md.Context(0))
+        assert np.array_equal(it.run(s, v, lj, 15, thermo=True), rows[k]), k
+        assert np.array_equal(parts[k][1].positions, s.positions), k
+        assert np.array_equal(parts[k][1].velocities, s.velocities), k
