@@ -79,20 +79,16 @@ int ctx_scratch(md_context* ctx, size_t bytes, void** out) {
     return MD_OK;
 }
 
-int ctx_read_results(md_context* ctx, int first, int count, double* out) {
-    MDB_CUDA(cudaMemcpyAsync(ctx->h_result + first, ctx->result.as<double>() + first,
-                             sizeof(double) * static_cast<size_t>(count), cudaMemcpyDeviceToHost,
+// The status word is copied with whatever a call reads back, so one synchronisation
+// serves both (copy, then report after it).
+static int ctx_copy_status(md_context* ctx) {
+    MDB_CUDA(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                              ctx->stream));
-    MDB_CUDA(cudaStreamSynchronize(ctx->stream));
-    std::memcpy(out, ctx->h_result + first, sizeof(double) * static_cast<size_t>(count));
-    return ctx_check_status(ctx);
+    return MD_OK;
 }
 
-int ctx_check_status(md_context* ctx) {
-    uint32_t st = 0;
-    MDB_CUDA(cudaMemcpyAsync(&st, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                             ctx->stream));
-    MDB_CUDA(cudaStreamSynchronize(ctx->stream));
+static int ctx_report_status(md_context* ctx) {
+    const uint32_t st = *ctx->h_status;
     if (st == 0) return MD_OK;
     // reported once: clear the word so the context can be used again
     MDB_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
@@ -104,6 +100,22 @@ int ctx_check_status(md_context* ctx) {
                 (st & MD_STATUS_SHAKE_SINGULAR) ? "SHAKE singular " : "",
                 (st & MD_STATUS_NONFINITE) ? "non-finite state " : "",
                 (st & MD_STATUS_WAIT_TIMEOUT) ? "bounded wait ran out" : "");
+}
+
+int ctx_read_results(md_context* ctx, int first, int count, double* out) {
+    MDB_CUDA(cudaMemcpyAsync(ctx->h_result + first, ctx->result.as<double>() + first,
+                             sizeof(double) * static_cast<size_t>(count), cudaMemcpyDeviceToHost,
+                             ctx->stream));
+    MDB_TRY(ctx_copy_status(ctx));
+    MDB_CUDA(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(out, ctx->h_result + first, sizeof(double) * static_cast<size_t>(count));
+    return ctx_report_status(ctx);
+}
+
+int ctx_check_status(md_context* ctx) {
+    MDB_TRY(ctx_copy_status(ctx));
+    MDB_CUDA(cudaStreamSynchronize(ctx->stream));
+    return ctx_report_status(ctx);
 }
 
 void ctx_time_begin(md_context* ctx, int kernel) {
@@ -176,7 +188,9 @@ int md_context_create(int device, md_context** out) {
     // buffer is never reallocated under queued kernels.
     MDB_TRY(ctx->partials.ensure(sizeof(double) * (size_t(1) << 20)));
     MDB_CUDA(cudaMemset(ctx->result.ptr, 0, sizeof(double) * kMaxResults));
-    MDB_CUDA(cudaMallocHost(&ctx->h_result, sizeof(double) * kMaxResults));
+    MDB_CUDA(cudaMallocHost(&ctx->h_result, sizeof(double) * (kMaxResults + 1)));
+    ctx->h_status = reinterpret_cast<uint32_t*>(ctx->h_result + kMaxResults);
+    ctx->h_flag = reinterpret_cast<int*>(ctx->h_status + 1);
     MDB_CUDA(cudaDeviceSynchronize());
     graph_epoch_bump();
     *out = ctx;

@@ -90,6 +90,8 @@ struct md_context {
     mdb::DevBuf scratch;                 // general scratch (staging, scans)
     mdb::DevBuf result;                  // small device results (energy, virial, ...)
     double* h_result = nullptr;          // pinned host mirror of `result`
+    uint32_t* h_status = nullptr;        // pinned, after it: the status word and
+    int* h_flag = nullptr;               // a flag a host call reads back
     int64_t launches = 0;
     int64_t graph_captures = 0;          // step graphs captured by fused loops
     int sm_count = 148;

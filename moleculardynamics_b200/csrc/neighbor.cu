@@ -1653,11 +1653,10 @@ int md_verlet_needs_rebuild(md_verlet* v, md_system* sys, int* flag) {
     if (!v || !sys || !flag) return fail(MD_ERR_INVALID_ARGUMENT, "md_verlet_needs_rebuild: NULL");
     MDB_TRY(verlet_ready(v, sys, "md_verlet_needs_rebuild"));
     MDB_TRY(verlet_check(v, sys));
-    int f = 0;
-    MDB_CUDA(cudaMemcpyAsync(&f, v->d_rebuild_flag, sizeof(int), cudaMemcpyDeviceToHost,
+    MDB_CUDA(cudaMemcpyAsync(sys->ctx->h_flag, v->d_rebuild_flag, sizeof(int), cudaMemcpyDeviceToHost,
                              sys->ctx->stream));
     MDB_CUDA(cudaStreamSynchronize(sys->ctx->stream));
-    *flag = f;
+    *flag = *sys->ctx->h_flag;
     return MD_OK;
 }
 

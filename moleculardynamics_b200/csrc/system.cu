@@ -37,32 +37,42 @@ __device__ __forceinline__ double* field_ptr(const md_atoms& a, int field) {
     }
 }
 
-// dev[k] = staging[orig[k]]  (host order -> device order)
-__global__ void k_set_field(md_atoms a, int field, const double* __restrict__ staging, int64_t n) {
+// The fields of one upload or read-back, column c of the staging buffer holding field f[c].
+constexpr int kMaxFields = MD_FIELD_CHARGE + 1;
+
+struct FieldList {
+    int count;
+    int f[kMaxFields];
+};
+
+// dev[k] = staging[orig[k]]  (host order -> device order), every column in one pass
+__global__ void k_set_fields(md_atoms a, FieldList l, const double* __restrict__ staging, int64_t n) {
     const int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (k >= n) return;
-    const double v = staging[a.orig[k]];
-    if (field <= MD_FIELD_Z) {
-        double* p = reinterpret_cast<double*>(a.pos + k);
-        p[field] = v;
-    } else {
-        field_ptr(a, field)[k] = v;
-        if (field == MD_FIELD_MASS) a.inv_mass[k] = 1.0 / v;  // velocity_verlet.hpp:59
+    const int64_t o = a.orig[k];
+    for (int c = 0; c < l.count; ++c) {
+        const int field = l.f[c];
+        const double v = staging[c * n + o];
+        if (field <= MD_FIELD_Z) {
+            double* p = reinterpret_cast<double*>(a.pos + k);
+            p[field] = v;
+        } else {
+            field_ptr(a, field)[k] = v;
+            if (field == MD_FIELD_MASS) a.inv_mass[k] = 1.0 / v;  // velocity_verlet.hpp:59
+        }
     }
 }
 
-// staging[orig[k]] = dev[k]  (device order -> host order)
-__global__ void k_get_field(md_atoms a, int field, double* __restrict__ staging, int64_t n) {
+// staging[orig[k]] = dev[k]  (device order -> host order), every column in one pass
+__global__ void k_get_fields(md_atoms a, FieldList l, double* __restrict__ staging, int64_t n) {
     const int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (k >= n) return;
-    double v;
-    if (field <= MD_FIELD_Z) {
-        const double* p = reinterpret_cast<const double*>(a.pos + k);
-        v = p[field];
-    } else {
-        v = field_ptr(a, field)[k];
+    const int64_t o = a.orig[k];
+    for (int c = 0; c < l.count; ++c) {
+        const int field = l.f[c];
+        staging[c * n + o] = field <= MD_FIELD_Z ? reinterpret_cast<const double*>(a.pos + k)[field]
+                                                 : field_ptr(a, field)[k];
     }
-    staging[a.orig[k]] = v;
 }
 
 __global__ void k_set_mol(md_atoms a, const int64_t* __restrict__ staging, int64_t n) {
@@ -302,8 +312,8 @@ int md_system_set(md_system* sys, int field, const double* src) {
     MDB_TRY(ctx_scratch(ctx, static_cast<size_t>(sys->n) * sizeof(double), &staging));
     MDB_CUDA(cudaMemcpyAsync(staging, src, static_cast<size_t>(sys->n) * sizeof(double),
                              cudaMemcpyHostToDevice, ctx->stream));
-    k_set_field<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(
-        sys->cur, field, static_cast<const double*>(staging), sys->n);
+    k_set_fields<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(
+        sys->cur, FieldList{1, {field}}, static_cast<const double*>(staging), sys->n);
     ++ctx->launches;
     MDB_CHECK_LAUNCH();
     // The staging buffer is reused by the next call: finish the host copy first.
@@ -319,8 +329,8 @@ int md_system_get(md_system* sys, int field, double* dst) {
     md_context* ctx = sys->ctx;
     void* staging;
     MDB_TRY(ctx_scratch(ctx, static_cast<size_t>(sys->n) * sizeof(double), &staging));
-    k_get_field<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(
-        sys->cur, field, static_cast<double*>(staging), sys->n);
+    k_get_fields<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(
+        sys->cur, FieldList{1, {field}}, static_cast<double*>(staging), sys->n);
     ++ctx->launches;
     MDB_CHECK_LAUNCH();
     MDB_CUDA(cudaMemcpyAsync(dst, staging, static_cast<size_t>(sys->n) * sizeof(double),
@@ -328,6 +338,45 @@ int md_system_get(md_system* sys, int field, double* dst) {
     MDB_CUDA(cudaStreamSynchronize(ctx->stream));
     return MD_OK;
 }
+
+}  // extern "C"
+
+namespace {
+
+FieldList field_list(const int* fields, int count) {
+    FieldList l;
+    l.count = std::min(count, kMaxFields);
+    for (int c = 0; c < l.count; ++c) l.f[c] = fields[c];
+    return l;
+}
+
+// Host columns to or from the staging columns at `st`, in as few copies as the host
+// layout allows: one for columns end to end, one strided copy for columns at a constant
+// distance (rows of a larger array), else one each.
+template <class P>
+int copy_columns(md_context* ctx, double* st, P const* host, int count, int64_t n, cudaMemcpyKind kind) {
+    const bool in = kind == cudaMemcpyHostToDevice;
+    const auto at = [&](int k) { return reinterpret_cast<uintptr_t>(host[k]); };
+    const size_t width = sizeof(double) * static_cast<size_t>(n);
+    for (int k = 0, run; k < count; k += run) {
+        run = 1;
+        const uintptr_t pitch = k + 1 < count && at(k + 1) > at(k) ? at(k + 1) - at(k) : 0;
+        if (pitch >= width && pitch < (uintptr_t(1) << 31))
+            while (k + run < count && at(k + run) - at(k + run - 1) == pitch) ++run;
+        double* dev = st + static_cast<int64_t>(k) * n;
+        double* h = const_cast<double*>(host[k]);
+        if (run > 1 && pitch != width)
+            MDB_CUDA(in ? cudaMemcpy2DAsync(dev, width, h, pitch, width, run, kind, ctx->stream)
+                        : cudaMemcpy2DAsync(h, pitch, dev, width, width, run, kind, ctx->stream));
+        else
+            MDB_CUDA(cudaMemcpyAsync(in ? dev : h, in ? h : dev, width * run, kind, ctx->stream));
+    }
+    return MD_OK;
+}
+
+}  // namespace
+
+extern "C" {
 
 int md_system_set_fields(md_system* sys, int count, const int* fields, const double* const* src) {
     if (!sys || count < 0 || (count > 0 && (!fields || !src)))
@@ -345,13 +394,12 @@ int md_system_set_fields(md_system* sys, int count, const int* fields, const dou
     double* st = static_cast<double*>(staging);
     // every column's copy is queued before any scatter, so the copy engine
     // streams them back to back; one synchronisation for all
-    for (int k = 0; k < count; ++k)
-        MDB_CUDA(cudaMemcpyAsync(st + k * col, src[k], col * sizeof(double), cudaMemcpyHostToDevice,
-                                 ctx->stream));
-    for (int k = 0; k < count; ++k)
-        k_set_field<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(sys->cur, fields[k],
-                                                                         st + k * col, sys->n);
-    ctx->launches += count;
+    MDB_TRY(copy_columns(ctx, st, src, count, sys->n, cudaMemcpyHostToDevice));
+    for (int k0 = 0; k0 < count; k0 += kMaxFields) {
+        k_set_fields<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(
+            sys->cur, field_list(fields + k0, count - k0), st + k0 * col, sys->n);
+        ++ctx->launches;
+    }
     MDB_CHECK_LAUNCH();
     MDB_CUDA(cudaStreamSynchronize(ctx->stream));
     return MD_OK;
@@ -369,14 +417,13 @@ int md_system_get_fields(md_system* sys, int count, const int* fields, double* c
     void* staging;
     MDB_TRY(ctx_scratch(ctx, col * sizeof(double) * count, &staging));
     double* st = static_cast<double*>(staging);
-    for (int k = 0; k < count; ++k)
-        k_get_field<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(sys->cur, fields[k],
-                                                                         st + k * col, sys->n);
-    ctx->launches += count;
+    for (int k0 = 0; k0 < count; k0 += kMaxFields) {
+        k_get_fields<<<grid_for(sys->n, kBlock), kBlock, 0, ctx->stream>>>(
+            sys->cur, field_list(fields + k0, count - k0), st + k0 * col, sys->n);
+        ++ctx->launches;
+    }
     MDB_CHECK_LAUNCH();
-    for (int k = 0; k < count; ++k)
-        MDB_CUDA(cudaMemcpyAsync(dst[k], st + k * col, col * sizeof(double), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
+    MDB_TRY(copy_columns(ctx, st, dst, count, sys->n, cudaMemcpyDeviceToHost));
     MDB_CUDA(cudaStreamSynchronize(ctx->stream));
     return MD_OK;
 }
