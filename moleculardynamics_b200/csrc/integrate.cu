@@ -302,6 +302,7 @@ __device__ __forceinline__ void nhc_post_body(NhcState* st, const double* ke_sum
     st->ke = ke;
 }
 
+
 __global__ void k_nhc_post(NhcState* st, const double* ke_sum, Weights w) { nhc_post_body(st, ke_sum, w); }
 
 __device__ double nhc_conserved(const NhcState& c) {
@@ -432,8 +433,13 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
 }
 
 // The closing half-kick for a force kernel to apply (the kick of post_force_async).
-KickArgs kick_args(const md_integrator* it, md_system* sys) {
+KickArgs kick_args(const md_integrator* it, md_system* sys, double* rows = nullptr,
+                   int* idx = nullptr) {
     KickArgs k;
+    if (it->kind < 2) {  // a chain's row waits for its closing half
+        k.rows = rows;
+        k.idx = idx;
+    }
     k.vx = sys->cur.vx;
     k.vy = sys->cur.vy;
     k.vz = sys->cur.vz;
@@ -445,8 +451,11 @@ KickArgs kick_args(const md_integrator* it, md_system* sys) {
 }
 
 // The step's end: the closing half-kick with the kinetic energy (unless the force
-// kernel took it: `kicked`), then the chain half of a Nose-Hoover integrator.
-int post_force_async(md_integrator* it, md_system* sys, bool apply_scale, bool kicked = false) {
+// kernel took it: `kicked`), then the chain half of a Nose-Hoover integrator.  rows, idx:
+// the step's thermo row; a force kernel that kicked recorded it already where there is no
+// chain (kick_args gives it the rows).
+int post_force_async(md_integrator* it, md_system* sys, bool apply_scale, bool kicked = false,
+                     double* rows = nullptr, int* idx = nullptr) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
     StepArgs s = step_args(it, sys);
@@ -472,6 +481,11 @@ int post_force_async(md_integrator* it, md_system* sys, bool apply_scale, bool k
             k_reset_scale<<<1, 1, 0, ctx->stream>>>(nhc);
             ++ctx->launches;
         }
+    }
+    if (rows && (nhc || !kicked)) {
+        k_record_at<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEnergy), ctx_result(ctx, kResKE),
+                                              nhc, rows, idx);
+        ++ctx->launches;
     }
     MDB_CHECK_LAUNCH();
     return MD_OK;
@@ -559,7 +573,6 @@ int step_quantize_target(md_integrator* it, md_system* sys, const md_lj* lj, int
 
 int lj_fused_step(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, double* rows,
                   int* idx, bool first) {
-    md_context* ctx = sys->ctx;
     // Kick/drift with the rebuild test of the ForceFn (apps/moldyn_run.cpp:581-587)
     // fused in; the rebuild itself is gated on the device flag.  A mixed force
     // takes the fixed-point positions the kick/drift wrote, re-quantized only after
@@ -570,16 +583,11 @@ int lj_fused_step(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, do
     // a rebuild that re-sorts the atoms also re-quantizes them (q stays current)
     bool requantized = false;
     MDB_TRY(verlet_build_q(v, sys, q, &requantized));
-    const KickArgs ka = kick_args(it, sys);
+    const KickArgs ka = kick_args(it, sys, rows, idx);
     bool kicked = false;
     MDB_TRY(lj_forces_verlet_async(lj, sys, v, q ? v->d_rebuild_flag : nullptr, requantized, &ka,
                                    &kicked));
-    MDB_TRY(post_force_async(it, sys, false, kicked));
-    if (rows) {
-        k_record_at<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEnergy), ctx_result(ctx, kResKE),
-                                              nhc_of(it), rows, idx);
-        ++ctx->launches;
-    }
+    MDB_TRY(post_force_async(it, sys, false, kicked, rows, idx));
     MDB_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -629,16 +637,11 @@ int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj*
     const int64_t l2 = ctx->launches;
     if (rc == MD_OK)
         rc = capture_into(ctx, graph, &cond, 1, [&]() -> int {
-            const KickArgs ka = kick_args(it, sys);
+            const KickArgs ka = kick_args(it, sys, rows, idx);
             bool kicked = false;
             MDB_TRY(lj_forces_verlet_async(lj, sys, v, q ? v->d_rebuild_flag : nullptr,
                                            q != nullptr, &ka, &kicked));
-            MDB_TRY(post_force_async(it, sys, false, kicked));
-            if (rows) {
-                k_record_at<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEnergy),
-                                                      ctx_result(ctx, kResKE), nhc, rows, idx);
-                ++ctx->launches;
-            }
+            MDB_TRY(post_force_async(it, sys, false, kicked, rows, idx));
             MDB_CHECK_LAUNCH();
             return MD_OK;
         }, nullptr);

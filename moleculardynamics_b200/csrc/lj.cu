@@ -258,6 +258,18 @@ __device__ __forceinline__ void near_pair(const LJArgs& a, const Fold3& f3,
 
 constexpr int kBlock = 256;
 
+// The thermo row of a step without a chain (k_record_at), by the block that ended the
+// step's sums out[0..2]: no launch of its own.
+__device__ __forceinline__ void record_row(bool last, const double* out, const KickArgs& kick) {
+    if (!last || threadIdx.x != 0 || !kick.rows) return;
+    double* row = kick.rows + 4 * static_cast<int64_t>(*kick.idx);
+    row[0] = out[0];
+    row[1] = out[1];
+    row[2] = out[2];
+    row[3] = 0.0;
+    ++*kick.idx;
+}
+
 // Full Verlet list, TPA lanes per atom; rows are nbr[i*stride .. +count[i]).
 // Register budget per unroll factor: U gather chains per thread need ~8U more
 // registers, traded against resident blocks per SM.  The mixed kernel is bound by
@@ -379,7 +391,7 @@ __device__ __forceinline__ void lj_verlet_body(
     }
     if constexpr (KICK) {
         double v[3] = {e, vir, ke};
-        grid_reduce_at<3>(v, part, ticket, out, kick.status, block, nblocks);
+        record_row(grid_reduce_at<3>(v, part, ticket, out, kick.status, block, nblocks), out, kick);
     } else {
         double v[2] = {e, vir};
         grid_reduce_at<2>(v, part, ticket, out, nullptr, block, nblocks);
@@ -424,7 +436,7 @@ __device__ __forceinline__ double finish_atom(int64_t i, double fx, double fy, d
 // warps (K values per thread of theirs): each warp's tree, then eight warps by the tree of
 // a warp whose other lanes are zero, then its blocks.
 template <int K, int W>
-__device__ __forceinline__ void reduce_as_two_thread(const double (&s_red)[K][W][32], double* part,
+__device__ __forceinline__ bool reduce_as_two_thread(const double (&s_red)[K][W][32], double* part,
                                                      unsigned* ticket, double* out,
                                                      uint32_t* status) {
     __shared__ double sm[K][32];
@@ -440,7 +452,7 @@ __device__ __forceinline__ void reduce_as_two_thread(const double (&s_red)[K][W]
     }
     __syncthreads();
     const unsigned warps = gridDim.x * W;
-    grid_reduce_tail<K>(sm, (warps + 7) / 8, ticket, out, status, gridDim.x, [=](unsigned p, int k) {
+    return grid_reduce_tail<K>(sm, (warps + 7) / 8, ticket, out, status, gridDim.x, [=](unsigned p, int k) {
         double v[8];
 #pragma unroll
         for (unsigned w = 0; w < 8; ++w)
@@ -505,7 +517,8 @@ k_lj_wide(const double4* __restrict__ pos, const int* __restrict__ nbr,
     if (i < n && g == 0) ke = finish_atom<KICK>(i, f, fy, fz, fxo, fyo, fzo, kick);
     if (comp == 3 || comp == 4) s_red[comp - 3][0][2 * ai + par] = acc;
     if (KICK && g < 2) s_red[K - 1][0][2 * ai + g] = ke;
-    reduce_as_two_thread<K, 1>(s_red, part, ticket, out, KICK ? kick.status : nullptr);
+    const bool last = reduce_as_two_thread<K, 1>(s_red, part, ticket, out, KICK ? kick.status : nullptr);
+    if (KICK) record_row(last, out, kick);
 }
 
 // The same for systems of 64 to 256 atoms per SM, four lanes an atom: lanes p and
@@ -569,7 +582,9 @@ k_lj_quad(const double4* __restrict__ pos, const int* __restrict__ nbr,
     } else if (KICK) {
         s_red[K - 1][tw][tl + g] = ke;
     }
-    reduce_as_two_thread<K, kTwoWarps>(s_red, part, ticket, out, KICK ? kick.status : nullptr);
+    const bool last =
+        reduce_as_two_thread<K, kTwoWarps>(s_red, part, ticket, out, KICK ? kick.status : nullptr);
+    if (KICK) record_row(last, out, kick);
 }
 
 // One system's arguments of the batched force pass.
@@ -814,7 +829,7 @@ k_lj_halo(const int4* __restrict__ q, const double4* __restrict__ pd, const int*
     }
     if constexpr (KICK) {  // energy, virial and kinetic energy (result slots 0, 1, 2)
         double v[3] = {e, vir, ke};
-        grid_reduce<3>(v, part, ticket, out, kick.status);
+        record_row(grid_reduce<3>(v, part, ticket, out, kick.status), out, kick);
     } else {
         double v[2] = {e, vir};
         grid_reduce<2>(v, part, ticket, out);
@@ -974,7 +989,7 @@ k_lj_halo64(const double4* __restrict__ pos, const int* __restrict__ nbr,
     }
     if constexpr (KICK) {
         double v[3] = {acc.e, acc.vir, ke};
-        grid_reduce<3>(v, part, ticket, out, kick.status);
+        record_row(grid_reduce<3>(v, part, ticket, out, kick.status), out, kick);
     } else {
         double v[2] = {acc.e, acc.vir};
         grid_reduce<2>(v, part, ticket, out);

@@ -386,6 +386,10 @@ struct KickArgs {
     const double* inv_mass = nullptr;
     double half_dt = 0.0;
     uint32_t* status = nullptr;  // MD_STATUS_NONFINITE when a sum is not finite
+    // thermo rows and the next row's index: the block that ends the sums also records the
+    // step (null: it does not)
+    double* rows = nullptr;
+    int* idx = nullptr;
 };
 // Verlet-list LJ forces, energy and virial.  With `kick`, a force kernel that can
 // apply it does, and sets *kicked; otherwise *kicked stays false and the caller
