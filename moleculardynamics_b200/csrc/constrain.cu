@@ -89,26 +89,69 @@ struct Mol {
     double x[3], y[3], z[3];
 };
 
-// min_image_wrapped of a bond: shorter than half the box, so only a molecule that straddles
-// its edge folds; one high-word compare per component finds that out.
+// min_image_wrapped without a branch for every value but those near half a box length: the
+// high word of |v| tells an unfolded component from one that is a box length off.  A warp
+// nearly always holds a molecule that straddles the box's edge, so a branch would run both
+// ways each time.  False: the general fold has to decide.
+__device__ __forceinline__ bool fold_straight(double v, const FoldBounds& b, double& out) {
+    const int h = __double2hiint(v) & 0x7fffffff;
+    const double w = __dsub_rn(v, copysign(b.L, v));
+    const bool keep = h < __double2hiint(b.lo);
+    out = keep ? v : w;
+    return keep || (h > __double2hiint(b.hi) && h < __double2hiint(b.top));
+}
+
+__device__ __noinline__ double fold_general(double v, double L, double invL) {
+    return fold_wrapped(v, fold_bounds(L, invL));
+}
+
 __device__ __forceinline__ void min_image_bond(const Fold3& f, const Mol& r, int i, int j, double& dx,
                                                double& dy, double& dz) {
-    dx = fold_pair(__dsub_rn(r.x[i], r.x[j]), f.b[0], true);
-    dy = fold_pair(__dsub_rn(r.y[i], r.y[j]), f.b[1], true);
-    dz = fold_pair(__dsub_rn(r.z[i], r.z[j]), f.b[2], true);
+    const double vx = __dsub_rn(r.x[i], r.x[j]), vy = __dsub_rn(r.y[i], r.y[j]),
+                 vz = __dsub_rn(r.z[i], r.z[j]);
+    const bool ox = fold_straight(vx, f.b[0], dx), oy = fold_straight(vy, f.b[1], dy),
+               oz = fold_straight(vz, f.b[2], dz);
+    if (!(ox && oy && oz)) {
+        dx = fold_general(vx, f.b[0].L, f.b[0].invL);
+        dy = fold_general(vy, f.b[1].L, f.b[1].invL);
+        dz = fold_general(vz, f.b[2].L, f.b[2].invL);
+    }
+}
+
+__device__ __noinline__ double divide(double a, double b) { return __ddiv_rn(a, b); }
+
+__device__ __forceinline__ bool masses_divide_fast(const double m[3]) {
+    return divides_fast(m[0]) && divides_fast(m[1]) && divides_fast(m[2]);
+}
+
+// r -= b gi on one end and += b gj on the other, where `act`; a select, not a branch.
+__device__ __forceinline__ void shift_ends(Mol& r, int i, int j, const double (&b)[3], double gi,
+                                           double gj, bool act) {
+    const double xi = __dsub_rn(r.x[i], __dmul_rn(b[0], gi)), xj = __dadd_rn(r.x[j], __dmul_rn(b[0], gj));
+    const double yi = __dsub_rn(r.y[i], __dmul_rn(b[1], gi)), yj = __dadd_rn(r.y[j], __dmul_rn(b[1], gj));
+    const double zi = __dsub_rn(r.z[i], __dmul_rn(b[2], gi)), zj = __dadd_rn(r.z[j], __dmul_rn(b[2], gj));
+    r.x[i] = act ? xi : r.x[i];
+    r.y[i] = act ? yi : r.y[i];
+    r.z[i] = act ? zi : r.z[i];
+    r.x[j] = act ? xj : r.x[j];
+    r.y[j] = act ? yj : r.y[j];
+    r.z[j] = act ? zj : r.z[j];
 }
 
 // rigid_water.cpp:61-116 for one molecule.  Returns iterations, -1 (no
 // convergence) or -2 (singular denominator).
 // The reference bond vectors, the inverse-mass sums and the masses' reciprocals do not
 // change during the iterations; they are formed once before the sweeps.  A sweep is a chain
-// of dependent FP64 operations, three constraints one after another: its divisions (126
-// clocks each, two of the three in the chain) are quotients by shared or precomputed
-// reciprocals, correctly rounded like the divisions they replace.  1,029 sites at tolerance
-// 1e-12: 65 us with IEEE divisions and 256-thread blocks, 40 us so.
+// of dependent FP64 operations, three constraints one after another, so what counts is the
+// chain: its divisions (126 clocks each, two of the three in the chain) are quotients by
+// shared or precomputed reciprocals, correctly rounded like the divisions they replace
+// (divide() for masses or denominators outside their range), and nothing in a constraint
+// branches: the fold and the update select.  1,029 sites at tolerance 1e-12: 65 us with IEEE
+// divisions and 256-thread blocks, 40 us with quotients, 32 us without branches.
 __device__ int shake_molecule(Mol& r, const Mol& ref, const double m[3], const RigidArgs& a,
                               const Fold3& f3) {
     double b[3][3], two_inv_mass[3];
+    const bool fast = masses_divide_fast(m);
     const double im[3] = {__ddiv_rn(1.0, m[0]), __ddiv_rn(1.0, m[1]), __ddiv_rn(1.0, m[2])};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -119,6 +162,7 @@ __device__ int shake_molecule(Mol& r, const Mol& ref, const double m[3], const R
     }
     for (int it = 0; it < a.max_iterations; ++it) {
         bool open = false;  // some violation above the tolerance (worst > tolerance)
+        bool singular = false;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const int i = cons_i(c), j = cons_j(c);
@@ -126,20 +170,21 @@ __device__ int shake_molecule(Mol& r, const Mol& ref, const double m[3], const R
             double ax, ay, az;
             min_image_bond(f3, r, i, j, ax, ay, az);
             const double s = __dsub_rn(norm2_exact(ax, ay, az), d2);
-            if (fabs(s) > a.within[c]) open = true;
-            if (fabs(s) <= a.within[c]) continue;
-            const double bx = b[c][0], by = b[c][1], bz = b[c][2];
-            const double denom = __dmul_rn(two_inv_mass[c], dot_exact(ax, ay, az, bx, by, bz));
-            if (fabs(denom) < 1e-30) return -2;
-            const double g = quotient(s, denom, reciprocal(denom));
-            const double gi = quotient(g, m[i], im[i]), gj = quotient(g, m[j], im[j]);
-            r.x[i] = __dsub_rn(r.x[i], __dmul_rn(bx, gi));
-            r.y[i] = __dsub_rn(r.y[i], __dmul_rn(by, gi));
-            r.z[i] = __dsub_rn(r.z[i], __dmul_rn(bz, gi));
-            r.x[j] = __dadd_rn(r.x[j], __dmul_rn(bx, gj));
-            r.y[j] = __dadd_rn(r.y[j], __dmul_rn(by, gj));
-            r.z[j] = __dadd_rn(r.z[j], __dmul_rn(bz, gj));
+            const bool act = !(fabs(s) <= a.within[c]);
+            open |= fabs(s) > a.within[c];
+            const double denom =
+                __dmul_rn(two_inv_mass[c], dot_exact(ax, ay, az, b[c][0], b[c][1], b[c][2]));
+            singular |= act && fabs(denom) < 1e-30;  // no update from here on
+            double g = quotient(s, denom, reciprocal(denom));
+            double gi = quotient(g, m[i], im[i]), gj = quotient(g, m[j], im[j]);
+            if (!(fast && divides_fast(fabs(denom))) && act) {
+                g = divide(s, denom);
+                gi = divide(g, m[i]);
+                gj = divide(g, m[j]);
+            }
+            shift_ends(r, i, j, b[c], gi, gj, act && !singular);
         }
+        if (singular) return -2;
         if (!open) return it + 1;
     }
     return -1;
@@ -295,10 +340,11 @@ __device__ __forceinline__ int constrain_positions(Mol& r, const Mol& ref, const
 // Positions are fixed during the iterations: the bond vectors, their squared
 // lengths times the inverse-mass sums and the reciprocals the sweeps divide with are
 // formed once before them.  1,029 sites: 54 us with IEEE divisions (two in each
-// constraint's chain) and 256-thread blocks, 22 us so.
+// constraint's chain) and 256-thread blocks, 22 us so (with or without branches).
 __device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const RigidArgs& a,
                                const Fold3& f3) {
     double b[3][3], mass_norm[3], inv_norm[3];
+    bool fast = masses_divide_fast(m);
     const double im[3] = {__ddiv_rn(1.0, m[0]), __ddiv_rn(1.0, m[1]), __ddiv_rn(1.0, m[2])};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -308,6 +354,7 @@ __device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const Ri
         const double inv_mass_sum = __dadd_rn(im[i], im[j]);
         mass_norm[c] = __dmul_rn(inv_mass_sum, norm2_exact(b[c][0], b[c][1], b[c][2]));
         inv_norm[c] = reciprocal(mass_norm[c]);
+        fast = fast && divides_fast(mass_norm[c]);
     }
     for (int it = 0; it < a.max_iterations; ++it) {
         bool open = false;  // some |r.v| / d2 above the tolerance
@@ -318,16 +365,16 @@ __device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const Ri
             const double ux = __dsub_rn(v.x[i], v.x[j]), uy = __dsub_rn(v.y[i], v.y[j]),
                          uz = __dsub_rn(v.z[i], v.z[j]);
             const double rv = dot_exact(ax, ay, az, ux, uy, uz);
-            if (fabs(rv) > a.within[c]) open = true;
-            if (fabs(rv) <= a.within[c]) continue;
-            const double k = quotient(rv, mass_norm[c], inv_norm[c]);
-            const double ki = quotient(k, m[i], im[i]), kj = quotient(k, m[j], im[j]);
-            v.x[i] = __dsub_rn(v.x[i], __dmul_rn(ax, ki));
-            v.y[i] = __dsub_rn(v.y[i], __dmul_rn(ay, ki));
-            v.z[i] = __dsub_rn(v.z[i], __dmul_rn(az, ki));
-            v.x[j] = __dadd_rn(v.x[j], __dmul_rn(ax, kj));
-            v.y[j] = __dadd_rn(v.y[j], __dmul_rn(ay, kj));
-            v.z[j] = __dadd_rn(v.z[j], __dmul_rn(az, kj));
+            const bool act = !(fabs(rv) <= a.within[c]);
+            open |= fabs(rv) > a.within[c];
+            double k = quotient(rv, mass_norm[c], inv_norm[c]);
+            double ki = quotient(k, m[i], im[i]), kj = quotient(k, m[j], im[j]);
+            if (!fast && act) {
+                k = divide(rv, mass_norm[c]);
+                ki = divide(k, m[i]);
+                kj = divide(k, m[j]);
+            }
+            shift_ends(v, i, j, b[c], ki, kj, act);
         }
         if (!open) return it + 1;
     }
