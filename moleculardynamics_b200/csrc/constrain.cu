@@ -340,10 +340,49 @@ __device__ __forceinline__ int constrain_positions(Mol& r, const Mol& ref, const
 // Positions are fixed during the iterations: the bond vectors, their squared
 // lengths times the inverse-mass sums and the reciprocals the sweeps divide with are
 // formed once before them.  1,029 sites: 54 us with IEEE divisions (two in each
-// constraint's chain) and 256-thread blocks, 22 us so (with or without branches).
-__device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const RigidArgs& a,
+// constraint's chain) and 256-thread blocks, 22.7 us with quotients, 20.3 us with the sweeps
+// for divisors outside their range in a loop of their own, so that this one has no branch.
+template <bool GENERAL>
+__device__ __forceinline__ int rattle_sweeps(Mol& v, const double (&b)[3][3], const double (&norm)[3],
+                                             const double (&inv_norm)[3], const double (&m)[3],
+                                             const double (&im)[3], const RigidArgs& a) {
+    for (int it = 0; it < a.max_iterations; ++it) {
+        bool open = false;  // some |r.v| / d2 above the tolerance
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int i = cons_i(c), j = cons_j(c);
+            const double ux = __dsub_rn(v.x[i], v.x[j]), uy = __dsub_rn(v.y[i], v.y[j]),
+                         uz = __dsub_rn(v.z[i], v.z[j]);
+            const double rv = dot_exact(b[c][0], b[c][1], b[c][2], ux, uy, uz);
+            const bool act = !(fabs(rv) <= a.within[c]);
+            open |= fabs(rv) > a.within[c];
+            double ki, kj;
+            if (GENERAL) {
+                const double k = __ddiv_rn(rv, norm[c]);
+                ki = __ddiv_rn(k, m[i]);
+                kj = __ddiv_rn(k, m[j]);
+            } else {
+                const double k = quotient(rv, norm[c], inv_norm[c]);
+                ki = quotient(k, m[i], im[i]);
+                kj = quotient(k, m[j], im[j]);
+            }
+            shift_ends(v, i, j, b[c], ki, kj, act);
+        }
+        if (!open) return it + 1;
+    }
+    return -1;
+}
+
+__device__ __noinline__ int rattle_sweeps_general(Mol& v, const double (&b)[3][3],
+                                                  const double (&norm)[3], const double (&m)[3],
+                                                  const RigidArgs& a) {
+    const double none[3] = {0.0, 0.0, 0.0};
+    return rattle_sweeps<true>(v, b, norm, none, m, none, a);
+}
+
+__device__ int rattle_molecule(const Mol& r, Mol& v, const double (&m)[3], const RigidArgs& a,
                                const Fold3& f3) {
-    double b[3][3], mass_norm[3], inv_norm[3];
+    double b[3][3], norm[3], inv_norm[3];
     bool fast = masses_divide_fast(m);
     const double im[3] = {__ddiv_rn(1.0, m[0]), __ddiv_rn(1.0, m[1]), __ddiv_rn(1.0, m[2])};
 #pragma unroll
@@ -352,33 +391,22 @@ __device__ int rattle_molecule(const Mol& r, Mol& v, const double m[3], const Ri
         min_image_wrapped(f3, r.x[i], r.y[i], r.z[i], r.x[j], r.y[j], r.z[j], b[c][0], b[c][1],
                           b[c][2]);
         const double inv_mass_sum = __dadd_rn(im[i], im[j]);
-        mass_norm[c] = __dmul_rn(inv_mass_sum, norm2_exact(b[c][0], b[c][1], b[c][2]));
-        inv_norm[c] = reciprocal(mass_norm[c]);
-        fast = fast && divides_fast(mass_norm[c]);
+        norm[c] = __dmul_rn(inv_mass_sum, norm2_exact(b[c][0], b[c][1], b[c][2]));
+        inv_norm[c] = reciprocal(norm[c]);
+        fast = fast && divides_fast(norm[c]);
     }
-    for (int it = 0; it < a.max_iterations; ++it) {
-        bool open = false;  // some |r.v| / d2 above the tolerance
+    if (fast) return rattle_sweeps<false>(v, b, norm, inv_norm, m, im, a);
+    Mol w = v;
+    double b2[3][3], norm2[3], m2[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int i = cons_i(c), j = cons_j(c);
-            const double ax = b[c][0], ay = b[c][1], az = b[c][2];
-            const double ux = __dsub_rn(v.x[i], v.x[j]), uy = __dsub_rn(v.y[i], v.y[j]),
-                         uz = __dsub_rn(v.z[i], v.z[j]);
-            const double rv = dot_exact(ax, ay, az, ux, uy, uz);
-            const bool act = !(fabs(rv) <= a.within[c]);
-            open |= fabs(rv) > a.within[c];
-            double k = quotient(rv, mass_norm[c], inv_norm[c]);
-            double ki = quotient(k, m[i], im[i]), kj = quotient(k, m[j], im[j]);
-            if (!fast && act) {
-                k = divide(rv, mass_norm[c]);
-                ki = divide(k, m[i]);
-                kj = divide(k, m[j]);
-            }
-            shift_ends(v, i, j, b[c], ki, kj, act);
-        }
-        if (!open) return it + 1;
+    for (int c = 0; c < 3; ++c) {
+        norm2[c] = norm[c];
+        m2[c] = m[c];
+        for (int d = 0; d < 3; ++d) b2[c][d] = b[c][d];
     }
-    return -1;
+    const int it = rattle_sweeps_general(w, b2, norm2, m2, a);
+    v = w;
+    return it;
 }
 
 struct MolSlots {
