@@ -18,13 +18,12 @@
 
 namespace mdb {
 int nhc_pre_async(md_integrator* it, md_context* ctx, const double* ke_now);
-int nhc_post_async(md_integrator* it, md_context* ctx, const double* ke_sum);
+int nhc_post_async(md_integrator* it, md_context* ctx, const double* ke_sum, const double* ev,
+                   double* rows, int* idx);
 int nhc_apply_scale_async(md_integrator* it, md_system* sys);
-int record_async(md_context* ctx, const double* ev, const double* ke, const NhcState* nhc,
-                 double* row);
-int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated);
+int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated, bool checked);
+int ewald_disp_args(md_ewald* ew, md_context* ctx, int nblocks, DispArgs* d);
 int system_kinetic_async(md_system* sys, int slot);
-int record_at_async(md_context* ctx, const NhcState* nhc, double* rows, int* idx);
 }  // namespace mdb
 
 namespace mdb {
@@ -510,54 +509,72 @@ struct CvvArgs {
 
 // constrained_velocity_verlet.hpp:31-52: reference = r; kick; drift (no wrap);
 // SHAKE along the reference bonds; velocity correction shift / dt.  An NHC
-// pending scale (if any) is applied to the velocities first.
-__global__ void k_cvv_pre(md_atoms a, const int* __restrict__ slot, int64_t nmol, CvvArgs c,
-                          const NhcState* nhc, int* max_it, uint32_t* status) {
+// pending scale (if any) is applied to the velocities first.  With CHECK the kernel also
+// reduces the sites' top-2 displacement since the last list build and writes the rebuild
+// flag, which saves the pass that would read the positions again (4.3 us and a launch a
+// step at 1,029 sites).
+template <bool CHECK>
+__global__ void __launch_bounds__(kBlock, 1)
+k_cvv_pre(md_atoms a, const int* __restrict__ slot, int64_t nmol, CvvArgs c, const NhcState* nhc,
+          int* max_it, uint32_t* status, DispArgs d) {
     const int64_t m = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (m >= nmol) return;
+    double far1 = 0.0, far2 = 0.0;
     const Fold3 f3 = fold3_of(c.box);
-    const MolSlots ms = mol_slots(slot, m);
-    Mol r, v, ref, unc;
-    load_pos(a, ms, r);
-    load_vel(a, ms, v);
-    ref = r;
-    double mass[3];
-    const double sc = nhc ? nhc->scale : 1.0;
+    if (m < nmol) {
+        const MolSlots ms = mol_slots(slot, m);
+        Mol r, v, ref, unc;
+        load_pos(a, ms, r);
+        load_vel(a, ms, v);
+        ref = r;
+        double mass[3];
+        const double sc = nhc ? nhc->scale : 1.0;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int s = ms.s[k];
-        mass[k] = a.mass[s];
-        if (nhc) {
-            v.x[k] = __dmul_rn(v.x[k], sc);
-            v.y[k] = __dmul_rn(v.y[k], sc);
-            v.z[k] = __dmul_rn(v.z[k], sc);
+        for (int k = 0; k < 3; ++k) {
+            const int s = ms.s[k];
+            mass[k] = a.mass[s];
+            if (nhc) {
+                v.x[k] = __dmul_rn(v.x[k], sc);
+                v.y[k] = __dmul_rn(v.y[k], sc);
+                v.z[k] = __dmul_rn(v.z[k], sc);
+            }
+            const double kc = __ddiv_rn(c.half_dt, mass[k]);  // 0.5 * dt_ / mass
+            v.x[k] = __dadd_rn(v.x[k], __dmul_rn(a.fx[s], kc));
+            v.y[k] = __dadd_rn(v.y[k], __dmul_rn(a.fy[s], kc));
+            v.z[k] = __dadd_rn(v.z[k], __dmul_rn(a.fz[s], kc));
+            r.x[k] = __dadd_rn(r.x[k], __dmul_rn(v.x[k], c.dt));
+            r.y[k] = __dadd_rn(r.y[k], __dmul_rn(v.y[k], c.dt));
+            r.z[k] = __dadd_rn(r.z[k], __dmul_rn(v.z[k], c.dt));
         }
-        const double kc = __ddiv_rn(c.half_dt, mass[k]);  // 0.5 * dt_ / mass
-        v.x[k] = __dadd_rn(v.x[k], __dmul_rn(a.fx[s], kc));
-        v.y[k] = __dadd_rn(v.y[k], __dmul_rn(a.fy[s], kc));
-        v.z[k] = __dadd_rn(v.z[k], __dmul_rn(a.fz[s], kc));
-        r.x[k] = __dadd_rn(r.x[k], __dmul_rn(v.x[k], c.dt));
-        r.y[k] = __dadd_rn(r.y[k], __dmul_rn(v.y[k], c.dt));
-        r.z[k] = __dadd_rn(r.z[k], __dmul_rn(v.z[k], c.dt));
-    }
-    unc = r;
-    const int it = constrain_positions(r, ref, mass, c.ra, f3);
-    report(it, max_it, status, MD_STATUS_SHAKE_DIVERGED);
+        unc = r;
+        const int it = constrain_positions(r, ref, mass, c.ra, f3);
+        report(it, max_it, status, MD_STATUS_SHAKE_DIVERGED);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        double sx, sy, sz;
-        min_image_wrapped(f3, r.x[k], r.y[k], r.z[k], unc.x[k], unc.y[k], unc.z[k], sx, sy, sz);
-        v.x[k] = __dadd_rn(v.x[k], __dmul_rn(sx, c.inv_dt));
-        v.y[k] = __dadd_rn(v.y[k], __dmul_rn(sy, c.inv_dt));
-        v.z[k] = __dadd_rn(v.z[k], __dmul_rn(sz, c.inv_dt));
+        for (int k = 0; k < 3; ++k) {
+            double sx, sy, sz;
+            min_image_wrapped(f3, r.x[k], r.y[k], r.z[k], unc.x[k], unc.y[k], unc.z[k], sx, sy, sz);
+            v.x[k] = __dadd_rn(v.x[k], __dmul_rn(sx, c.inv_dt));
+            v.y[k] = __dadd_rn(v.y[k], __dmul_rn(sy, c.inv_dt));
+            v.z[k] = __dadd_rn(v.z[k], __dmul_rn(sz, c.inv_dt));
+        }
+        store_pos(a, ms, r);
+        store_vel(a, ms, v);
+        if (CHECK) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const double4 o = d.ref[ms.s[k]];
+                double dx, dy, dz;
+                min_image_wrapped(f3, r.x[k], r.y[k], r.z[k], o.x, o.y, o.z, dx, dy, dz);
+                top2_insert(far1, far2, norm2_exact(dx, dy, dz));
+            }
+        }
     }
-    store_pos(a, ms, r);
-    store_vel(a, ms, v);
+    if (CHECK) top2_grid(far1, far2, d);
 }
 
 // The kinetic-energy sum of a launch of one-warp blocks, in the order and tree of a launch
 // of kBlock threads a block (grid_reduce there): four consecutive blocks are its four warps.
-__device__ __forceinline__ void warp_blocks_reduce(double v, double* part, unsigned* ticket,
+// True in the block that finished the sum.
+__device__ __forceinline__ bool warp_blocks_reduce(double v, double* part, unsigned* ticket,
                                                    double* out) {
     static_assert(kBlock == 128, "four warps a block");
     const unsigned lane = threadIdx.x, nb = gridDim.x;
@@ -568,7 +585,7 @@ __device__ __forceinline__ void warp_blocks_reduce(double v, double* part, unsig
         __threadfence();
         t = atomicAdd(ticket, 1u);
     }
-    if (__shfl_sync(0xffffffffu, t, 0) != nb - 1) return;
+    if (__shfl_sync(0xffffffffu, t, 0) != nb - 1) return false;
     __threadfence();
     const auto at = [=](unsigned b) { return b < nb ? __ldcg(part + b) : 0.0; };
     const unsigned parts = (nb + 3) / 4;
@@ -584,12 +601,42 @@ __device__ __forceinline__ void warp_blocks_reduce(double v, double* part, unsig
         *out = (s[0] + s[2]) + (s[1] + s[3]);
         *ticket = 0u;
     }
+    return true;
+}
+
+// What is left of a fused step once the kinetic energy is known.  SPC/E potential energy
+// from the Ewald result slots (spce_forcefield.cpp:40): disp + elrc + (real + reciprocal +
+// self + intra); self = self_coef * sum q^2.  Then, without a thermostat, the thermo row at
+// a device-held index.
+struct SpceTail {
+    const double* ew;  // null: not a fused step.  Slots: 0 real, 1 W real, 2 lj, 3 W lj,
+                       // 4 intra, 5 W intra, 6 sum q^2, 7 recip, 8 W recip
+    double elrc, self_coef;
+    double* ev;
+    double* rows;  // null: no row here
+    int* idx;
+};
+
+__device__ __forceinline__ void spce_tail(const SpceTail& t, double ke) {
+    const double* ew = t.ew;
+    const double self = t.self_coef * ew[6];
+    const double e = ew[2] + t.elrc + (ew[0] + ew[7] + self + ew[4]);
+    const double w = ew[1] + ew[3] + ew[5] + ew[8];
+    t.ev[0] = e;
+    t.ev[1] = w;
+    if (!t.rows) return;
+    double* row = t.rows + 4 * static_cast<int64_t>(*t.idx);
+    row[0] = e;
+    row[1] = w;
+    row[2] = ke;
+    row[3] = 0.0;
+    ++*t.idx;
 }
 
 // constrained_velocity_verlet.hpp:54-56: kick; RATTLE; kinetic-energy sum.
 __global__ void __launch_bounds__(kBlock)
 k_cvv_post(md_atoms a, const int* __restrict__ slot, int64_t nmol, CvvArgs c, int* max_it,
-           uint32_t* status, double* part, unsigned* ticket, double* ke_out) {
+           uint32_t* status, double* part, unsigned* ticket, double* ke_out, SpceTail tail) {
     const int64_t m = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     double ke[1] = {0.0};
     if (m < nmol) {
@@ -615,17 +662,9 @@ k_cvv_post(md_atoms a, const int* __restrict__ slot, int64_t nmol, CvvArgs c, in
         for (int k = 0; k < 3; ++k)
             ke[0] += 0.5 * mass[k] * (v.x[k] * v.x[k] + v.y[k] * v.y[k] + v.z[k] * v.z[k]);
     }
-    if (blockDim.x == 32) warp_blocks_reduce(ke[0], part, ticket, ke_out);
-    else grid_reduce<1>(ke, part, ticket, ke_out);
-}
-
-// SPC/E potential energy from the Ewald result slots (spce_forcefield.cpp:40):
-// disp + elrc + (real + reciprocal + self + intra); self = self_coef * sum q^2.
-__global__ void k_spce_total(const double* ew, double elrc, double self_coef, double* ev) {
-    // ew slots: 0 real, 1 W real, 2 lj, 3 W lj, 4 intra, 5 W intra, 6 recip, 7 W recip, 8 sum q^2
-    const double self = self_coef * ew[8];
-    ev[0] = ew[2] + elrc + (ew[0] + ew[6] + self + ew[4]);
-    ev[1] = ew[1] + ew[3] + ew[5] + ew[7];
+    const bool last = blockDim.x == 32 ? warp_blocks_reduce(ke[0], part, ticket, ke_out)
+                                       : grid_reduce<1>(ke, part, ticket, ke_out);
+    if (last && threadIdx.x == 0 && tail.ew) spce_tail(tail, *ke_out);  // thread 0 wrote it
 }
 
 Box3 box_of(const md_system* sys) {
@@ -723,32 +762,34 @@ int spce_loop_begin(md_integrator* it, md_system* sys, md_ewald* ff, const char*
     return MD_OK;
 }
 
-// One step; `first` feeds the chain the entry kinetic energy, `row` (device,
-// or null) receives [energy, virial, kinetic, conserved].  The step's kinetic
-// energy is left in the kResKE result slot.
-int spce_step_async(SpceLoop& L, bool first, double* row) {
+// One step; `first` feeds the chain the entry kinetic energy; rows and idx (device, or
+// null): where [energy, virial, kinetic, conserved] goes, at the index held there.  The
+// step's kinetic energy is left in the kResKE result slot.
+int spce_step_async(SpceLoop& L, bool first, double* rows, int* idx) {
     md_system* sys = L.sys;
     md_integrator* it = L.it;
     md_context* ctx = sys->ctx;
     if (L.nhc) MDB_TRY(nhc_pre_async(it, ctx, first ? ctx_result(ctx, kResKE) : nullptr));
     if (L.nmol > 0) {
         sys->wrapped = false;  // molecules keep their own image
-        k_cvv_pre<<<grid_for(L.nmol, L.block), L.block, 0, ctx->stream>>>(
-            sys->cur, sys->slot, L.nmol, cvv_args(it, sys), L.nhc, it->counters.as<int>(),
-            ctx->d_status);
+        DispArgs d;
+        MDB_TRY(ewald_disp_args(L.ff, ctx, L.g, &d));
+        k_cvv_pre<true><<<L.g, L.block, 0, ctx->stream>>>(sys->cur, sys->slot, L.nmol,
+                                                          cvv_args(it, sys), L.nhc,
+                                                          it->counters.as<int>(), ctx->d_status, d);
         ++ctx->launches;
     }
-    MDB_TRY(ewald_eval_async(L.ff, sys, 1, true));
-    k_spce_total<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEwald), L.elrc, L.self_coef,
-                                           ctx_result(ctx, kResEnergy));
+    MDB_TRY(ewald_eval_async(L.ff, sys, 1, true, L.nmol > 0));
     double* part;  // fetched after the Ewald sum, which may grow the partials
     MDB_TRY(ctx_partials(ctx, static_cast<size_t>(L.g), &part));
+    const SpceTail tail{ctx_result(ctx, kResEwald), L.elrc, L.self_coef,
+                        ctx_result(ctx, kResEnergy), L.nhc ? nullptr : rows, idx};
     k_cvv_post<<<L.g, L.block, 0, ctx->stream>>>(sys->cur, sys->slot, L.nmol, cvv_args(it, sys),
                                                it->counters.as<int>() + 1, ctx->d_status, part,
-                                               ctx_counter(ctx, 8), ctx_result(ctx, kResKE));
-    ctx->launches += 2;
-    if (L.nhc) MDB_TRY(nhc_post_async(it, ctx, ctx_result(ctx, kResKE)));
-    if (row) MDB_TRY(record_async(ctx, ctx_result(ctx, kResEnergy), ctx_result(ctx, kResKE), L.nhc, row));
+                                               ctx_counter(ctx, 8), ctx_result(ctx, kResKE), tail);
+    ++ctx->launches;
+    if (L.nhc)
+        MDB_TRY(nhc_post_async(it, ctx, ctx_result(ctx, kResKE), ctx_result(ctx, kResEnergy), rows, idx));
     MDB_CHECK_LAUNCH();
     return MD_OK;
 }
@@ -811,8 +852,9 @@ int constrained_pre_force(md_integrator* it, md_system* sys) {
     if (nmol > 0) {
         const int block = mol_block(ctx, nmol);
         sys->wrapped = false;  // molecules keep their own image
-        k_cvv_pre<<<grid_for(nmol, block), block, 0, ctx->stream>>>(
-            sys->cur, sys->slot, nmol, cvv_args(it, sys), nhc, it->counters.as<int>(), ctx->d_status);
+        k_cvv_pre<false><<<grid_for(nmol, block), block, 0, ctx->stream>>>(
+            sys->cur, sys->slot, nmol, cvv_args(it, sys), nhc, it->counters.as<int>(),
+            ctx->d_status, DispArgs{});
         ++ctx->launches;
         MDB_CHECK_LAUNCH();
     }
@@ -828,11 +870,12 @@ int constrained_post_force(md_integrator* it, md_system* sys, bool apply_scale) 
     MDB_TRY(ctx_partials(ctx, static_cast<size_t>(g), &part));
     k_cvv_post<<<g, block, 0, ctx->stream>>>(sys->cur, sys->slot, nmol, cvv_args(it, sys),
                                              it->counters.as<int>() + 1, ctx->d_status, part,
-                                             ctx_counter(ctx, 8), ctx_result(ctx, kResKE));
+                                             ctx_counter(ctx, 8), ctx_result(ctx, kResKE),
+                                             SpceTail{});
     ++ctx->launches;
     MDB_CHECK_LAUNCH();
     if (it->kind == 4) {
-        MDB_TRY(nhc_post_async(it, ctx, ctx_result(ctx, kResKE)));
+        MDB_TRY(nhc_post_async(it, ctx, ctx_result(ctx, kResKE), nullptr, nullptr, nullptr));
         if (apply_scale) MDB_TRY(nhc_apply_scale_async(it, sys));
     }
     if (apply_scale) return status_to_error(ctx);
@@ -1001,9 +1044,7 @@ int md_run_spce(md_integrator* it, md_system* sys, md_ewald* ff, int64_t steps, 
     // One step with its thermo row at a device-held index; after the first (eager)
     // step it is captured once and replayed, unless kernel timing is on.
     auto one_step = [&](bool first) -> int {
-        MDB_TRY(spce_step_async(L, first, nullptr));
-        if (rows.ptr) MDB_TRY(record_at_async(ctx, L.nhc, rows.as<double>(), idx.as<int>()));
-        return MD_OK;
+        return spce_step_async(L, first, rows.as<double>(), idx.as<int>());
     };
     BlockGraph bg;
     const bool want_graph = ctx->graphs && !ctx->timing && steps >= 4;
@@ -1045,7 +1086,7 @@ int md_water_rdf_run(md_integrator* it, md_system* sys, md_ewald* ff, md_rdf* rd
     // scaled toward the target and put back on the constraint surface (RATTLE's
     // velocity half, rigid_water.cpp:107-162, as constrainVelocities does).
     auto eq_block = [&](int64_t steps, bool first, bool rescale) -> int {
-        for (int64_t k = 0; k < steps; ++k) MDB_TRY(spce_step_async(L, first && k == 0, nullptr));
+        for (int64_t k = 0; k < steps; ++k) MDB_TRY(spce_step_async(L, first && k == 0, nullptr, nullptr));
         if (!rescale) return MD_OK;
         MDB_TRY(md_system_rescale_temperature(sys, dof, temperature));
         if (L.nmol > 0) {
@@ -1062,7 +1103,7 @@ int md_water_rdf_run(md_integrator* it, md_system* sys, md_ewald* ff, md_rdf* rd
     // binned every sample_every steps.
     auto prod_block = [&](int64_t steps, bool first, bool frame) -> int {
         for (int64_t k = 0; k < steps; ++k) {
-            MDB_TRY(spce_step_async(L, first && k == 0, nullptr));
+            MDB_TRY(spce_step_async(L, first && k == 0, nullptr, nullptr));
             k_sum_temperature<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResKE),
                                                         static_cast<double>(dof), acc.as<double>());
             ++ctx->launches;

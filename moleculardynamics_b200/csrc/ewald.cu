@@ -27,6 +27,7 @@
 namespace mdb {
 int verlet_build(md_verlet* v, md_system* sys, bool conditional);
 int verlet_check(md_verlet* v, md_system* sys);
+DispArgs disp_args(md_verlet* v, md_context* ctx, double* part);
 int verlet_ensure_ready(md_verlet* v, md_system* sys, const char* who);
 }  // namespace mdb
 
@@ -200,7 +201,8 @@ k_ewald_real(const double4* __restrict__ pos, const double* __restrict__ q,
 }
 
 // Intramolecular correction (ewald.cpp:79-110) per atom over its molecule partners
-// (original indices, CSR); adds to forces.  out[0..1]: E_intra, W_intra.
+// (original indices, CSR); adds to forces, and the sum of q^2 of the self term with it.
+// out[0..2]: E_intra, W_intra, sum q^2.
 __global__ void k_ewald_intra(const double4* __restrict__ pos, const double* __restrict__ q,
                               const int* __restrict__ orig, const int* __restrict__ slot,
                               const int* __restrict__ off, const int* __restrict__ partner,
@@ -209,10 +211,11 @@ __global__ void k_ewald_intra(const double4* __restrict__ pos, const double* __r
                               double* out) {
     const int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     const Fold3 f3 = fold3_of(box);
-    double e = 0.0, vir = 0.0;
+    double e = 0.0, vir = 0.0, q2 = 0.0;
     if (k < n) {
         const double4 pi = pos[k];
         const int oi = orig[k];
+        q2 = q[k] * q[k];
         double fx = 0.0, fy = 0.0, fz = 0.0;
         for (int p = off[oi]; p < off[oi + 1]; ++p) {
             const int oj = partner[p];
@@ -242,17 +245,8 @@ __global__ void k_ewald_intra(const double4* __restrict__ pos, const double* __r
             fzo[k] += fz;
         }
     }
-    double v[2] = {e, vir};
-    grid_reduce<2>(v, part, ticket, out);
-}
-
-__global__ void k_sum_q2(const double* __restrict__ q, int64_t n, double* part, unsigned* ticket,
-                         double* out) {
-    double v[1] = {0.0};
-    for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < n;
-         k += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        v[0] += q[k] * q[k];
-    grid_reduce<1>(v, part, ticket, out);
+    double v[3] = {e, vir, q2};
+    grid_reduce<3>(v, part, ticket, out);
 }
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
@@ -662,7 +656,7 @@ void launch_real(md_system* sys, md_verlet* v, const RealArgs& a, int mode, int 
 
 // Result slots inside kResEwald (doubles).
 enum {
-    kEwReal = 0, kEwRealW, kEwLj, kEwLjW, kEwIntra, kEwIntraW, kEwRecip, kEwRecipW, kEwQ2,
+    kEwReal = 0, kEwRealW, kEwLj, kEwLjW, kEwIntra, kEwIntraW, kEwQ2, kEwRecip, kEwRecipW,
     kEwCount
 };
 
@@ -788,8 +782,8 @@ int ewald_kvectors(md_ewald* ew, const double box[3], double alpha) {
     return MD_OK;
 }
 
-int ewald_list_gated(md_ewald* ew, md_system* sys) {
-    MDB_TRY(verlet_check(ew->list, sys));
+int ewald_list_gated(md_ewald* ew, md_system* sys, bool checked) {
+    if (!checked) MDB_TRY(verlet_check(ew->list, sys));
     return verlet_build(ew->list, sys, true);
 }
 
@@ -816,10 +810,6 @@ int ewald_list(md_ewald* ew, md_system* sys) {
 
 }  // namespace
 
-// Everything of one evaluation, asynchronously; results land in kResEwald slots.
-// mode: 0 energies only, 1 zero + accumulate forces, 2 accumulate onto forces.
-// gated: the neighbour list is maintained by device-decided rebuilds (no host
-// synchronisation; the list must already be built for this system).
 // k-space forces added to the system's forces (charge = false), or
 // dE_recip/dq added to dq (device order); the coefficients must be current.
 int recip_force_async(md_ewald* ew, md_system* sys, const KArgs& ka, bool charge, double* dq) {
@@ -883,14 +873,19 @@ KArgs kargs_of(md_ewald* ew, const md_system* sys) {
     return ka;
 }
 
-int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated) {
+// Everything of one evaluation, asynchronously; results land in kResEwald slots.
+// mode: 0 energies only, 1 zero + accumulate forces, 2 accumulate onto forces.
+// gated: the neighbour list is maintained by device-decided rebuilds (no host
+// synchronisation; the list must already be built for this system); checked: the kernel
+// that moved the sites has set the list's rebuild flag (ewald_disp_args).
+int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated, bool checked) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
     double min_len = std::min(sys->box[0], std::min(sys->box[1], sys->box[2]));
     const double alpha = ew->alpha_in > 0.0 ? ew->alpha_in : 5.6 / min_len;  // ewald.cpp:40
     ew->alpha = alpha;
     if (gated) {
-        MDB_TRY(ewald_list_gated(ew, sys));
+        MDB_TRY(ewald_list_gated(ew, sys, checked));
     } else {
         MDB_TRY(ewald_topology(ew, sys));
         if (!ew->pme) MDB_TRY(ewald_kvectors(ew, sys->box, alpha));
@@ -927,9 +922,6 @@ int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated) {
             sys->cur.pos, sys->cur.charge, sys->cur.orig, sys->slot, ew->partner_off.as<int>(),
             ew->partner_idx.as<int>(), n, box, a, mode != 0 ? 1 : 0, sys->cur.fx, sys->cur.fy,
             sys->cur.fz, part, ctx_counter(ctx, 5), res + kEwIntra);
-        const int g = std::min<int>(grid_for(n, kBlock), ctx->sm_count * 4);
-        k_sum_q2<<<g, kBlock, 0, ctx->stream>>>(sys->cur.charge, n, part, ctx_counter(ctx, 6),
-                                                res + kEwQ2);
     }
     // reciprocal space
     ctx_time_begin(ctx, MD_KERNEL_EWALD_RECIP);
@@ -969,7 +961,15 @@ int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated) {
     }
     ctx_time_end(ctx, MD_KERNEL_EWALD_RECIP);
     MDB_CHECK_LAUNCH();
-    ctx->launches += 6;
+    ctx->launches += 5;
+    return MD_OK;
+}
+
+// The displacement check of the built list, for a kernel of nblocks blocks that moves the sites.
+int ewald_disp_args(md_ewald* ew, md_context* ctx, int nblocks, DispArgs* d) {
+    double* part;
+    MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(nblocks), &part));
+    *d = disp_args(ew->list, ctx, part);
     return MD_OK;
 }
 
@@ -1054,7 +1054,7 @@ int md_ewald_compute(md_ewald* ew, md_system* sys, int mode, double terms[4], do
     if (!ew || !sys) return fail(MD_ERR_INVALID_ARGUMENT, "md_ewald_compute: NULL argument");
     if (mode < 0 || mode > 2) return fail(MD_ERR_INVALID_ARGUMENT, "md_ewald_compute: mode %d", mode);
     if (sys->ctx != ew->ctx) return fail(MD_ERR_INVALID_ARGUMENT, "md_ewald_compute: context mismatch");
-    MDB_TRY(ewald_eval_async(ew, sys, mode, false));
+    MDB_TRY(ewald_eval_async(ew, sys, mode, false, false));
     MDB_TRY(ewald_read(ew, sys->ctx));
     fill_terms(ew, terms, virial);
     return MD_OK;
@@ -1133,7 +1133,7 @@ int md_ewald_charge_gradient(md_ewald* ew, md_system* sys, double* dedq) {
     if (n == 0) return MD_OK;
     md_context* ctx = sys->ctx;
     // energies (also builds the list, topology, k vectors and S(k))
-    MDB_TRY(ewald_eval_async(ew, sys, 0, false));
+    MDB_TRY(ewald_eval_async(ew, sys, 0, false, false));
     DevBuf buf;
     MDB_TRY(buf.ensure(2 * sizeof(double) * static_cast<size_t>(n)));
     double* dq = buf.as<double>();
@@ -1163,7 +1163,7 @@ int md_ewald_real_hvp(md_ewald* ew, md_system* sys, const double* u, double* out
     const int64_t n = sys->n;
     if (n == 0) return MD_OK;
     md_context* ctx = sys->ctx;
-    MDB_TRY(ewald_eval_async(ew, sys, 0, false));  // list and alpha for this state
+    MDB_TRY(ewald_eval_async(ew, sys, 0, false, false));  // list and alpha for this state
     DevBuf buf;
     MDB_TRY(buf.ensure(4 * sizeof(double4) * static_cast<size_t>(n)));
     double4* uo = buf.as<double4>();
@@ -1230,7 +1230,7 @@ int md_spce_compute(md_ewald* ew, md_system* sys, int forces, double* energy, do
     if (sys->n % 3 != 0)  // spce_forcefield.cpp:14-17
         return fail(MD_ERR_INVALID_ARGUMENT,
                     "SpceForceField: atom count is not a multiple of 3; expected O,H,H triples");
-    MDB_TRY(ewald_eval_async(ew, sys, forces ? 1 : 0, false));
+    MDB_TRY(ewald_eval_async(ew, sys, forces ? 1 : 0, false, false));
     MDB_TRY(ewald_read(ew, sys->ctx));
     double terms[4], vir;
     fill_terms(ew, terms, &vir);

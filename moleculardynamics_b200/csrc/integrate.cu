@@ -313,25 +313,28 @@ __device__ double nhc_conserved(const NhcState& c) {
     return sum;
 }
 
-// thermo row: energy, virial, kinetic energy, conserved contribution.
-__global__ void k_record(const double* ev, const double* ke, const NhcState* nhc, double* row) {
-    row[0] = ev[0];
-    row[1] = ev[1];
-    row[2] = nhc ? nhc->ke : *ke;
-    row[3] = nhc ? nhc_conserved(*nhc) : 0.0;
-}
-
 __global__ void k_conserved(const NhcState* nhc, double* out) { *out = nhc_conserved(*nhc); }
 
 // Thermo row at a device-held index (graph replays cannot change a pointer).
-__global__ void k_record_at(const double* ev, const double* ke, const NhcState* nhc, double* rows,
-                            int* idx) {
+__device__ __forceinline__ void record_at(const double* ev, const double* ke, const NhcState* nhc,
+                                          double* rows, int* idx) {
     double* row = rows + 4 * static_cast<int64_t>(*idx);
     row[0] = ev[0];
     row[1] = ev[1];
     row[2] = nhc ? nhc->ke : *ke;
     row[3] = nhc ? nhc_conserved(*nhc) : 0.0;
     ++*idx;
+}
+
+__global__ void k_record_at(const double* ev, const double* ke, const NhcState* nhc, double* rows,
+                            int* idx) {
+    record_at(ev, ke, nhc, rows, idx);
+}
+
+__global__ void k_nhc_post_record(NhcState* st, const double* ke_sum, Weights w, const double* ev,
+                                  double* rows, int* idx) {
+    nhc_post_body(st, ke_sum, w);
+    record_at(ev, ke_sum, st, rows, idx);
 }
 
 // Opens the rebuild branch of a step graph when the fused check asked for one.
@@ -553,14 +556,6 @@ int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check) {
 
 int vv_post_async(md_integrator* it, md_system* sys) { return post_force_async(it, sys, true); }
 
-int record_at_async(md_context* ctx, const NhcState* nhc, double* rows, int* idx) {
-    k_record_at<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEnergy), ctx_result(ctx, kResKE), nhc,
-                                          rows, idx);
-    ++ctx->launches;
-    MDB_CHECK_LAUNCH();
-    return MD_OK;
-}
-
 // The fixed-point position buffer the step's first kernel fills for a mixed force (null
 // when the force is FP64).
 int step_quantize_target(md_integrator* it, md_system* sys, const md_lj* lj, int4** q) {
@@ -675,8 +670,12 @@ int nhc_pre_async(md_integrator* it, md_context* ctx, const double* ke_now) {
     return MD_OK;
 }
 
-int nhc_post_async(md_integrator* it, md_context* ctx, const double* ke_sum) {
-    k_nhc_post<<<1, 1, 0, ctx->stream>>>(it->chain_state.as<NhcState>(), ke_sum, yoshida());
+// With rows, the thermo row of [ev, kinetic, conserved] at *idx follows in the same launch.
+int nhc_post_async(md_integrator* it, md_context* ctx, const double* ke_sum, const double* ev,
+                   double* rows, int* idx) {
+    NhcState* st = it->chain_state.as<NhcState>();
+    if (rows) k_nhc_post_record<<<1, 1, 0, ctx->stream>>>(st, ke_sum, yoshida(), ev, rows, idx);
+    else k_nhc_post<<<1, 1, 0, ctx->stream>>>(st, ke_sum, yoshida());
     ++ctx->launches;
     MDB_CHECK_LAUNCH();
     return MD_OK;
@@ -690,14 +689,6 @@ int nhc_apply_scale_async(md_integrator* it, md_system* sys) {
         ++ctx->launches;
     }
     k_reset_scale<<<1, 1, 0, ctx->stream>>>(nhc);
-    ++ctx->launches;
-    MDB_CHECK_LAUNCH();
-    return MD_OK;
-}
-
-int record_async(md_context* ctx, const double* ev, const double* ke, const NhcState* nhc,
-                 double* row) {
-    k_record<<<1, 1, 0, ctx->stream>>>(ev, ke, nhc, row);
     ++ctx->launches;
     MDB_CHECK_LAUNCH();
     return MD_OK;
