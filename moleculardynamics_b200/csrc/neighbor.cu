@@ -349,10 +349,117 @@ __device__ __forceinline__ bool beyond_half(double v, int half_hi) {
     return (__double2hiint(v) & 0x7fffffff) >= half_hi;
 }
 
+// A cell as the list build sees it: the centre its atoms' FP32 offsets are relative to, the
+// conservative thresholds, and the ranges of the 27 cells around it, end to end.
+struct BuildCell {
+    double ox, oy, oz;
+    float hi_thr;            // the list cutoff^2, widened by 2^-12
+    float hwx, hwy, hwz;     // half widths of the cell's box
+    int half_x, half_y, half_z;
+    int beg, excl, total;    // lane q: cell q's first atom, candidates before it; all candidates
+};
+
+__device__ __forceinline__ BuildCell build_cell(const GridArgs& g, const int* __restrict__ start,
+                                                double rl2, int r, int lane) {
+    BuildCell b;
+    const int cell = g.cell_of_rank[r];
+    const int cx = cell % g.nx, cy = (cell / g.nx) % g.ny, cz = cell / (g.nx * g.ny);
+    b.ox = -0.5 * g.box.L[0] + (cx + 0.5) * g.wx;
+    b.oy = -0.5 * g.box.L[1] + (cy + 0.5) * g.wy;
+    b.oz = -0.5 * g.box.L[2] + (cz + 0.5) * g.wz;
+    b.hi_thr = static_cast<float>(rl2 * (1.0 + 1.0 / 4096.0));
+    // half widths of the cell's box, widened a little (its atoms were binned with
+    // the reference arithmetic, their offsets here are FP64 then FP32)
+    b.hwx = static_cast<float>(0.5 * g.wx * (1.0 + 1e-6)) + 1e-6f;
+    b.hwy = static_cast<float>(0.5 * g.wy * (1.0 + 1e-6)) + 1e-6f;
+    b.hwz = static_cast<float>(0.5 * g.wz * (1.0 + 1e-6)) + 1e-6f;
+    // high words of just under half the box: offsets below them need no image
+    b.half_x = __double2hiint(0.4999 * g.box.L[0]);
+    b.half_y = __double2hiint(0.4999 * g.box.L[1]);
+    b.half_z = __double2hiint(0.4999 * g.box.L[2]);
+    int cnt = 0;
+    b.beg = 0;
+    if (lane < 27) {
+        int jx = cx + (lane % 3) - 1, jy = cy + ((lane / 3) % 3) - 1, jz = cz + (lane / 9) - 1;
+        jx = jx < 0 ? jx + g.nx : (jx >= g.nx ? jx - g.nx : jx);
+        jy = jy < 0 ? jy + g.ny : (jy >= g.ny ? jy - g.ny : jy);
+        jz = jz < 0 ? jz + g.nz : (jz >= g.nz ? jz - g.nz : jz);
+        const int rr = g.rank_of_cell[jx + g.nx * (jy + g.ny * jz)];
+        b.beg = start[rr];
+        cnt = start[rr + 1] - b.beg;
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    b.total = __shfl_sync(0xffffffffu, incl, 31);
+    b.excl = incl - cnt;
+    return b;
+}
+
+// The atom index of candidate f of the cell's flattened ranges (any f); whole warps.
+__device__ __forceinline__ int build_candidate(const BuildCell& b, int f) {
+    int q = 0;  // the last cell that starts at or before candidate f
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, b.excl, q + step) <= f) q += step;
+    return __shfl_sync(0xffffffffu, b.beg, q) + (f - __shfl_sync(0xffffffffu, b.excl, q));
+}
+
+// A candidate's offset from the cell centre (nearest image); true when it is live and
+// within the list cutoff of the cell's own box (a quarter of the 27-cell volume is farther
+// from every atom of the cell).  Whole warps.
+__device__ __forceinline__ bool build_offset(const BuildCell& b, const GridArgs& g, bool live,
+                                             const double4& p, float& x, float& y, float& z) {
+    double vx = 0.0, vy = 0.0, vz = 0.0;
+    bool wraps = false;
+    if (live) {
+        vx = p.x - b.ox;
+        vy = p.y - b.oy;
+        vz = p.z - b.oz;
+        wraps = beyond_half(vx, b.half_x) || beyond_half(vy, b.half_y) || beyond_half(vz, b.half_z);
+    }
+    if (__any_sync(0xffffffffu, wraps)) {  // rint below is 0 otherwise
+        vx -= g.box.L[0] * rint(vx * g.box.inv[0]);
+        vy -= g.box.L[1] * rint(vy * g.box.inv[1]);
+        vz -= g.box.L[2] * rint(vz * g.box.inv[2]);
+    }
+    x = static_cast<float>(vx);
+    y = static_cast<float>(vy);
+    z = static_cast<float>(vz);
+    const float ex = fmaxf(fabsf(x) - b.hwx, 0.f), ey = fmaxf(fabsf(y) - b.hwy, 0.f),
+                ez = fmaxf(fabsf(z) - b.hwz, 0.f);
+    return live && fmaf(ez, ez, fmaf(ey, ey, ex * ex)) < b.hi_thr;
+}
+
+// An atom of the cell, relative to its centre.
+__device__ __forceinline__ void build_atom(const BuildCell& b, const GridArgs& g, const double4& p,
+                                           float& x, float& y, float& z) {
+    double ux = p.x - b.ox, uy = p.y - b.oy, uz = p.z - b.oz;
+    ux -= g.box.L[0] * rint(ux * g.box.inv[0]);
+    uy -= g.box.L[1] * rint(uy * g.box.inv[1]);
+    uz -= g.box.L[2] * rint(uz * g.box.inv[2]);
+    x = static_cast<float>(ux);
+    y = static_cast<float>(uy);
+    z = static_cast<float>(uz);
+}
+
+__device__ __forceinline__ void build_report(int local_max, int lane, int stride, uint32_t* status,
+                                             int* max_count) {
+    const int mx = __reduce_max_sync(0xffffffffu, local_max);
+    if (lane == 0) {
+        if (mx > 0) atomicMax(max_count, mx);
+        if (mx > stride) atomicOr(status, MD_STATUS_NEIGHBOR_OVERFLOW);
+    }
+}
+
 // One warp per (Morton-ranked) cell; device order == sorted order, so cell r holds
 // atoms [start[r], start[r+1]).  The candidates of the 27 surrounding cells are
 // staged in shared memory once per cell as FP32 coordinates relative to the cell
-// centre (nearest periodic image), 32 at a time of the 27 ranges end to end (a lane finds
+// centre (nearest periodic image), 32 at a time of the 27 ranges end to end, in order and
+// without those too far from the cell for any of its atoms (a lane finds
 // its range by binary search; range by range a few atoms a cell left most lanes idle:
 // whole build of 256,000 atoms at density 0.3 291 us, 210 so, of 1,048,576 at 0.8442 760
 // and 717); then each lane takes one atom of the cell and
@@ -382,75 +489,23 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
     const int wid = static_cast<int>(block) * kBuildWarps + warp;
     const int r = wid / groups, grp = wid % groups;
     if (r >= g.ncells) return;
-    const int cell = g.cell_of_rank[r];
-    const int cx = cell % g.nx, cy = (cell / g.nx) % g.ny, cz = cell / (g.nx * g.ny);
-    const double ox = -0.5 * g.box.L[0] + (cx + 0.5) * g.wx;
-    const double oy = -0.5 * g.box.L[1] + (cy + 0.5) * g.wy;
-    const double oz = -0.5 * g.box.L[2] + (cz + 0.5) * g.wz;
-    const float hi_thr = static_cast<float>(rl2 * (1.0 + 1.0 / 4096.0));
-    // half widths of the cell's box, widened a little (its atoms were binned with
-    // the reference arithmetic, their offsets here are FP64 then FP32)
-    const float hwx = static_cast<float>(0.5 * g.wx * (1.0 + 1e-6)) + 1e-6f;
-    const float hwy = static_cast<float>(0.5 * g.wy * (1.0 + 1e-6)) + 1e-6f;
-    const float hwz = static_cast<float>(0.5 * g.wz * (1.0 + 1e-6)) + 1e-6f;
-    // high words of just under half the box: offsets below them need no image
-    const int half_x = __double2hiint(0.4999 * g.box.L[0]), half_y = __double2hiint(0.4999 * g.box.L[1]),
-              half_z = __double2hiint(0.4999 * g.box.L[2]);
-    // the 27 neighbour cell ranges (lane q holds cell q of the stencil)
-    int beg = 0, cnt = 0;
-    if (lane < 27) {
-        int jx = cx + (lane % 3) - 1, jy = cy + ((lane / 3) % 3) - 1, jz = cz + (lane / 9) - 1;
-        jx = jx < 0 ? jx + g.nx : (jx >= g.nx ? jx - g.nx : jx);
-        jy = jy < 0 ? jy + g.ny : (jy >= g.ny ? jy - g.ny : jy);
-        jz = jz < 0 ? jz + g.nz : (jz >= g.nz ? jz - g.nz : jz);
-        const int rr = g.rank_of_cell[jx + g.nx * (jy + g.ny * jz)];
-        beg = start[rr];
-        cnt = start[rr + 1] - beg;
-    }
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int excl = incl - cnt;
+    const BuildCell bc = build_cell(g, start, rl2, r, lane);
+    const int total = bc.total;
+    const float hi_thr = bc.hi_thr;
     const int a0 = start[r], a1 = start[r + 1];
     int local_max = 0;
     for (int wb = 0; wb < total; wb += kMaxCand) {
         const int wlen = min(kMaxCand, total - wb);
         __syncwarp();
-        // stage candidates [wb, wb + wlen), 32 of the flattened cell ranges at a time, keeping
-        // only those within the list cutoff of the cell's own box (a quarter of the 27-cell
-        // volume is farther from every atom of the cell); order is kept
+        // stage candidates [wb, wb + wlen)
         int ns = 0;
         for (int fb = wb; fb < wb + wlen; fb += 32) {
-            const int f = fb + lane;
-            int q = 0;  // the last cell that starts at or before candidate f
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1)
-                if (__shfl_sync(0xffffffffu, excl, q + step) <= f) q += step;
-            const int j = __shfl_sync(0xffffffffu, beg, q) + (f - __shfl_sync(0xffffffffu, excl, q));
-            double vx = 0.0, vy = 0.0, vz = 0.0;
-            const bool live = f < wb + wlen;
-            bool wraps = false;
-            if (live) {
-                const double4 pj = ldg4(pos + j);
-                vx = pj.x - ox;
-                vy = pj.y - oy;
-                vz = pj.z - oz;
-                wraps = beyond_half(vx, half_x) || beyond_half(vy, half_y) || beyond_half(vz, half_z);
-            }
-            if (__any_sync(0xffffffffu, wraps)) {  // rint below is 0 otherwise
-                vx -= g.box.L[0] * rint(vx * g.box.inv[0]);
-                vy -= g.box.L[1] * rint(vy * g.box.inv[1]);
-                vz -= g.box.L[2] * rint(vz * g.box.inv[2]);
-            }
-            const float cx32 = static_cast<float>(vx), cy32 = static_cast<float>(vy),
-                        cz32 = static_cast<float>(vz);
-            const float ex = fmaxf(fabsf(cx32) - hwx, 0.f), ey = fmaxf(fabsf(cy32) - hwy, 0.f),
-                        ez = fmaxf(fabsf(cz32) - hwz, 0.f);
-            const bool keep = live && fmaf(ez, ez, fmaf(ey, ey, ex * ex)) < hi_thr;
+            const int j = build_candidate(bc, fb + lane);
+            const bool live = fb + lane < wb + wlen;
+            double4 pj = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (live) pj = ldg4(pos + j);
+            float cx32, cy32, cz32;
+            const bool keep = build_offset(bc, g, live, pj, cx32, cy32, cz32);
             const unsigned m = __ballot_sync(0xffffffffu, keep);
             if (keep) {
                 const int tt = ns + __popc(m & ((1u << lane) - 1u)), pr = tt >> 1, h = tt & 1;
@@ -473,18 +528,10 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
         for (int ib = a0 + 32 * grp; ib < a1; ib += 32 * groups) {
             const int i = ib + lane;
             const bool active = i < a1;
-            double4 pi = make_double4(0.0, 0.0, 0.0, 0.0);
             float fx = 0.f, fy = 0.f, fz = 0.f;
             int c = 0;
             if (active) {
-                pi = pos[i];
-                double ux = pi.x - ox, uy = pi.y - oy, uz = pi.z - oz;
-                ux -= g.box.L[0] * rint(ux * g.box.inv[0]);
-                uy -= g.box.L[1] * rint(uy * g.box.inv[1]);
-                uz -= g.box.L[2] * rint(uz * g.box.inv[2]);
-                fx = static_cast<float>(ux);
-                fy = static_cast<float>(uy);
-                fz = static_cast<float>(uz);
+                build_atom(bc, g, pos[i], fx, fy, fz);
                 c = wb == 0 ? 0 : count[i];
             }
             int* row = nbr + static_cast<int64_t>(active ? i : 0) * stride;
@@ -513,11 +560,7 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
             }
         }
     }
-    const int mx = __reduce_max_sync(0xffffffffu, local_max);
-    if (lane == 0) {
-        if (mx > 0) atomicMax(max_count, mx);
-        if (mx > stride) atomicOr(status, MD_STATUS_NEIGHBOR_OVERFLOW);
-    }
+    build_report(local_max, lane, stride, status, max_count);
 }
 
 __global__ void __launch_bounds__(kBuildWarps * 32)
@@ -526,6 +569,194 @@ k_verlet_cells(const double4* __restrict__ pos, const int* __restrict__ start, G
                uint32_t* status, int* max_count, const int* flag, int groups) {
     if (!gate(flag)) return;
     verlet_cells_body(pos, start, g, rl2, nbr, count, stride, status, max_count, groups, blockIdx.x);
+}
+
+// The atoms ib .. ib + A of a cell against 32 candidates, one a lane: the hits in candidate
+// order (a ballot) at the ends of the atoms' rows.
+template <int A>
+__device__ __forceinline__ void append_hits(const float (&fx)[A], const float (&fy)[A],
+                                            const float (&fz)[A], int (&c)[A], float x, float y,
+                                            float z, float thr, int j, int ib, int* rows, int stride,
+                                            unsigned below) {
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+        const float dx = fx[a] - x, dy = fy[a] - y, dz = fz[a] - z;
+        const float r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        const bool h = r2 < thr && j != ib + a;
+        const unsigned m = __ballot_sync(0xffffffffu, h);
+        const int at = c[a] + __popc(m & below);
+        if (h && at < stride) rows[a * stride + at] = j;
+        c[a] += __popc(m);
+    }
+}
+
+// Atoms ib .. min(ib + A, a1) broadcast to every lane; absent ones far from everything.
+template <int A>
+__device__ __forceinline__ void load_atoms(const BuildCell& bc, const GridArgs& g,
+                                           const double4* __restrict__ pos, int ib, int a1, int lane,
+                                           float (&fx)[A], float (&fy)[A], float (&fz)[A],
+                                           int (&c)[A]) {
+    float x = 1e30f, y = 1e30f, z = 1e30f;
+    if (lane < A && ib + lane < a1) build_atom(bc, g, pos[ib + lane], x, y, z);
+#pragma unroll
+    for (int a = 0; a < A; ++a) {
+        fx[a] = __shfl_sync(0xffffffffu, x, a);
+        fy[a] = __shfl_sync(0xffffffffu, y, a);
+        fz[a] = __shfl_sync(0xffffffffu, z, a);
+        c[a] = 0;
+    }
+}
+
+template <int A>
+__device__ __forceinline__ void store_counts(const int (&c)[A], int ib, int a1, int lane, int* count,
+                                             int& local_max) {
+    int own = 0;
+#pragma unroll
+    for (int a = 0; a < A; ++a)
+        if (lane == a) own = c[a];
+    if (lane < A && ib + lane < a1) {
+        count[ib + lane] = own;
+        local_max = max(local_max, own);
+    }
+}
+
+// The same rows for sparse cells: with a lane an atom, two atoms a cell leave 30 lanes idle.
+// Here lanes go over the candidates, 32 a step (the next ones' positions already loading), and
+// a warp takes kSparseAtoms atoms of the cell.  256,000 atoms at density 0.1 (2.2 a cell),
+// whole build: 254 us by lanes over atoms, 180 so (two atoms a warp 204, eight 220); at
+// density 0.3 (6.6 a cell) 213 and 231.
+constexpr int kSparseAtoms = 4;
+
+__device__ __forceinline__ void verlet_sparse_body(const double4* __restrict__ pos,
+                                                   const int* __restrict__ start, const GridArgs& g,
+                                                   double rl2, int* __restrict__ nbr,
+                                                   int* __restrict__ count, int stride,
+                                                   uint32_t* status, int* max_count, int groups,
+                                                   unsigned block) {
+    constexpr int A = kSparseAtoms;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wid = static_cast<int>(block) * kBuildWarps + warp;
+    const int r = wid / groups, grp = wid % groups;
+    if (r >= g.ncells) return;
+    const int a0 = start[r], a1 = start[r + 1];
+    if (a0 + A * grp >= a1) return;
+    const BuildCell bc = build_cell(g, start, rl2, r, lane);
+    const unsigned below = (1u << lane) - 1u;
+    int local_max = 0;
+    for (int ib = a0 + A * grp; ib < a1; ib += A * groups) {
+        float fx[A], fy[A], fz[A];
+        int c[A];
+        load_atoms(bc, g, pos, ib, a1, lane, fx, fy, fz, c);
+        int* const rows = nbr + static_cast<int64_t>(ib) * stride;
+        double4 pn = make_double4(0.0, 0.0, 0.0, 0.0);
+        int jn = build_candidate(bc, lane);
+        if (lane < bc.total) pn = ldg4(pos + jn);
+        for (int fb = 0; fb < bc.total; fb += 32) {
+            const int j = jn;
+            const double4 p = pn;
+            if (fb + 32 < bc.total) {
+                jn = build_candidate(bc, fb + 32 + lane);
+                if (fb + 32 + lane < bc.total) pn = ldg4(pos + jn);
+            }
+            float x, y, z;
+            const bool keep = build_offset(bc, g, true, p, x, y, z) && fb + lane < bc.total;
+            if (!__any_sync(0xffffffffu, keep)) continue;
+            append_hits(fx, fy, fz, c, x, y, z, keep ? bc.hi_thr : 0.f, j, ib, rows, stride, below);
+        }
+        store_counts(c, ib, a1, lane, count, local_max);
+    }
+    build_report(local_max, lane, stride, status, max_count);
+}
+
+__global__ void __launch_bounds__(kBuildWarps * 32)
+k_verlet_sparse(const double4* __restrict__ pos, const int* __restrict__ start, GridArgs g,
+                double rl2, int* __restrict__ nbr, int* __restrict__ count, int stride,
+                uint32_t* status, int* max_count, const int* flag, int groups) {
+    if (!gate(flag)) return;
+    verlet_sparse_body(pos, start, g, rl2, nbr, count, stride, status, max_count, groups, blockIdx.x);
+}
+
+// The same rows for systems too small to fill the GPU with a warp a cell (864 atoms are 27
+// cells; 12,288 water sites at a 10 A cutoff 64 of 192 sites each): a block of kTeamWarps
+// warps stages the candidates of a cell together, each warp 32 of every 256 with the warps'
+// counts giving their places, and then takes kTeamAtoms atoms a warp with lanes over the
+// staged candidates.  More instructions than a lane an atom (a ballot and a scan for every
+// 32 tests), so it loses where the GPU is full: taken while the other build has at most ten
+// warps with atoms per SM.  Whole build, lane an atom and so: 864 atoms 64 and 44 us; 16,384
+// liquid atoms 66 and 58, 32,000 (twelve warps per SM) 72.5 and 70, 119,000 128 and 167; at a
+// cutoff of 5 (126 a cell) 10,976 atoms 209 and 104, 32,000 267 and 194.  Two or eight atoms
+// a warp: 109 and 121 us for the 10,976.
+constexpr int kTeamWarps = 8, kTeamAtoms = 4;
+constexpr int kTeamSlots = 1024;  // staged at a time
+
+__global__ void __launch_bounds__(32 * kTeamWarps)
+k_verlet_team(const double4* __restrict__ pos, const int* __restrict__ start, GridArgs g,
+              double rl2, int* __restrict__ nbr, int* __restrict__ count, int stride,
+              uint32_t* status, int* max_count, const int* flag, int groups) {
+    if (!gate(flag)) return;
+    constexpr int A = kTeamAtoms, kTeam = 32 * kTeamWarps, kAtoms = A * kTeamWarps;
+    __shared__ float4 s_c[kTeamSlots];  // x, y, z relative to the cell centre, index
+    __shared__ int s_n[2][kTeamWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // `groups` blocks share a crowded cell
+    const int r = static_cast<int>(blockIdx.x) / groups, grp = static_cast<int>(blockIdx.x) % groups;
+    const int a0 = start[r], a1 = start[r + 1];
+    if (a0 + kAtoms * grp >= a1) return;  // the whole block
+    const BuildCell bc = build_cell(g, start, rl2, r, lane);
+    const unsigned below = (1u << lane) - 1u;
+    const int mine = 32 * warp + lane;
+    int local_max = 0, ns = 0, buf = 0;
+    bool whole = false;  // every candidate of the cell is staged
+    for (int it = a0 + kAtoms * grp; it < a1; it += kAtoms * groups) {
+        const int ib = it + A * warp;  // may lie beyond a1: the warp still stages
+        float fx[A], fy[A], fz[A];
+        int c[A];
+        load_atoms(bc, g, pos, ib, a1, lane, fx, fy, fz, c);
+        int* const rows = nbr + static_cast<int64_t>(ib) * stride;
+        int fb = 0;
+        do {
+            if (!whole) {
+                __syncthreads();  // the window before has been read
+                const bool first = fb == 0;
+                ns = 0;
+                double4 pn = make_double4(0.0, 0.0, 0.0, 0.0);
+                int jn = build_candidate(bc, fb + mine);
+                if (fb + mine < bc.total) pn = ldg4(pos + jn);
+                for (; fb < bc.total && ns + kTeam <= kTeamSlots; fb += kTeam) {
+                    const int j = jn, next = fb + kTeam + mine;
+                    const double4 p = pn;
+                    if (fb + kTeam < bc.total) {
+                        jn = build_candidate(bc, next);
+                        if (next < bc.total) pn = ldg4(pos + jn);
+                    }
+                    float x, y, z;
+                    const bool keep = build_offset(bc, g, true, p, x, y, z) && fb + mine < bc.total;
+                    const unsigned m = __ballot_sync(0xffffffffu, keep);
+                    if (lane == 0) s_n[buf][warp] = __popc(m);
+                    __syncthreads();  // s_n alternates: one barrier a step orders it
+                    int at = ns + __popc(m & below);
+#pragma unroll
+                    for (int w = 0; w < kTeamWarps; ++w) {
+                        const int k = s_n[buf][w];
+                        if (w < warp) at += k;
+                        ns += k;
+                    }
+                    if (keep) s_c[at] = make_float4(x, y, z, __int_as_float(j));
+                    buf ^= 1;
+                }
+                whole = first && fb >= bc.total;
+                __syncthreads();
+            }
+#pragma unroll 2
+            for (int s = 0; s < ns; s += 32) {
+                const float4 q = s_c[s + lane];
+                append_hits(fx, fy, fz, c, q.x, q.y, q.z, s + lane < ns ? bc.hi_thr : 0.f,
+                            __float_as_int(q.w), ib, rows, stride, below);
+            }
+        } while (!whole && fb < bc.total);
+        store_counts(c, ib, a1, lane, count, local_max);
+    }
+    build_report(local_max, lane, stride, status, max_count);
 }
 
 // Boxes with fewer than 3 cells per side (verlet_list.cpp:26-33): one warp per atom
@@ -842,6 +1073,27 @@ GridArgs make_args(const CellGrid& gr, const md_system* sys) {
     return g;
 }
 
+// Which list build a grid takes, from the mean occupancy of its cells and whether the system
+// fills the GPU; the kernels' comments give both sides of each line.  groups: warps (Team:
+// blocks) that share a cell.
+enum class BuildKind { Cells, Sparse, Team };
+
+struct BuildShape {
+    BuildKind kind;
+    int groups;
+};
+
+BuildShape build_shape(int64_t n, int ncells, int sm_count) {
+    const double mean = static_cast<double>(n) / ncells;
+    const auto share = [=](double spread, int atoms, int most) {
+        return static_cast<int>(std::min<double>(most, std::max(1.0, std::ceil(spread * mean / atoms))));
+    };
+    if (mean < 4.0) return {BuildKind::Sparse, share(1.25, kSparseAtoms, 16)};
+    if (std::max<int64_t>(ncells, n / 32) <= 10 * static_cast<int64_t>(sm_count))
+        return {BuildKind::Team, share(1.25, kTeamAtoms * kTeamWarps, 16)};
+    return {BuildKind::Cells, share(1.5, 32, 16)};
+}
+
 Box3 make_box(const md_system* sys) {
     Box3 b;
     for (int d = 0; d < 3; ++d) {
@@ -906,7 +1158,7 @@ struct RebuildRep {
     const int* flag;
     int64_t n;
     int m;       // cells (0 for a brute-force build)
-    int groups;  // warps per cell in the list build
+    int groups, sparse;  // the list build's warps per cell, and whether lanes go over candidates
     GridArgs g;
     md_atoms cur, alt;
     int* slot;
@@ -1020,8 +1272,12 @@ k_batch_rebuild_cells(const RebuildRep* __restrict__ reps, const int4* __restric
     const int4 e = __ldg(blk + blockIdx.x);
     const RebuildRep& d = reps[e.x];
     if (!gate(d.flag)) return;
-    verlet_cells_body(d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
-                      d.max_count, d.groups, e.y);
+    if (d.sparse)
+        verlet_sparse_body(d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
+                           d.max_count, d.groups, e.y);
+    else
+        verlet_cells_body(d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
+                          d.max_count, d.groups, e.y);
 }
 
 }  // namespace
@@ -1154,13 +1410,20 @@ int verlet_build_impl(md_verlet* v, md_system* sys, const int* flag, int4* q = n
             if (quantized) *quantized = q != nullptr;
         }
         const GridArgs g = make_args(v->grid, sys);
-        // warps per cell from the mean occupancy (crowded cells, e.g. a long cutoff)
-        const double mean = static_cast<double>(n) / v->grid.ncells;
-        const int groups = static_cast<int>(std::min(16.0, std::max(1.0, std::ceil(1.5 * mean / 32.0))));
-        const int64_t warps = static_cast<int64_t>(v->grid.ncells) * groups;
-        k_verlet_cells<<<grid_for(warps, kBuildWarps), kBuildWarps * 32, 0, ctx->stream>>>(
-            sys->cur.pos, start, g, rl2, v->nbr.as<int>(), v->count.as<int>(), v->stride,
-            ctx->d_status, v->d_max_count, flag, groups);
+        const BuildShape sh = build_shape(n, v->grid.ncells, ctx->sm_count);
+        const int64_t units = static_cast<int64_t>(v->grid.ncells) * sh.groups;
+        const auto launch = [&](auto kernel, int blocks, int threads) {
+            kernel<<<blocks, threads, 0, ctx->stream>>>(sys->cur.pos, start, g, rl2,
+                                                        v->nbr.as<int>(), v->count.as<int>(),
+                                                        v->stride, ctx->d_status, v->d_max_count,
+                                                        flag, sh.groups);
+        };
+        if (sh.kind == BuildKind::Sparse)
+            launch(k_verlet_sparse, grid_for(units, kBuildWarps), 32 * kBuildWarps);
+        else if (sh.kind == BuildKind::Team)
+            launch(k_verlet_team, static_cast<int>(units), 32 * kTeamWarps);
+        else
+            launch(k_verlet_cells, grid_for(units, kBuildWarps), 32 * kBuildWarps);
         ++ctx->launches;
         if (v->halo_on && n > 0) MDB_TRY(halo_build(v, sys, flag));
     } else if (n > 0) {
@@ -1296,8 +1559,10 @@ int batch_rebuild_create(const BatchRepView* v, int nrep, BatchRebuild** out) {
         d.flag = lst->d_rebuild_flag;
         d.n = n;
         d.m = m;
-        const double mean = cells ? static_cast<double>(n) / m : 0.0;  // as verlet_build_impl
-        d.groups = static_cast<int>(std::min(16.0, std::max(1.0, std::ceil(1.5 * mean / 32.0))));
+        // as verlet_build_impl; the replicas fill the GPU together, so none takes a team
+        const BuildShape sh = cells ? build_shape(n, m, 0) : BuildShape{BuildKind::Cells, 1};
+        d.groups = sh.groups;
+        d.sparse = sh.kind == BuildKind::Sparse;
         d.g = make_args(lst->grid, sys);
         d.cur = sys->cur;
         d.alt = sys->alt;
