@@ -99,12 +99,11 @@ int capture_to(cudaStream_t stream, cudaGraph_t g, const cudaGraphNode_t* deps, 
     return MD_OK;
 }
 
-// The step graph of batched stage kernels: the chain halves and kick/drift of
-// every replica in one launch (with each replica's rebuild test), the gated
-// rebuild of every replica as one launch per stage (each replica's blocks leave
-// at once unless its own test asked for a rebuild), then the force pass and the
-// kick, kinetic energy, chain half and thermo row of every replica in three
-// launches: about fifteen kernel nodes and no conditional node.  Per replica the
+// The step graph of batched stage kernels: one launch for the chain halves and thermo
+// rows of every replica between two steps, one for its kick/drift and rebuild test, the
+// gated rebuild of every replica as one launch per stage (each replica's blocks leave
+// at once unless its own test asked for a rebuild), then the force pass with the closing
+// kick: about ten kernel nodes and no conditional node.  Per replica the
 // work and its order are those of its solo step.
 struct BatchedStep {
     cudaGraph_t graph = nullptr;
@@ -310,6 +309,7 @@ int md_batch_run(md_batch* b, int64_t steps, double* thermo) {
             }
             md_context* lctx = b->reps[0].sys->ctx;
             MDB_TRY(batch_rebuild_prime(c->step.rebuild, lead, &lctx->launches));
+            MDB_TRY(batch_kick_begin(c->step.kick, lead));
             if (warm) {
                 if (cudaGraphLaunch(c->step.first_exec, lead) != cudaSuccess)
                     return fail(MD_ERR_CUDA, "md_batch_run: graph launch failed");
@@ -319,7 +319,7 @@ int md_batch_run(md_batch* b, int64_t steps, double* thermo) {
                 if (cudaGraphLaunch(c->step.exec, lead) != cudaSuccess)
                     return fail(MD_ERR_CUDA, "md_batch_run: graph launch failed");
             lctx->launches += (steps - 1) * c->step.lead_launches;
-            // The end of the run on the lead stream: the chains' pending scales, then
+            // The end of the run on the lead stream: the last step's, the chains' pending scales, then
             // every replica's thermo rows, status word and energy/virial slots read
             // back, one synchronisation for all.
             MDB_TRY(batch_kick_finish(c->step.kick, lead, &lctx->launches));

@@ -337,11 +337,6 @@ __global__ void k_nhc_post_record(NhcState* st, const double* ke_sum, Weights w,
     record_at(ev, ke_sum, st, rows, idx);
 }
 
-// Opens the rebuild branch of a step graph when the fused check asked for one.
-__global__ void k_set_rebuild(cudaGraphConditionalHandle h, const int* flag) {
-    cudaGraphSetConditional(h, *flag != 0 ? 1u : 0u);
-}
-
 Weights yoshida() {
     // nose_hoover.cpp:15-18
     const double w1 = 1.0 / (2.0 - std::cbrt(2.0));
@@ -386,8 +381,10 @@ NhcState* nhc_of(md_integrator* it) {
 // previous step's rescalings (fused loops, after their first step).
 // q: also write the fixed-point positions for a mixed-precision force.  run: a captured
 // step takes its step number from there (a Langevin step's noise depends on it).
+// branch: the captured step's rebuild branch, which the test opens.
 int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke = true,
-              int4* q = nullptr, const RunCursor* run = nullptr) {
+              int4* q = nullptr, const RunCursor* run = nullptr,
+              const cudaGraphConditionalHandle* branch = nullptr) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
     if (n == 0) return MD_OK;
@@ -403,6 +400,10 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         double* part;
         MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(blocks), &part));
         d = disp_args(check, ctx, part);
+        if (branch) {
+            d.branch = *branch;
+            d.in_graph = 1;
+        }
     }
     if (it->kind == 1) {
         if (it->noise.ptr) {
@@ -506,9 +507,9 @@ namespace {
 
 // One fused LJ step captured as a CUDA graph: [chain half,] kick/drift with the
 // displacement check, a conditional node whose body is the gated neighbour
-// rebuild (opened by k_set_rebuild from the device flag, so steps without a
-// rebuild launch none of its kernels), forces, the closing kick and the thermo
-// row.  Replaying it runs the same kernels with the same arguments as the host
+// rebuild (opened by the displacement check's last block, so steps without a
+// rebuild launch none of its kernels; a kernel of its own to open it cost 3 us a step),
+// forces, the closing kick and the thermo row.  Replaying it runs the same kernels with the same arguments as the host
 // loop.
 struct StepGraph {
     cudaGraph_t graph = nullptr;
@@ -601,11 +602,7 @@ int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj*
     int4* q = nullptr;
     MDB_TRY(step_quantize_target(it, sys, lj, &q));  // allocated by the first, eager step
     rc = capture_into(ctx, graph, nullptr, 0, [&]() -> int {
-        MDB_TRY(pre_force(it, sys, v, false, q, reinterpret_cast<const RunCursor*>(idx)));
-        k_set_rebuild<<<1, 1, 0, ctx->stream>>>(h, v->d_rebuild_flag);
-        ++ctx->launches;
-        MDB_CHECK_LAUNCH();
-        return MD_OK;
+        return pre_force(it, sys, v, false, q, reinterpret_cast<const RunCursor*>(idx), &h);
     }, &leaves);
     const int64_t l1 = ctx->launches;
     cudaGraphNode_t cond = nullptr;
@@ -721,24 +718,46 @@ struct BatchKickRep {
 
 namespace {
 
-// Start-of-step chain halves, one thread per replica (k_nhc_pre without a fresh KE).
+// End-of-step chain half and thermo row (k_nhc_post, k_record_at) of one replica.
+__device__ __forceinline__ void batch_step_end(const BatchKickRep& d, const Weights& w) {
+    if (d.nhc) nhc_post_body(d.nhc, d.ke_out, w);
+    if (d.rows) record_at(d.ev, d.ke_out, d.nhc, d.rows, d.idx);
+}
+
+// Between two steps, one thread per replica: the end of the step before, when one is
+// pending, and the start-of-step chain half (k_nhc_pre without a fresh KE) -- one launch
+// a step for both halves.
 // (The chain half is serial FP64 work, exp-bound; computing it in every kick block
 // instead, or both halves in the block that ends the kinetic-energy sum, measured
 // slower: each block then waits on that chain before its atoms.)
-__global__ void k_batch_nhc_pre(const BatchKickRep* __restrict__ reps, int nrep, Weights w) {
+__global__ void k_batch_turn(const BatchKickRep* __restrict__ reps, int nrep, Weights w, int* pending) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < nrep && reps[r].nhc) nhc_pre_body(reps[r].nhc, nullptr, w);
+    if (r >= nrep) return;
+    const BatchKickRep& d = reps[r];
+    if (pending[r]) batch_step_end(d, w);
+    if (d.nhc) nhc_pre_body(d.nhc, nullptr, w);
+    pending[r] = 1;
+}
+
+// The last step's end.
+__global__ void k_batch_last(const BatchKickRep* __restrict__ reps, int nrep, Weights w, int* pending) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nrep) return;
+    if (pending[r]) batch_step_end(reps[r], w);
+    pending[r] = 0;
 }
 
 // The first step of a run: every row index back to 0, and a chain's start-of-step
 // half from the kinetic energy summed just before (k_nhc_pre with a fresh KE, as
 // the first step of md_run_lj runs it).
-__global__ void k_batch_first_pre(const BatchKickRep* __restrict__ reps, int nrep, Weights w) {
+__global__ void k_batch_first_pre(const BatchKickRep* __restrict__ reps, int nrep, Weights w,
+                                  int* pending) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nrep) return;
     const BatchKickRep& d = reps[r];
     if (d.idx) *d.idx = 0;
     if (d.nhc) nhc_pre_body(d.nhc, d.ke_out, w);
+    pending[r] = 1;
 }
 
 // Kick/drift with the rebuild test of every replica, kBatchKickAtoms atoms per
@@ -753,22 +772,6 @@ __global__ void k_batch_kick_ke(const BatchKickRep* __restrict__ reps, const int
     const int4 e = __ldg(blk + blockIdx.x);
     const BatchKickRep& d = reps[e.x];
     kick_ke_body(d.a, d.n, d.s, d.ke_part, d.ke_ticket, d.ke_out, d.status, e.y, e.z);
-}
-
-// End-of-step chain halves and thermo rows (k_nhc_post, k_record_at), one thread per replica.
-__global__ void k_batch_nhc_post(const BatchKickRep* __restrict__ reps, int nrep, Weights w) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nrep) return;
-    const BatchKickRep& d = reps[r];
-    if (d.nhc) nhc_post_body(d.nhc, d.ke_out, w);
-    if (d.rows) {
-        double* row = d.rows + 4 * static_cast<int64_t>(*d.idx);
-        row[0] = d.ev[0];
-        row[1] = d.ev[1];
-        row[2] = d.nhc ? d.nhc->ke : *d.ke_out;
-        row[3] = d.nhc ? nhc_conserved(*d.nhc) : 0.0;
-        ++*d.idx;
-    }
 }
 
 // The end of a batched run: every chain's pending velocity scale applied (k_scale)
@@ -799,6 +802,7 @@ __global__ void k_batch_reset_scale(const BatchKickRep* __restrict__ reps, int n
 struct BatchKick {
     DevBuf reps, kick_blk, ke_blk;  // block tables (block_table) of the kick launches
     DevBuf kin_reps, kin_blk;  // the chains' entry kinetic energies (first step of a run)
+    DevBuf pending;            // per replica: a step whose end (batch_step_end) is to come
     int nrep = 0, kick_total = 0, ke_total = 0, kin_total = 0;
     bool any_nhc = false, any_rows = false;
 };
@@ -863,6 +867,7 @@ int batch_kick_create(const BatchRepView* v, int nrep, BatchKick** out) {
     int rc = b->reps.ensure(sizeof(BatchKickRep) * h.size());
     if (rc == MD_OK) rc = b->kick_blk.ensure(sizeof(int4) * kt.size());
     if (rc == MD_OK) rc = b->ke_blk.ensure(sizeof(int4) * et.size());
+    if (rc == MD_OK) rc = b->pending.ensure(sizeof(int) * h.size());
     if (rc == MD_OK) rc = b->kin_reps.ensure(sizeof(BatchKineticRep) * kh.size());
     if (rc == MD_OK) rc = b->kin_blk.ensure(sizeof(int4) * std::max<size_t>(nt.size(), 1));
     if (rc == MD_OK &&
@@ -888,9 +893,9 @@ int batch_kick_create(const BatchRepView* v, int nrep, BatchKick** out) {
 }
 
 int batch_kick_pre(BatchKick* b, cudaStream_t stream, int64_t* launches) {
-    if (b->any_nhc) {
-        k_batch_nhc_pre<<<grid_for(b->nrep, 128), 128, 0, stream>>>(b->reps.as<BatchKickRep>(),
-                                                                   b->nrep, yoshida());
+    if (b->any_nhc || b->any_rows) {
+        k_batch_turn<<<grid_for(b->nrep, 128), 128, 0, stream>>>(
+            b->reps.as<BatchKickRep>(), b->nrep, yoshida(), b->pending.as<int>());
         if (launches) ++*launches;
     }
     k_batch_kick_drift<<<b->kick_total, kBlock, 0, stream>>>(b->reps.as<BatchKickRep>(),
@@ -904,7 +909,8 @@ int batch_kick_first(BatchKick* b, cudaStream_t stream, int64_t* launches) {
     MDB_TRY(batch_kinetic_launch(b->kin_reps.as<BatchKineticRep>(), b->kin_blk.as<int4>(),
                                  b->kin_total, stream));
     k_batch_first_pre<<<grid_for(b->nrep, 128), 128, 0, stream>>>(b->reps.as<BatchKickRep>(),
-                                                                 b->nrep, yoshida());
+                                                                 b->nrep, yoshida(),
+                                                                 b->pending.as<int>());
     k_batch_kick_drift<<<b->kick_total, kBlock, 0, stream>>>(b->reps.as<BatchKickRep>(),
                                                              b->kick_blk.as<int4>());
     if (launches) *launches += (b->kin_total > 0 ? 1 : 0) + 2;
@@ -918,16 +924,22 @@ int batch_kick_post(BatchKick* b, cudaStream_t stream, int64_t* launches, bool k
                                                             b->ke_blk.as<int4>());
         if (launches) ++*launches;
     }
-    if (b->any_nhc || b->any_rows) {
-        k_batch_nhc_post<<<grid_for(b->nrep, 128), 128, 0, stream>>>(b->reps.as<BatchKickRep>(),
-                                                                    b->nrep, yoshida());
-        if (launches) ++*launches;
-    }
     MDB_CHECK_LAUNCH();
     return MD_OK;
 }
 
+int batch_kick_begin(BatchKick* b, cudaStream_t stream) {
+    MDB_CUDA(cudaMemsetAsync(b->pending.ptr, 0, sizeof(int) * static_cast<size_t>(b->nrep), stream));
+    return MD_OK;
+}
+
 int batch_kick_finish(BatchKick* b, cudaStream_t stream, int64_t* launches) {
+    if (b->any_nhc || b->any_rows) {
+        k_batch_last<<<grid_for(b->nrep, 128), 128, 0, stream>>>(
+            b->reps.as<BatchKickRep>(), b->nrep, yoshida(), b->pending.as<int>());
+        if (launches) ++*launches;
+        MDB_CHECK_LAUNCH();
+    }
     if (!b->any_nhc) return MD_OK;
     k_batch_scale<<<b->kick_total, kBlock, 0, stream>>>(b->reps.as<BatchKickRep>(),
                                                         b->kick_blk.as<int4>());
@@ -945,6 +957,7 @@ void batch_kick_destroy(BatchKick* b) {
     b->ke_blk.release();
     b->kin_reps.release();
     b->kin_blk.release();
+    b->pending.release();
     delete b;
 }
 

@@ -288,6 +288,9 @@ struct DispArgs {
     unsigned* ticket;
     int* flag;
     double* top2;
+    // a captured step's rebuild branch (when in_graph), opened by the thread that decides
+    cudaGraphConditionalHandle branch;
+    int in_graph;
 };
 
 __device__ inline void top2_grid_at(double a1, double a2, const DispArgs& d, unsigned block,
@@ -341,6 +344,7 @@ __device__ inline void top2_grid_at(double a1, double a2, const DispArgs& d, uns
         const int rebuild = (d.criterion == 0 ? (r1 + r2) > d.skin : r1 > 0.5 * d.skin) ? 1 : 0;
         *d.flag = rebuild;
         *d.ticket = 0u;
+        if (d.in_graph) cudaGraphSetConditional(d.branch, static_cast<unsigned>(rebuild));
     }
 }
 

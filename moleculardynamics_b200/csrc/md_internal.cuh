@@ -231,14 +231,19 @@ struct BatchKick;     // integrate.cu: chain halves, kick/drift (+ rebuild test)
 struct BatchForce;    // lj.cu: the Verlet-list force pass
 struct BatchRebuild;  // neighbor.cu: the gated rebuild of every replica, stage by stage
 int batch_kick_create(const BatchRepView* reps, int nrep, BatchKick** out);
+int batch_kick_begin(BatchKick* b, cudaStream_t stream);  // once per run, before its first step
+// The end of the step before (chain half, thermo row), if one is pending, the chain's next
+// half, and the kick/drift.
 int batch_kick_pre(BatchKick* b, cudaStream_t stream, int64_t* launches);
 // The first step of a run instead of batch_kick_pre: row indices reset, the chains'
 // entry kinetic energies summed afresh, then the same kick/drift.
 int batch_kick_first(BatchKick* b, cudaStream_t stream, int64_t* launches);
 // The step's end: the closing half-kick with the kinetic energy (unless the force
-// kernel took it: `kicked`), then the chain halves and thermo rows.
+// kernel took it: `kicked`); the chain halves and thermo rows follow in the next
+// batch_kick_pre or batch_kick_finish.
 int batch_kick_post(BatchKick* b, cudaStream_t stream, int64_t* launches, bool kicked);
-// After the last step of a batched run: every chain's pending scale applied.
+// After the last step of a batched run: its chain halves and thermo rows, then every
+// chain's pending scale applied.
 int batch_kick_finish(BatchKick* b, cudaStream_t stream, int64_t* launches);
 void batch_kick_destroy(BatchKick* b);
 // MD_ERR_INVALID_ARGUMENT when the replicas' force kernels cannot share a launch

@@ -1178,7 +1178,7 @@ struct RebuildRep {
 };
 
 enum RebuildStage : int {
-    kStZero, kStBin, kStScan, kStScatter, kStOrder, kStPermute, kStCopy, kStCells, kStBrute,
+    kStZero, kStBin, kStScan, kStScatter, kStOrder, kStPermute, kStCopy, kStCells,
     kRebuildStages
 };
 
@@ -1203,6 +1203,18 @@ k_batch_rebuild(const RebuildRep* __restrict__ reps, const int4* __restrict__ bl
     } else if constexpr (STAGE == kStPermute) {
         permute_body(d.cur, d.alt, d.perm, d.slot, d.n, 0, b);
     } else if constexpr (STAGE == kStCopy) {
+        if (d.m == 0) {  // no cells, no re-sort: the brute-force build, one warp per atom
+            brute_body(d.cur.pos, d.n, d.g.box, d.rl2, d.nbr, d.count, d.stride, d.status,
+                       d.max_count, b);
+            const int64_t i = (b * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+            if ((threadIdx.x & 31) == 0 && i < d.n) {  // the reference and fixed-point copies
+                const double4 p = d.cur.pos[i];
+                d.ref[i] = p;
+                if (d.q) d.q[i] = quantize_position(p, d.qs[0], d.qs[1], d.qs[2]);
+            }
+            if (b == 0 && threadIdx.x == 0) ++*d.total;
+            return;
+        }
         // the copy back also writes what the solo rebuild writes from the same
         // positions after the list build: the reference positions of the rebuild
         // test and the fixed-point copy
@@ -1214,15 +1226,6 @@ k_batch_rebuild(const RebuildRep* __restrict__ reps, const int4* __restrict__ bl
             if (d.q) d.q[k] = quantize_position(p, d.qs[0], d.qs[1], d.qs[2]);
         }
         if (k == 0) ++*d.total;
-    } else if constexpr (STAGE == kStBrute) {  // no re-sort: one warp per atom
-        brute_body(d.cur.pos, d.n, d.g.box, d.rl2, d.nbr, d.count, d.stride, d.status, d.max_count, b);
-        const int64_t i = (b * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
-        if ((threadIdx.x & 31) == 0 && i < d.n) {  // the reference and fixed-point copies
-            const double4 p = d.cur.pos[i];
-            d.ref[i] = p;
-            if (d.q) d.q[i] = quantize_position(p, d.qs[0], d.qs[1], d.qs[2]);
-        }
-        if (b == 0 && threadIdx.x == 0) ++*d.total;
     }
 }
 
@@ -1507,7 +1510,7 @@ void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj, bool bat
 }
 
 DispArgs disp_args(md_verlet* v, md_context* ctx, double* part) {
-    DispArgs d;
+    DispArgs d{};
     d.ref = v->ref.as<double4>();
     d.skin = v->skin;
     d.criterion = v->criterion;
@@ -1591,8 +1594,8 @@ int batch_rebuild_create(const BatchRepView* v, int nrep, BatchRebuild** out) {
             c * static_cast<int>(std::min<int64_t>(grid_for(2 * static_cast<int64_t>(m), kBlock), 4096)),
             c * nblk, c, c * nblk,
             cells ? grid_for(32 * static_cast<int64_t>(m), 256) : 1,  // + clearing the row maximum
-            c * nblk, c * nblk, c * grid_for(static_cast<int64_t>(m) * d.groups, kBuildWarps),
-            cells ? 0 : grid_for(n * 32, kBlock)};
+            c * nblk, cells ? nblk : grid_for(n * 32, kBlock),
+            c * grid_for(static_cast<int64_t>(m) * d.groups, kBuildWarps)};
         for (int st = 0; st < kRebuildStages; ++st) {
             int* o = off.data() + static_cast<size_t>(st) * (nrep + 1);
             o[r + 1] = o[r] + per[st];
@@ -1647,7 +1650,6 @@ int batch_rebuild_launch(BatchRebuild* b, cudaStream_t stream, int64_t* launches
                                 stream>>>(reps, table(kStCells));
         ++l;
     }
-    stage(kStBrute, k_batch_rebuild<kStBrute>);
     if (launches) *launches += l;
     MDB_CHECK_LAUNCH();
     return MD_OK;
