@@ -355,7 +355,7 @@ int md_batch_run(md_batch* b, int64_t steps, double* thermo) {
         for (size_t k = 0; k < nr && rc == MD_OK; ++k) {
             auto& r = b->reps[k];
             rc = capture_lj_step_into(r.it, r.sys, r.list, r.lj, run[k].rows.as<double>(),
-                                      run[k].idx.as<int>(), graph, &main_l[k], &body_l[k]);
+                                      run[k].idx.as<int>(), graph, &main_l[k], &body_l[k], nullptr);
         }
         if (rc == MD_OK && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess)
             rc = fail(MD_ERR_CUDA, "md_batch_run: graph instantiation failed");

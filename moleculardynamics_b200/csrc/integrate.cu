@@ -28,7 +28,7 @@ constexpr int kBlock = 256;
 // Where a fused run stands, on the device: a captured step cannot carry a step number.
 struct RunCursor {
     int done;  // steps recorded (the next thermo row)
-    int pad;
+    int left;  // captured steps to go, counted down by each one's displacement check
     uint64_t first;  // the integrator's step counter when the run began
 };
 
@@ -374,6 +374,13 @@ NhcState* nhc_of(md_integrator* it) {
     return (it->kind == 2 || it->kind == 4) ? it->chain_state.as<NhcState>() : nullptr;
 }
 
+// What the displacement check of a captured step sets: its rebuild branch and, when the step
+// is the body of a loop, whether the loop goes round again (left: steps to go, or null).
+struct StepHandles {
+    cudaGraphConditionalHandle branch, loop;
+    int* left;
+};
+
 // The pre-force half of a step.  With `check` the rebuild test of that Verlet
 // list is fused into the position update (fused stepping loops).
 // fresh_ke: the chain half of a Nose-Hoover step sums the kinetic energy of the
@@ -381,10 +388,10 @@ NhcState* nhc_of(md_integrator* it) {
 // previous step's rescalings (fused loops, after their first step).
 // q: also write the fixed-point positions for a mixed-precision force.  run: a captured
 // step takes its step number from there (a Langevin step's noise depends on it).
-// branch: the captured step's rebuild branch, which the test opens.
+// handles: the captured step's conditional nodes, which the test sets.
 int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke = true,
               int4* q = nullptr, const RunCursor* run = nullptr,
-              const cudaGraphConditionalHandle* branch = nullptr) {
+              const StepHandles* handles = nullptr) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
     if (n == 0) return MD_OK;
@@ -400,9 +407,11 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         double* part;
         MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(blocks), &part));
         d = disp_args(check, ctx, part);
-        if (branch) {
-            d.branch = *branch;
+        if (handles) {
+            d.branch = handles->branch;
             d.in_graph = 1;
+            d.loop = handles->loop;
+            d.left = handles->left;
         }
     }
     if (it->kind == 1) {
@@ -505,12 +514,15 @@ int verlet_build_q(md_verlet* v, md_system* sys, int4* q, bool* quantized);
 // ------------------------------------------------------------ step graphs
 namespace {
 
-// One fused LJ step captured as a CUDA graph: [chain half,] kick/drift with the
-// displacement check, a conditional node whose body is the gated neighbour
-// rebuild (opened by the displacement check's last block, so steps without a
-// rebuild launch none of its kernels; a kernel of its own to open it cost 3 us a step),
-// forces, the closing kick and the thermo row.  Replaying it runs the same kernels with the same arguments as the host
-// loop.
+// Fused LJ steps as a CUDA graph: a loop node, one launch for all steps of a run, whose body
+// is one captured step.  (A graph launch a step left the GPU idle between two of them: 864
+// atoms 30.8 us a step, 28.4 in the loop; graphs of ten steps 28.1, but their capture costs a
+// first run more than the loop's.)  A step is [chain half,] kick/drift with the displacement
+// check, a conditional node whose body is the gated neighbour rebuild (opened by the check's
+// last block, so steps without a rebuild launch none of its kernels; a kernel of its own to
+// open it cost 2 us a step), forces, the closing kick and the thermo row: the same kernels
+// with the same arguments as the host loop.  The loop ends: every step's check counts
+// RunCursor::left down and sets the loop's condition from it.
 struct StepGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -590,7 +602,7 @@ int lj_fused_step(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, do
 
 int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj,
                          double* rows, int* idx, cudaGraph_t graph, int64_t* main_launches,
-                         int64_t* body_launches) {
+                         int64_t* body_launches, const cudaGraphConditionalHandle* loop) {
     md_context* ctx = sys->ctx;
     NhcState* nhc = nhc_of(it);
     const int64_t l0 = ctx->launches;
@@ -598,11 +610,12 @@ int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj*
     cudaGraphConditionalHandle h;
     if (cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault) != cudaSuccess)
         return fail(MD_ERR_CUDA, "cudaGraphConditionalHandleCreate failed");
+    const StepHandles hs{h, loop ? *loop : 0, loop ? idx + 1 : nullptr};  // RunCursor::left
     std::vector<cudaGraphNode_t> leaves;
     int4* q = nullptr;
     MDB_TRY(step_quantize_target(it, sys, lj, &q));  // allocated by the first, eager step
     rc = capture_into(ctx, graph, nullptr, 0, [&]() -> int {
-        return pre_force(it, sys, v, false, q, reinterpret_cast<const RunCursor*>(idx), &h);
+        return pre_force(it, sys, v, false, q, reinterpret_cast<const RunCursor*>(idx), &hs);
     }, &leaves);
     const int64_t l1 = ctx->launches;
     cudaGraphNode_t cond = nullptr;
@@ -649,8 +662,18 @@ int capture_lj_step(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, 
                     int* idx, StepGraph& sg) {
     if (cudaGraphCreate(&sg.graph, 0) != cudaSuccess)
         return fail(MD_ERR_CUDA, "cudaGraphCreate failed");
-    int rc = capture_lj_step_into(it, sys, v, lj, rows, idx, sg.graph, &sg.main_launches,
-                                  &sg.body_launches);
+    cudaGraphNode_t node = nullptr;
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaError_t e = cudaGraphConditionalHandleCreate(&cp.conditional.handle, sg.graph, 1,
+                                                     cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) e = cudaGraphAddNode(&node, sg.graph, nullptr, 0, &cp);
+    int rc = e == cudaSuccess ? MD_OK : fail(MD_ERR_CUDA, "loop node: %s", cudaGetErrorString(e));
+    if (rc == MD_OK)
+        rc = capture_lj_step_into(it, sys, v, lj, rows, idx, cp.conditional.phGraph_out[0],
+                                  &sg.main_launches, &sg.body_launches, &cp.conditional.handle);
     if (rc == MD_OK && cudaGraphInstantiate(&sg.exec, sg.graph, 0) != cudaSuccess)
         rc = fail(MD_ERR_CUDA, "step graph instantiation failed");
     if (rc != MD_OK) sg.release();
@@ -1112,10 +1135,6 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
         MDB_TRY(it->run_idx.ensure(sizeof(RunCursor)));
         if (!it->h_rebuilt)
             MDB_CUDA(cudaMallocHost(&it->h_rebuilt, sizeof(RunCursor) + 2 * sizeof(int)));
-        RunCursor* cursor = reinterpret_cast<RunCursor*>(it->h_rebuilt + 2);
-        *cursor = RunCursor{0, 0, it->step};
-        MDB_CUDA(cudaMemcpyAsync(it->run_idx.ptr, cursor, sizeof(RunCursor), cudaMemcpyHostToDevice,
-                                 ctx->stream));
     }
     double* rows = it->run_rows.as<double>();
     int* idx = it->run_idx.as<int>();
@@ -1135,6 +1154,13 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
     bool cached = want_graph && sg && sg->exec && it->run_epoch == graph_epoch() &&
                   key[0] == it->run_key[0] && key[1] == it->run_key[1] && key[2] == it->run_key[2];
     int64_t k = 0;
+    if (steps > 0) {
+        RunCursor* cursor = reinterpret_cast<RunCursor*>(it->h_rebuilt + 2);
+        const int eager = !cached || nhc ? 1 : 0;  // the first step, from the host
+        *cursor = RunCursor{0, static_cast<int>(steps - eager), it->step};
+        MDB_CUDA(cudaMemcpyAsync(it->run_idx.ptr, cursor, sizeof(RunCursor), cudaMemcpyHostToDevice,
+                                 ctx->stream));
+    }
     if (steps > 0 && (!cached || nhc)) {
         MDB_TRY(lj_fused_step(it, sys, v, lj, rows, idx, true));
         k = 1;
@@ -1161,7 +1187,7 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
         const int64_t graph_steps = steps - k;
         MDB_CUDA(cudaMemcpyAsync(it->h_rebuilt, v->d_rebuild_total, sizeof(int),
                                  cudaMemcpyDeviceToHost, ctx->stream));
-        for (int64_t g = 0; g < graph_steps; ++g) MDB_CUDA(cudaGraphLaunch(sg->exec, ctx->stream));
+        MDB_CUDA(cudaGraphLaunch(sg->exec, ctx->stream));  // all of them: RunCursor::left
         MDB_CUDA(cudaMemcpyAsync(it->h_rebuilt + 1, v->d_rebuild_total, sizeof(int),
                                  cudaMemcpyDeviceToHost, ctx->stream));
         if (it->kind == 1) it->step += static_cast<uint64_t>(graph_steps);

@@ -291,6 +291,9 @@ struct DispArgs {
     // a captured step's rebuild branch (when in_graph), opened by the thread that decides
     cudaGraphConditionalHandle branch;
     int in_graph;
+    // the loop of steps the captured step is the body of, and the steps left, when it is
+    cudaGraphConditionalHandle loop;
+    int* left;
 };
 
 __device__ inline void top2_grid_at(double a1, double a2, const DispArgs& d, unsigned block,
@@ -345,6 +348,11 @@ __device__ inline void top2_grid_at(double a1, double a2, const DispArgs& d, uns
         *d.flag = rebuild;
         *d.ticket = 0u;
         if (d.in_graph) cudaGraphSetConditional(d.branch, static_cast<unsigned>(rebuild));
+        if (d.left) {  // one less each time round: the loop ends
+            const int left = *d.left - 1;
+            *d.left = left;
+            cudaGraphSetConditional(d.loop, left > 0 ? 1u : 0u);
+        }
     }
 }
 

@@ -371,9 +371,10 @@ int nhc_apply_scale_async(md_integrator* it, md_system* sys);
 // displacement check against `check`'s reference positions; post_force).
 int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check);
 int vv_post_async(md_integrator* it, md_system* sys);
+// One fused step captured into `graph`; loop: the loop node whose body that is, or null.
 int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj,
                          double* rows, int* idx, cudaGraph_t graph, int64_t* main_launches,
-                         int64_t* body_launches);
+                         int64_t* body_launches, const cudaGraphConditionalHandle* loop);
 
 // Pair-force kernels over the Verlet list; results land in the context result
 // slots kResEnergy / kResVirial (device), no synchronisation.
