@@ -84,7 +84,8 @@ __device__ __forceinline__ void kick_drift_scaled(md_atoms a, int64_t n, const S
             vy = fma(c, a.fy[k], vy);
             vz = fma(c, a.fz[k], vz);
             const Fold3 f3 = fold3_of(s.box);
-            double4 p = a.pos[k];
+            double4 p = a.pos[k], ref;
+            if (CHECK && ATOMS == 1) ref = ldg4(d.ref + k);  // a load the stores would hold back
             p.x = fold_wrapped(fma(s.dt, vx, p.x), f3.b[0]);
             p.y = fold_wrapped(fma(s.dt, vy, p.y), f3.b[1]);
             p.z = fold_wrapped(fma(s.dt, vz, p.z), f3.b[2]);
@@ -95,7 +96,8 @@ __device__ __forceinline__ void kick_drift_scaled(md_atoms a, int64_t n, const S
             a.vz[k] = vz;
             if (s.q) s.q[k] = quantize_position(p, s.qs[0], s.qs[1], s.qs[2]);
             if (CHECK) {
-                const double x = disp2(f3, p, d.ref[k]);
+                if (ATOMS != 1) ref = d.ref[k];
+                const double x = disp2(f3, p, ref);
                 if (u == 0) a1 = x;
                 else top2_insert(a1, a2, x);
             }
@@ -123,6 +125,21 @@ k_kick_drift(md_atoms a, int64_t n, StepArgs s, const NhcState* nhc, DispArgs d)
     kick_drift_body<CHECK, kKickAtoms>(a, n, s, nhc, d, blockIdx.x, gridDim.x);
 }
 
+// A system that does not fill the GPU waits on one block's chain of loads, barrier and
+// atomics: small blocks, an atom a thread.  A whole fused FP64 step, 256-thread blocks of
+// 512 atoms and these: 864 atoms 22.0 and 19.0 us (64 threads 19.4), 6,912 27.9 and 25.5,
+// 16,384 32.4 and 29.8 (32 threads 30.8), 32,000 41.6 and 40.2 (42.6), 119,000 93.8 and 95.5.
+int few_threads(const md_context* ctx, int64_t n) {
+    const int64_t sms = ctx->sm_count;
+    return n <= 32 * sms ? 32 : (n <= 256 * sms ? 64 : 0);
+}
+
+template <bool CHECK>
+__global__ void __launch_bounds__(64)
+k_kick_drift_few(md_atoms a, int64_t n, StepArgs s, const NhcState* nhc, DispArgs d) {
+    kick_drift_body<CHECK, 1>(a, n, s, nhc, d, blockIdx.x, gridDim.x);
+}
+
 // langevin.hpp:55-80: B, A (wrap), O, A (wrap).
 template <bool CHECK>
 __global__ void k_baoab_pre(md_atoms a, int64_t n, StepArgs s, DispArgs d) {
@@ -134,7 +151,8 @@ __global__ void k_baoab_pre(md_atoms a, int64_t n, StepArgs s, DispArgs d) {
         double vx = fma(c, a.fx[k], a.vx[k]);
         double vy = fma(c, a.fy[k], a.vy[k]);
         double vz = fma(c, a.fz[k], a.vz[k]);
-        double4 p = a.pos[k];
+        double4 p = a.pos[k], ref;
+        if (CHECK) ref = ldg4(d.ref + k);
         p.x = fold_wrapped(fma(s.half_dt, vx, p.x), f3.b[0]);
         p.y = fold_wrapped(fma(s.half_dt, vy, p.y), f3.b[1]);
         p.z = fold_wrapped(fma(s.half_dt, vz, p.z), f3.b[2]);
@@ -171,7 +189,7 @@ __global__ void k_baoab_pre(md_atoms a, int64_t n, StepArgs s, DispArgs d) {
         a.vy[k] = vy;
         a.vz[k] = vz;
         if (s.q) s.q[k] = quantize_position(p, s.qs[0], s.qs[1], s.qs[2]);
-        if (CHECK) a1 = disp2(f3, p, d.ref[k]);
+        if (CHECK) a1 = disp2(f3, p, ref);
     }
     if (CHECK) top2_grid(a1, 0.0, d);
 }
@@ -402,7 +420,8 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         for (int d = 0; d < 3; ++d) s.qs[d] = 4294967296.0 / sys->box[d];
     }
     DispArgs d{};
-    const int blocks = grid_for(n, kBlock);
+    const int few = few_threads(ctx, n);
+    const int threads = few ? few : kBlock, blocks = grid_for(n, threads);
     if (check) {
         double* part;
         MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(blocks), &part));
@@ -421,8 +440,8 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
             s.noise = it->noise.as<double>() + it->noise_used;
             it->noise_used += 3 * n;
         }
-        if (check) k_baoab_pre<true><<<blocks, kBlock, 0, ctx->stream>>>(sys->cur, n, s, d);
-        else k_baoab_pre<false><<<blocks, kBlock, 0, ctx->stream>>>(sys->cur, n, s, d);
+        if (check) k_baoab_pre<true><<<blocks, threads, 0, ctx->stream>>>(sys->cur, n, s, d);
+        else k_baoab_pre<false><<<blocks, threads, 0, ctx->stream>>>(sys->cur, n, s, d);
         if (!run) ++it->step;  // a replay's steps are counted by the run
     } else {
         NhcState* nhc = nhc_of(it);
@@ -435,8 +454,14 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         }
         ctx_time_begin(ctx, MD_KERNEL_INTEGRATE);
         const int kd = grid_for(n, kKickAtoms * kBlock);
-        if (check) k_kick_drift<true><<<kd, kBlock, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
-        else k_kick_drift<false><<<kd, kBlock, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
+        if (few && check)
+            k_kick_drift_few<true><<<blocks, few, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
+        else if (few)
+            k_kick_drift_few<false><<<blocks, few, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
+        else if (check)
+            k_kick_drift<true><<<kd, kBlock, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
+        else
+            k_kick_drift<false><<<kd, kBlock, 0, ctx->stream>>>(sys->cur, n, s, nhc, d);
         ctx_time_end(ctx, MD_KERNEL_INTEGRATE);
     }
     sys->wrapped = true;
