@@ -104,14 +104,12 @@ __global__ void k_vec_from_orig(const int* __restrict__ slot, int64_t n, const d
     if (o < n) out[slot[o]] = in[o];
 }
 
-__global__ void k_or_flag(const int* flag, int* acc) {
-    if (*flag) *acc = 1;
-}
-
-__global__ void k_record3(const double* ev, const double* ke, double* rows, int64_t k) {
-    rows[3 * k + 0] = ev[0];
-    rows[3 * k + 1] = ev[1];
-    rows[3 * k + 2] = *ke;
+__global__ void k_record(const double* ev, const double* ke, double* rows, int* idx) {
+    double* row = rows + 4 * static_cast<int64_t>(*idx);
+    row[0] = ev[0];
+    row[1] = ev[1];
+    row[2] = *ke;
+    ++*idx;
 }
 
 // ---------------------------------------------------------------- reverse step
@@ -281,12 +279,23 @@ int segment_start(md_adjoint* a) {
     return MD_OK;
 }
 
-int segment_step(md_adjoint* a) {
-    MDB_TRY(vv_pre_async(a->vv, a->sys, a->list));
-    k_or_flag<<<1, 1, 0, a->ctx->stream>>>(a->list->d_rebuild_flag, a->flag.as<int>());
-    ++a->ctx->launches;
-    MDB_TRY(lj_forces_verlet_async(&a->lj, a->sys, a->list));
+// One step: two launches where the force kernel can apply the closing half-kick and record
+// the row (energy, virial, kinetic energy; rows, idx: device, or null).  32,000 atoms, five
+// launches and two of them: 6 us of 60 us a step.
+int segment_step(md_adjoint* a, double* rows, int* idx) {
+    md_context* ctx = a->ctx;
+    MDB_TRY(vv_pre_async(a->vv, a->sys, a->list, a->flag.as<int>()));
+    KickArgs kick = integrator_kick_args(a->vv, a->sys);
+    kick.rows = rows;
+    kick.idx = idx;
+    bool kicked = false;
+    MDB_TRY(lj_forces_verlet_async(&a->lj, a->sys, a->list, nullptr, false, &kick, &kicked));
+    if (kicked) return MD_OK;
     MDB_TRY(vv_post_async(a->vv, a->sys));
+    if (rows) {
+        k_record<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEnergy), ctx_result(ctx, kResKE), rows, idx);
+        ++ctx->launches;
+    }
     return MD_OK;
 }
 
@@ -356,10 +365,10 @@ int md_adjoint_forward(md_adjoint* a, md_system* sys, const md_lj* lj, double dt
     const int64_t nseg = segments(a);
     const size_t state = 2 * sizeof(double4) * static_cast<size_t>(n);
     MDB_TRY(a->ck.ensure(state * static_cast<size_t>(nseg + 1)));  // + the final state
-    MDB_TRY(a->flag.ensure(sizeof(int)));
+    MDB_TRY(a->flag.ensure(2 * sizeof(int)));  // the sticky rebuild flag, the next row
     DevBuf drows;
-    MDB_TRY(drows.ensure(3 * sizeof(double) * static_cast<size_t>(steps)));
-    MDB_CUDA(cudaMemsetAsync(a->flag.ptr, 0, sizeof(int), ctx->stream));
+    MDB_TRY(drows.ensure(4 * sizeof(double) * static_cast<size_t>(steps)));
+    MDB_CUDA(cudaMemsetAsync(a->flag.ptr, 0, 2 * sizeof(int), ctx->stream));
     const int g = grid_for(n, kBlock);
     for (int64_t sg = 0; sg < nseg; ++sg) {
         double4* ckp = a->ck.as<double4>() + 2 * n * sg;
@@ -367,12 +376,8 @@ int md_adjoint_forward(md_adjoint* a, md_system* sys, const md_lj* lj, double dt
         ++ctx->launches;
         MDB_TRY(segment_start(a));
         const int64_t k0 = sg * every, k1 = std::min(steps, k0 + every);
-        for (int64_t k = k0; k < k1; ++k) {
-            MDB_TRY(segment_step(a));
-            k_record3<<<1, 1, 0, ctx->stream>>>(ctx_result(ctx, kResEnergy), ctx_result(ctx, kResKE),
-                                                drows.as<double>(), k);
-            ++ctx->launches;
-        }
+        for (int64_t k = k0; k < k1; ++k)
+            MDB_TRY(segment_step(a, drows.as<double>(), a->flag.as<int>() + 1));
         MDB_CHECK_LAUNCH();
     }
     {
@@ -382,9 +387,10 @@ int md_adjoint_forward(md_adjoint* a, md_system* sys, const md_lj* lj, double dt
     }
     int bad = 0;
     MDB_CUDA(cudaMemcpyAsync(&bad, a->flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    if (rows)
-        MDB_CUDA(cudaMemcpyAsync(rows, drows.ptr, 3 * sizeof(double) * static_cast<size_t>(steps),
-                                 cudaMemcpyDeviceToHost, ctx->stream));
+    if (rows)  // the first three of each row's four
+        MDB_CUDA(cudaMemcpy2DAsync(rows, 3 * sizeof(double), drows.ptr, 4 * sizeof(double),
+                                   3 * sizeof(double), static_cast<size_t>(steps),
+                                   cudaMemcpyDeviceToHost, ctx->stream));
     MDB_CUDA(cudaStreamSynchronize(ctx->stream));
     drows.release();
     MDB_TRY(ctx_check_status(ctx));
@@ -435,12 +441,12 @@ int md_adjoint_backward(md_adjoint* a, const double* grad_rows, double grad_thet
         // recompute the segment from its checkpoint, keeping every state
         const double4* ckp = a->ck.as<double4>() + 2 * n * sg;
         sys->wrapped = false;
-    k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
+        k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
         MDB_TRY(segment_start(a));
         double4* snap = a->snap.as<double4>();
         k_snapshot<<<g, kBlock, 0, ctx->stream>>>(sys->cur, n, snap, snap + n);
         for (int64_t j = 1; j <= len; ++j) {
-            MDB_TRY(segment_step(a));
+            MDB_TRY(segment_step(a, nullptr, nullptr));
             k_snapshot<<<g, kBlock, 0, ctx->stream>>>(sys->cur, n, snap + 2 * n * j,
                                                      snap + 2 * n * j + n);
         }
@@ -475,7 +481,7 @@ int md_adjoint_backward(md_adjoint* a, const double* grad_rows, double grad_thet
         // leave the system where the forward left it (forces too)
         const double4* ckp = a->ck.as<double4>() + 2 * n * nseg;
         sys->wrapped = false;
-    k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
+        k_state_from_orig<<<g, kBlock, 0, ctx->stream>>>(sys->cur, sys->slot, n, ckp, ckp + n);
         ++ctx->launches;
         MDB_TRY(verlet_build(a->list, sys, false));
         MDB_TRY(lj_forces_verlet_async(&a->lj, sys, a->list));

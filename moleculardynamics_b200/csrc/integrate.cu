@@ -406,10 +406,10 @@ struct StepHandles {
 // previous step's rescalings (fused loops, after their first step).
 // q: also write the fixed-point positions for a mixed-precision force.  run: a captured
 // step takes its step number from there (a Langevin step's noise depends on it).
-// handles: the captured step's conditional nodes, which the test sets.
+// handles: the captured step's conditional nodes, which the test sets; sticky: see DispArgs.
 int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke = true,
               int4* q = nullptr, const RunCursor* run = nullptr,
-              const StepHandles* handles = nullptr) {
+              const StepHandles* handles = nullptr, int* sticky = nullptr) {
     md_context* ctx = sys->ctx;
     const int64_t n = sys->n;
     if (n == 0) return MD_OK;
@@ -426,6 +426,7 @@ int pre_force(md_integrator* it, md_system* sys, md_verlet* check, bool fresh_ke
         double* part;
         MDB_TRY(ctx_partials(ctx, 2 * static_cast<size_t>(blocks), &part));
         d = disp_args(check, ctx, part);
+        d.sticky = sticky;
         if (handles) {
             d.branch = handles->branch;
             d.in_graph = 1;
@@ -588,8 +589,8 @@ int capture_into(md_context* ctx, cudaGraph_t g, const cudaGraphNode_t* deps, si
 
 }  // namespace (the step graph helpers above are private to this file)
 
-int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check) {
-    return pre_force(it, sys, check, true);
+int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check, int* sticky) {
+    return pre_force(it, sys, check, true, nullptr, nullptr, nullptr, sticky);
 }
 
 int vv_post_async(md_integrator* it, md_system* sys) { return post_force_async(it, sys, true); }

@@ -291,6 +291,7 @@ struct DispArgs {
     // a captured step's rebuild branch (when in_graph), opened by the thread that decides
     cudaGraphConditionalHandle branch;
     int in_graph;
+    int* sticky;  // set when a rebuild is due and left alone otherwise, or null
     // the loop of steps the captured step is the body of, and the steps left, when it is
     cudaGraphConditionalHandle loop;
     int* left;
@@ -347,6 +348,7 @@ __device__ inline void top2_grid_at(double a1, double a2, const DispArgs& d, uns
         const int rebuild = (d.criterion == 0 ? (r1 + r2) > d.skin : r1 > 0.5 * d.skin) ? 1 : 0;
         *d.flag = rebuild;
         *d.ticket = 0u;
+        if (rebuild && d.sticky) *d.sticky = 1;
         if (d.in_graph) cudaGraphSetConditional(d.branch, static_cast<unsigned>(rebuild));
         if (d.left) {  // one less each time round: the loop ends
             const int left = *d.left - 1;

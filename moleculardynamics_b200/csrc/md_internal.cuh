@@ -368,8 +368,9 @@ int lj_fused_step(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, do
                   int* idx, bool first);
 int nhc_apply_scale_async(md_integrator* it, md_system* sys);
 // The two halves of one host-driven step (pre_force with an optional fused
-// displacement check against `check`'s reference positions; post_force).
-int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check);
+// displacement check against `check`'s reference positions, which also sets *sticky (device)
+// when a rebuild is due; post_force).
+int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check, int* sticky);
 int vv_post_async(md_integrator* it, md_system* sys);
 // One fused step captured into `graph`; loop: the loop node whose body that is, or null.
 int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj,
