@@ -350,26 +350,30 @@ FieldList field_list(const int* fields, int count) {
     return l;
 }
 
-// Host columns to or from the staging columns at `st`, in as few copies as the host
-// layout allows: one for columns end to end, one strided copy for columns at a constant
-// distance (rows of a larger array), else one each.
+// Host columns to or from the staging columns at `st`: one copy for a run of columns end to
+// end, else one each.  Columns that touch may still be page-locked apart, which one copy
+// cannot span: the runtime refuses it, before it copies anything, and each column goes alone.
 template <class P>
 int copy_columns(md_context* ctx, double* st, P const* host, int count, int64_t n, cudaMemcpyKind kind) {
     const bool in = kind == cudaMemcpyHostToDevice;
-    const auto at = [&](int k) { return reinterpret_cast<uintptr_t>(host[k]); };
     const size_t width = sizeof(double) * static_cast<size_t>(n);
-    for (int k = 0, run; k < count; k += run) {
-        run = 1;
-        const uintptr_t pitch = k + 1 < count && at(k + 1) > at(k) ? at(k + 1) - at(k) : 0;
-        if (pitch >= width && pitch < (uintptr_t(1) << 31))
-            while (k + run < count && at(k + run) - at(k + run - 1) == pitch) ++run;
+    const auto copy = [&](int k, int run) {
         double* dev = st + static_cast<int64_t>(k) * n;
         double* h = const_cast<double*>(host[k]);
-        if (run > 1 && pitch != width)
-            MDB_CUDA(in ? cudaMemcpy2DAsync(dev, width, h, pitch, width, run, kind, ctx->stream)
-                        : cudaMemcpy2DAsync(h, pitch, dev, width, width, run, kind, ctx->stream));
-        else
-            MDB_CUDA(cudaMemcpyAsync(in ? dev : h, in ? h : dev, width * run, kind, ctx->stream));
+        return cudaMemcpyAsync(in ? dev : h, in ? h : dev, width * run, kind, ctx->stream);
+    };
+    for (int k = 0, run; k < count; k += run) {
+        run = 1;
+        while (k + run < count && reinterpret_cast<uintptr_t>(host[k + run]) ==
+                                      reinterpret_cast<uintptr_t>(host[k]) + width * run)
+            ++run;
+        cudaError_t e = copy(k, run);
+        if (e == cudaErrorInvalidValue && run > 1) {
+            cudaGetLastError();
+            e = cudaSuccess;
+            for (int j = k; j < k + run && e == cudaSuccess; ++j) e = copy(j, 1);
+        }
+        MDB_CUDA(e);
     }
     return MD_OK;
 }
