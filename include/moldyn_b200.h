@@ -122,8 +122,8 @@ MD_API int md_context_graph_captures(md_context* ctx, int64_t* count);
 #define MD_KERNEL_EWALD_REAL 3   /* Ewald real-space pairs */
 #define MD_KERNEL_EWALD_RECIP 4  /* Ewald structure factors and k-space forces */
 MD_API int md_context_set_timing(md_context* ctx, int enable);
-/* Fused device loops (md_run_lj) replay one captured CUDA graph per step, the
- * device-decided neighbour rebuild being a conditional node, when enabled
+/* Fused device loops (md_run_lj) run one captured step in a loop on the device, one
+ * graph launch a call, the device-decided neighbour rebuild being a branch of it, when enabled
  * (default) and timing is off; 0 launches every kernel from the host instead.
  * Results are identical either way.  No reference counterpart. */
 MD_API int md_context_set_graphs(md_context* ctx, int enable);
@@ -236,16 +236,16 @@ MD_API int md_lj_lrc(const md_lj* lj, int64_t n, const double box[3], double* u_
 /* Launch shape of the Verlet-list force kernel (process-wide tuning knobs; no
  * reference counterpart -- the reference is scalar): threads per atom 1, 2, 4 or 8
  * (default 2) and independent neighbour gathers in flight per thread 1, 2 or 4
- * (default 2). */
+ * (default 2).  At the defaults an FP64 system of up to 64 atoms per SM takes sixteen
+ * lanes per atom and one of up to 256 four, adding in the order of two. */
 MD_API int md_lj_set_threads_per_atom(int tpa);
 MD_API int md_lj_set_unroll(int unroll);
 /* Launch shape of this LJ object's Verlet force kernel (threads per atom 1/2/4/8,
  * gathers in flight 1/2/4; 0 = the library default).  Set by the autotuner
  * (moleculardynamics_b200/autotune.py); no reference counterpart. */
 MD_API int md_lj_set_launch(md_lj* lj, int tpa, int unroll);
-/* Mixed precision only: read neighbours through the list's halo tiles when it
- * keeps them (on = 1, the default) or always gather them through the int32 rows
- * (0).  A halo tile holds a block of 128 cell-sorted atoms and every atom of the
+/* Read neighbours through the list's halo tiles when it keeps them (on = 1, the
+ * default) or always gather them through the int32 rows (0).  A halo tile holds a block of 128 cell-sorted atoms and every atom of the
  * cells around them in shared memory; rows then also exist as 16-bit tile slots.
  * Forces are identical either way.  No reference counterpart. */
 MD_API int md_lj_set_halo(md_lj* lj, int on);
@@ -258,8 +258,8 @@ MD_API int md_lj_set_halo(md_lj* lj, int on);
 MD_API int md_lj_set_tile_threads(md_lj* lj, int tpa);
 /* Halo tiles of a Verlet list: built now from the current list and again at
  * every rebuild (on = 1), or dropped (0).  md_run_lj and md_batch_run turn them on
- * by themselves for mixed-precision runs of >= 16 steps on >= 65,536 atoms, where
- * the faster force kernel pays for building them.  Lists without a cell grid
+ * by themselves for mixed-precision systems of >= 65,536 atoms, and md_run_lj for
+ * FP64 ones of >= 196,608, where the faster force kernel pays for building them.  Lists without a cell grid
  * (fewer than 3 cells per side) keep none.  No reference counterpart. */
 MD_API int md_verlet_set_halo(md_verlet* v, int on);
 /* How many of a list's halo tiles are staged in shared memory (the rest gather

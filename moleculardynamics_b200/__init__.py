@@ -550,7 +550,7 @@ class VerletList:
         _check(lib().md_verlet_set_capacity(self._h, int(capacity), 1 if fixed else 0))
 
     def set_halo(self, on=True):
-        """Keep halo tiles for the mixed-precision force kernel (built now and at
+        """Keep halo tiles for the force kernel (built now and at
         every rebuild), or drop them.  Fused runs of large systems turn them on."""
         _check(lib().md_verlet_set_halo(self._h, 1 if on else 0))
 
@@ -618,7 +618,7 @@ class LennardJones:
         _check(lib().md_lj_set_tile_threads(self._h, int(tpa)))
 
     def set_halo(self, on=True):
-        """Mixed precision: read neighbours through shared-memory halo tiles (the
+        """Read neighbours through the list's shared-memory halo tiles (the
         default) or gather them through the int32 rows; forces are identical."""
         _check(lib().md_lj_set_halo(self._h, 1 if on else 0))
 

@@ -8,6 +8,7 @@
 // rescalings per step; the rescalings are folded into one factor applied by the
 // next kick.
 #include <cmath>
+#include <limits>
 #include <new>
 #include <vector>
 
@@ -1174,7 +1175,7 @@ int md_run_lj(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj, int64_
     // always runs from the host: it sums the entry kinetic energy instead of using
     // the tracked value, which the caller may have changed between calls.
     const bool want_graph = ctx->graphs && !ctx->timing && !(it->kind == 1 && it->noise.ptr) &&
-                            steps >= 1 && sys->n > 0;
+                            steps >= 1 && steps <= std::numeric_limits<int>::max() && sys->n > 0;
     StepGraph* sg = static_cast<StepGraph*>(it->run_graph);
     const void* key[3] = {sys, v, lj};
     bool cached = want_graph && sg && sg->exec && it->run_epoch == graph_epoch() &&
