@@ -350,28 +350,43 @@ FieldList field_list(const int* fields, int count) {
     return l;
 }
 
+bool page_locked(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return false;
+}
+
 // Host columns to or from the staging columns at `st`: one copy for a run of columns end to
-// end, else one each.  Columns that touch may still be page-locked apart, which one copy
-// cannot span: the runtime refuses it, before it copies anything, and each column goes alone.
+// end, one strided copy for page-locked columns at a constant distance (rows of a larger
+// array; what lies between them is not touched), else one each.  Columns may be page-locked
+// apart, which one copy cannot span: the runtime refuses it, before it copies anything, and
+// each column goes alone.
 template <class P>
 int copy_columns(md_context* ctx, double* st, P const* host, int count, int64_t n, cudaMemcpyKind kind) {
     const bool in = kind == cudaMemcpyHostToDevice;
+    const auto at = [&](int k) { return reinterpret_cast<uintptr_t>(host[k]); };
     const size_t width = sizeof(double) * static_cast<size_t>(n);
-    const auto copy = [&](int k, int run) {
+    const auto copy = [&](int k, int run, size_t pitch) {
         double* dev = st + static_cast<int64_t>(k) * n;
         double* h = const_cast<double*>(host[k]);
+        if (pitch != width)
+            return in ? cudaMemcpy2DAsync(dev, width, h, pitch, width, run, kind, ctx->stream)
+                      : cudaMemcpy2DAsync(h, pitch, dev, width, width, run, kind, ctx->stream);
         return cudaMemcpyAsync(in ? dev : h, in ? h : dev, width * run, kind, ctx->stream);
     };
     for (int k = 0, run; k < count; k += run) {
         run = 1;
-        while (k + run < count && reinterpret_cast<uintptr_t>(host[k + run]) ==
-                                      reinterpret_cast<uintptr_t>(host[k]) + width * run)
+        size_t pitch = k + 1 < count && at(k + 1) > at(k) ? at(k + 1) - at(k) : 0;
+        if (pitch > width && (pitch >= (size_t(1) << 31) || !page_locked(host[k]))) pitch = 0;
+        while (pitch >= width && k + run < count && at(k + run) - at(k + run - 1) == pitch &&
+               (pitch == width || page_locked(host[k + run])))
             ++run;
-        cudaError_t e = copy(k, run);
+        cudaError_t e = copy(k, run, run > 1 ? pitch : width);
         if (e == cudaErrorInvalidValue && run > 1) {
             cudaGetLastError();
             e = cudaSuccess;
-            for (int j = k; j < k + run && e == cudaSuccess; ++j) e = copy(j, 1);
+            for (int j = k; j < k + run && e == cudaSuccess; ++j) e = copy(j, 1, width);
         }
         MDB_CUDA(e);
     }
