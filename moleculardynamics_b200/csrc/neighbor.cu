@@ -821,9 +821,64 @@ __device__ __forceinline__ int2 cell_ranks_of(const int* __restrict__ start, int
     return make_int2(__shfl_sync(0xffffffffu, lo, 0), __shfl_sync(0xffffffffu, lo, 16));
 }
 
+// Bitonic sort, ascending, of 32 E values held E to a lane; sorted, lane l has places
+// l E .. l E + E - 1.  Strides below E stay in the lane's registers, the rest are shuffles.
+template <int E>
+__device__ __forceinline__ void sort_warp(int (&v)[E], int lane) {
+#pragma unroll
+    for (int k = 2; k <= 32 * E; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const bool up = k < E || (lane & (k / E)) == 0;  // k < E: by register, below
+            if (j >= E) {
+                const bool low = ((lane & (j / E)) == 0) == up;
+#pragma unroll
+                for (int r = 0; r < E; ++r) {
+                    const int y = __shfl_xor_sync(0xffffffffu, v[r], j / E);
+                    v[r] = low ? min(v[r], y) : max(v[r], y);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < E; ++r) {
+                    if (r & j) continue;
+                    const bool asc = k < E ? (r & k) == 0 : up;
+                    const int lo = min(v[r], v[r | j]), hi = max(v[r], v[r | j]);
+                    v[r] = asc ? lo : hi;
+                    v[r | j] = asc ? hi : lo;
+                }
+            }
+        }
+}
+
+// The ranks of the cells around cells r0, r0 + 1, ... (27 each, ne in all, at most 32 E),
+// sorted into ent.
+template <int E>
+__device__ __forceinline__ void sorted_neighbours(const GridArgs& g, int r0, int ne, int lane, int* ent) {
+    int v[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {  // unrolled: the loads go out together
+        const int e = lane + 32 * k;
+        v[k] = 0x7fffffff;
+        if (e < ne) {
+            const int cell = g.cell_of_rank[r0 + e / 27], q = e % 27;
+            const int cx = cell % g.nx, cy = (cell / g.nx) % g.ny, cz = cell / (g.nx * g.ny);
+            int jx = cx + (q % 3) - 1, jy = cy + ((q / 3) % 3) - 1, jz = cz + (q / 9) - 1;
+            jx = jx < 0 ? jx + g.nx : (jx >= g.nx ? jx - g.nx : jx);
+            jy = jy < 0 ? jy + g.ny : (jy >= g.ny ? jy - g.ny : jy);
+            jz = jz < 0 ? jz + g.nz : (jz >= g.nz ? jz - g.nz : jz);
+            v[k] = g.rank_of_cell[jx + g.nx * (jy + g.ny * jz)];
+        }
+    }
+    sort_warp<E>(v, lane);
+#pragma unroll
+    for (int k = 0; k < E; ++k) ent[E * lane + k] = v[k];
+    __syncwarp();
+}
+
 // Plan of the halo tiles, one warp per tile (kHaloAtoms consecutive sorted
 // atoms): the cell ranks the tile's atoms span, their 27-cell neighbourhoods
-// sorted (bitonic, in shared memory) and merged into runs of consecutive ranks --
+// sorted (in registers; in shared memory the plan of 1,048,576 atoms took 79 us,
+// 31 so) and merged into runs of consecutive ranks --
 // each run one contiguous range of sorted atoms -- and each run's first slot in
 // the staged tile.  A tile spanning more than kHaloSpan cells, needing more than
 // kHaloRuns runs or kHaloCap slots, or lying inside one crowded cell, is not
@@ -851,39 +906,8 @@ k_halo_plan(const int* __restrict__ start, GridArgs g, int64_t n, int64_t tiles,
     }
     int* ent = s_ent[warp];
     const int ne = (r1 - r0 + 1) * 27;
-    const int np2 = ne <= 256 ? 256 : kPlanEntries;  // sort only the filled power of two
-#pragma unroll
-    for (int k = 0; k < kPlanEntries / 32; ++k) {  // unrolled: the loads go out together
-        const int e = lane + 32 * k;
-        if (e >= np2) break;
-        int v = 0x7fffffff;
-        if (e < ne) {
-            const int cell = g.cell_of_rank[r0 + e / 27], q = e % 27;
-            const int cx = cell % g.nx, cy = (cell / g.nx) % g.ny, cz = cell / (g.nx * g.ny);
-            int jx = cx + (q % 3) - 1, jy = cy + ((q / 3) % 3) - 1, jz = cz + (q / 9) - 1;
-            jx = jx < 0 ? jx + g.nx : (jx >= g.nx ? jx - g.nx : jx);
-            jy = jy < 0 ? jy + g.ny : (jy >= g.ny ? jy - g.ny : jy);
-            jz = jz < 0 ? jz + g.nz : (jz >= g.nz ? jz - g.nz : jz);
-            v = g.rank_of_cell[jx + g.nx * (jy + g.ny * jz)];
-        }
-        ent[e] = v;
-    }
-    __syncwarp();
-    for (int k = 2; k <= np2; k <<= 1) {  // bitonic sort, ascending
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int e = lane; e < np2; e += 32) {
-                const int p = e ^ j;
-                if (p > e) {
-                    const int x = ent[e], y = ent[p];
-                    if ((x > y) == ((e & k) == 0)) {
-                        ent[e] = y;
-                        ent[p] = x;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-    }
+    if (ne <= 256) sorted_neighbours<8>(g, r0, ne, lane, ent);
+    else sorted_neighbours<kPlanEntries / 32>(g, r0, ne, lane, ent);
     // runs of consecutive distinct ranks (duplicates neither open nor close one)
     int nopen = 0, nclose = 0;
     for (int c = 0; c < ne; c += 32) {
