@@ -93,7 +93,8 @@ __device__ __forceinline__ RealTerms<T> real_terms(T r2, T r, T cqq, bool coulom
     return t;
 }
 
-// Separations whose quotients could leave the normal range divide in IEEE arithmetic.
+// Separations whose quotients could leave the normal range, and in FP64 the squares that
+// reciprocal() does not serve with sigma^2 a power of two, divide in IEEE arithmetic.
 template <class T>
 __device__ __noinline__ RealTerms<T> real_terms_ieee(T r2, T cqq, bool coulomb, bool lj,
                                                      const RealArgs* a) {
@@ -105,7 +106,9 @@ __device__ __noinline__ RealTerms<T> real_terms_ieee(T r2, T cqq, bool coulomb, 
 template <class T>
 __device__ __forceinline__ RealTerms<T> real_pair(T r2, T cqq, bool coulomb, bool lj,
                                                   const RealArgs& a) {
-    if (!(r2 > T(1e-15))) return real_terms_ieee<T>(r2, cqq, coulomb, lj, &a);
+    bool fast = r2 > T(1e-15);
+    if constexpr (sizeof(T) == 8) fast = fast && !low_ones(r2);
+    if (!fast) return real_terms_ieee<T>(r2, cqq, coulomb, lj, &a);
     T r;
     if constexpr (sizeof(T) == 4) r = __fsqrt_rn(r2);
     else r = __dsqrt_rn(r2);

@@ -89,12 +89,12 @@ __device__ __noinline__ PairTerms pair_terms_ieee(double sig2, double four_eps, 
     return pair_terms<LFS>(a, r2, [r2](double x) { return __ddiv_rn(x, r2); });
 }
 
-// Both divisions of a pair share one reciprocal (bit-identical quotients).  Returns false
-// outside rc.
+// Both divisions of a pair share one reciprocal; sigma^2, a dividend, may be a power of two.
+// Returns false outside rc.
 template <bool LFS>
 __device__ __forceinline__ bool pair_exact(const LJArgs& a, double r2, PairTerms& t) {
     if (!(r2 < a.rc2)) return false;
-    if (divides_fast(r2)) {
+    if (divides_fast(r2) && !low_ones(r2)) {
         const double y = reciprocal(r2);
         t = pair_terms<LFS>(a, r2, [r2, y](double x) { return quotient(x, r2, y); });
     } else {
@@ -936,8 +936,8 @@ k_lj_halo64(const double4* __restrict__ pos, const int* __restrict__ nbr,
                 const bool in = r2 < a.rc2 && live;
                 const double y = reciprocal(r2);
                 PairTerms p = pair_terms<LFS>(a, r2, [r2, y](double x) { return quotient(x, r2, y); });
-                // below 2^-100 (rc^2 is below 2^400 on this path): as pair_exact
-                if (in && __double2hiint(r2) < 0x39b00000)
+                // as pair_exact (rc^2 is below 2^400 on this path)
+                if (in && (__double2hiint(r2) < 0x39b00000 || low_ones(r2)))
                     p = pair_terms_ieee<LFS>(a.sig2, a.four_eps, a.tf_eps, a.rc, a.uc, a.dudrc, r2);
                 if (in) {
                     acc.fx = __dadd_rn(acc.fx, __dmul_rn(dx, p.s));

@@ -102,7 +102,12 @@ __device__ __forceinline__ void min_image_pair(const Fold3& f, const double4& a,
 // the hardware's approximation (PTX rcp.approx.ftz.f64, about 20 bits), twice; quotient()
 // is Markstein's division (P. Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): q = a y, then q + y (a - b q)
-// with the remainder exact in one fused multiply-add, the correctly rounded a / b.  An
+// with the remainder exact in one fused multiply-add: the correctly rounded a / b wherever
+// y is the correctly rounded 1 / b.  Two steps leave y an ulp low where 1 / b lies above the
+// midpoint of two doubles by less than the iteration's error, 2^-80.  The quotient is then
+// an ulp off only for a dividend that comes within about 2^-106 of such a midpoint itself: one
+// or two of the 2^52 significands of a for such a b, and a power of two only for the b of all
+// ones, so a caller whose dividends may be powers of two leaves out low_ones(b).  An
 // IEEE division has a latency of 126 clocks and costs 12 multiply-adds of throughput
 // here, a shared reciprocal 4 and each quotient 3.  For divisors with divides_fast().
 __device__ __forceinline__ double reciprocal(double b) {
@@ -122,10 +127,12 @@ __device__ __forceinline__ bool divides_fast(double b) {
     return static_cast<unsigned>(__double2hiint(b)) - 0x39b00000u < 0x58f00000u - 0x39b00000u;
 }
 
+// A low word of all ones, the significand of all ones among them.
+__device__ __forceinline__ bool low_ones(double b) { return __double2loint(b) == -1; }
+
 // The same in FP32: one Newton step from rcp.approx gives the correctly rounded reciprocal
-// of every normal divisor (all 2^23 significands tested) but one whose significand is all
-// ones, and quotient() then the IEEE quotient, branch-free.  For 2^-60 <= b < 2^60 and
-// quotients in the normal range.
+// of every divisor (tests/test_gpu_quotients.py: all 2^23 significands), and quotient() then
+// the IEEE quotient, branch-free.  For 2^-60 <= b < 2^60 and quotients in the normal range.
 __device__ __forceinline__ float reciprocal(float b) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
