@@ -51,6 +51,7 @@ struct RealArgs {
     double sig2, four_eps, tf_eps;
     int lj_lfs;             // O-O LJ with linear force shift at the cutoff
     double rc, uc, dudrc;
+    float quotient_r2;      // above this r^2 every dividend and quotient is finite
 };
 
 // Terms of one pair inside the cutoff: force coefficient (F = s d), real-space energy and
@@ -93,7 +94,8 @@ __device__ __forceinline__ RealTerms<T> real_terms(T r2, T r, T cqq, bool coulom
     return t;
 }
 
-// Separations whose quotients could leave the normal range, and in FP64 the squares that
+// Separations whose dividends or quotients could leave the normal range (quotient() turns an
+// infinite dividend into NaN, a division does not), and in FP64 the squares that
 // reciprocal() does not serve with sigma^2 a power of two, divide in IEEE arithmetic.
 template <class T>
 __device__ __noinline__ RealTerms<T> real_terms_ieee(T r2, T cqq, bool coulomb, bool lj,
@@ -106,7 +108,7 @@ __device__ __noinline__ RealTerms<T> real_terms_ieee(T r2, T cqq, bool coulomb, 
 template <class T>
 __device__ __forceinline__ RealTerms<T> real_pair(T r2, T cqq, bool coulomb, bool lj,
                                                   const RealArgs& a) {
-    bool fast = r2 > T(1e-15);
+    bool fast = static_cast<float>(r2) > a.quotient_r2;
     if constexpr (sizeof(T) == 8) fast = fast && !low_ones(r2);
     if (!fast) return real_terms_ieee<T>(r2, cqq, coulomb, lj, &a);
     T r;
@@ -844,7 +846,7 @@ int recip_force_async(md_ewald* ew, md_system* sys, const KArgs& ka, bool charge
     return MD_OK;
 }
 
-RealArgs real_args_of(const md_ewald* ew, double alpha) {
+RealArgs real_args_of(const md_ewald* ew, double alpha, bool mixed) {
     RealArgs a;
     a.rc2 = ew->cutoff * ew->cutoff;
     a.alpha = alpha;
@@ -861,6 +863,10 @@ RealArgs real_args_of(const md_ewald* ew, double alpha) {
     const double s2 = a.sig2 / a.rc2, s6 = s2 * s2 * s2;
     a.uc = 4.0 * ew->epsilon_o * (s6 * s6 - s6);
     a.dudrc = -(24.0 * ew->epsilon_o * (2.0 * s6 * s6 - s6)) / ew->cutoff;
+    // 48 eps (sigma^2 / r^2)^6 and that over r^2 below the largest numbers
+    const double top = std::pow(a.sig2, 6.0) * std::max(2.0, 2.0 * a.tf_eps) / (mixed ? 1e37 : 1e307);
+    a.quotient_r2 = static_cast<float>(
+        std::max({1e-15, std::pow(top, 1.0 / 6.0), std::pow(top, 1.0 / 7.0)}));
     return a;
 }
 
@@ -895,7 +901,7 @@ int ewald_eval_async(md_ewald* ew, md_system* sys, int mode, bool gated, bool ch
         MDB_TRY(ewald_list(ew, sys));
     }
     md_verlet* v = ew->list;
-    const RealArgs a = real_args_of(ew, alpha);
+    const RealArgs a = real_args_of(ew, alpha, ew->mixed);
     double* res = ctx_result(ctx, kResEwald);
     const Box3 box{{sys->box[0], sys->box[1], sys->box[2]},
                    {sys->inv_box[0], sys->inv_box[1], sys->inv_box[2]}};
@@ -1143,7 +1149,7 @@ int md_ewald_charge_gradient(md_ewald* ew, md_system* sys, double* dedq) {
     double* dq_o = dq + n;
     const Box3 box{{sys->box[0], sys->box[1], sys->box[2]},
                    {sys->inv_box[0], sys->inv_box[1], sys->inv_box[2]}};
-    const RealArgs a = real_args_of(ew, ew->alpha);
+    const RealArgs a = real_args_of(ew, ew->alpha, false);
     md_verlet* v = ew->list;
     const int g = grid_for(n, kBlock);
     k_ewald_dq<<<g, kBlock, 0, ctx->stream>>>(
@@ -1180,7 +1186,8 @@ int md_ewald_real_hvp(md_ewald* ew, md_system* sys, const double* u, double* out
     const int g = grid_for(n, kBlock);
     k_ewald_real_hvp<<<g, kBlock, 0, ctx->stream>>>(sys->cur.pos, sys->cur.charge, sys->cur.mol,
                                                    v->nbr.as<int>(), v->count.as<int>(), v->stride,
-                                                   n, box, real_args_of(ew, ew->alpha), ud, res);
+                                                   n, box, real_args_of(ew, ew->alpha, false), ud,
+                                                   res);
     k_to_orig4<<<g, kBlock, 0, ctx->stream>>>(sys->cur.orig, n, res, res_o);
     ctx->launches += 3;
     MDB_CHECK_LAUNCH();
