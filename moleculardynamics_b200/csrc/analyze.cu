@@ -36,7 +36,7 @@ struct md_rdf {
     double sum_rho = 0.0;
     CellGrid grid;
     double grid_box[3] = {0, 0, 0};
-    DevBuf sorted, start;
+    DevBuf sorted, start, crowd;
 };
 
 struct md_corr {                 // shared state of md_msd and md_vacf
@@ -129,26 +129,39 @@ __device__ __forceinline__ int rdf_bin_of(const RdfArgs& a, double r2) {
     return q < static_cast<double>(a.bins) ? static_cast<int>(q) : -1;
 }
 
-// One block per cell (of width rMax or a little more): its atoms against those of itself
+// A block takes a cell (of width rMax or a little more): its atoms against those of itself
 // and 13 of its 26 neighbours, so that every pair of cells is met once.  A warp takes 32 candidates of the flattened
 // neighbour ranges at a time, one per lane, skips them if none lies within rMax of the
 // cell's box, and tests them against the cell's atoms (shared-memory broadcasts) in FP32
 // units of rMax, widened by 1e-4 (their error is below 1e-6); hits, about one test in
 // eight, are queued and settled 32 at a time with the reference's displacement and bin,
-// so no lane idles through the FP64 part.  108,000 atoms, rMax 4: 1,084 us with a thread
-// per atom scanning 27 cells in FP64 (a square root and a division per pair), 247 us.
+// so no lane idles through the FP64 part.
+// Few cells: blocks share a cell's candidates in slices, up to eight blocks per SM in all and
+// no slice below four steps of the block; one block a cell left most SMs idle.
+// Few atoms a cell (a mean below kRdfSparse): k_rdf_sparse, which loads and barriers of a
+// block would dwarf, unless there are too few cells for a thread an atom to hide its chain of
+// loads (64 an SM).  Many bins for a cell's tests (more than 3 mean^2): blocks walk the
+// cells, five an SM (those resident), else each pays for clearing and adding up the bins.
+// Whole frame with the cell sort (us; a thread per atom over 27 cells with a square root and
+// a division a pair; one block a cell; so): 108,000 atoms at density 0.8442 and rMax 4 1,131,
+// 304 and 305; rMax L/6 8,600, 4,260 and 2,080, L/4 113,000, 126,000 and 92,000 (the sort most
+// of it), 10,976 atoms L/3 5,870, 3,240 and 551; density 0.1, rMax 2.5 160, 472 and 120, with
+// 8,000 bins 172, 1,085 and 132; 10,976 atoms, rMax 1.5, 3,375 cells 154, 74 and 70
+// (k_rdf_sparse 105); 500,000 atoms, rMax 2.5, 8,000 bins 1,105, 1,078 and 635.
 constexpr int kRdfWarps = 4;
 constexpr int kRdfTile = 128;  // atoms of the cell staged at once
 
-__global__ void __launch_bounds__(32 * kRdfWarps)
-k_rdf_cells(const double4* __restrict__ pos, RdfGrid g, RdfArgs a, unsigned long long* hist) {
-    extern __shared__ unsigned s_hist[];
+// Cell r against slice `slice` of `slices` of its candidates.  pending: pairs tested since the
+// block's 32-bit histogram was last flushed, at most.
+__device__ __forceinline__ void rdf_cell(const double4* __restrict__ pos, const RdfGrid& g,
+                                         const RdfArgs& a, int r, int slice, int slices,
+                                         unsigned* s_hist, unsigned long long* hist,
+                                         unsigned long long& pending) {
     __shared__ double4 s_p[kRdfTile];
     __shared__ float4 s_f[kRdfTile];
     __shared__ unsigned short s_hit[kRdfWarps][64];  // tile index * 32 + candidate lane
-    const int r = blockIdx.x, h0 = g.start[r], h1 = g.start[r + 1];
+    const int h0 = g.start[r], h1 = g.start[r + 1];
     if (h0 == h1) return;
-    rdf_zero(a, s_hist);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Fold3 f3 = fold3_of(a.box);
     const int cell = g.cell_of_rank[r];
@@ -190,8 +203,17 @@ k_rdf_cells(const double4* __restrict__ pos, RdfGrid g, RdfArgs a, unsigned long
         if (lane >= o) incl += y;
     }
     const int total = __shfl_sync(0xffffffffu, incl, 13), excl = incl - cnt;
+    const int stride = 32 * kRdfWarps * slices;
     for (int hb = h0; hb < h1; hb += kRdfTile) {
         const int hl = min(kRdfTile, h1 - hb);
+        const unsigned long long tests =
+            static_cast<unsigned long long>(hl) * (32 * kRdfWarps) * ((total + stride - 1) / stride);
+        if (pending + tests > 0xffffffffull) {
+            rdf_flush(a, s_hist, hist);
+            rdf_zero(a, s_hist);
+            pending = 0;
+        }
+        pending += tests;
         __syncthreads();
         if (threadIdx.x < hl) {
             const double4 p = ldg4(pos + g.sorted[hb + threadIdx.x]);
@@ -201,7 +223,7 @@ k_rdf_cells(const double4* __restrict__ pos, RdfGrid g, RdfArgs a, unsigned long
             s_f[threadIdx.x] = make_float4(v.x, v.y, v.z, 0.f);
         }
         __syncthreads();
-        for (int c = 32 * warp; c < total; c += 32 * kRdfWarps) {
+        for (int c = 32 * (warp + kRdfWarps * slice); c < total; c += stride) {
             const int f = c + lane;
             int t = f;  // sorted position of this lane's candidate
 #pragma unroll
@@ -259,6 +281,103 @@ k_rdf_cells(const double4* __restrict__ pos, RdfGrid g, RdfArgs a, unsigned long
             __syncwarp();
             settle(lane < queued, lane);
             __syncwarp();
+        }
+    }
+}
+
+// Cells that k_rdf_sparse leaves to k_rdf_cells, a slice of their candidates for every 128 of
+// their atoms, so that a clump in an empty box is not one block's.
+struct RdfCrowd {
+    int2* unit;  // cell, slice
+    int* count;
+};
+
+__device__ __forceinline__ int crowd_slices(int atoms) { return (atoms + kRdfTile - 1) / kRdfTile; }
+
+// One block a unit (cell, slice of its candidates), or with WALK blocks that walk the units, of
+// the crowd list or else `slices` of every cell, and clear and add up the histogram once.
+template <bool WALK>
+__global__ void __launch_bounds__(32 * kRdfWarps, 5)
+k_rdf_cells(const double4* __restrict__ pos, RdfGrid g, RdfArgs a, RdfCrowd crowd, int slices,
+            unsigned long long* hist) {
+    extern __shared__ unsigned s_hist[];
+    unsigned long long pending = 0;
+    if (!WALK) {
+        const int r = blockIdx.x / slices;
+        if (g.start[r] == g.start[r + 1]) return;
+        rdf_zero(a, s_hist);
+        rdf_cell(pos, g, a, r, blockIdx.x % slices, slices, s_hist, hist, pending);
+    } else {
+        const int units = crowd.unit ? *crowd.count : g.ncells * slices;
+        if (static_cast<int>(blockIdx.x) >= units) return;
+        rdf_zero(a, s_hist);
+        for (int u = blockIdx.x; u < units; u += gridDim.x) {
+            int r = u / slices, slice = u % slices, of = slices;
+            if (crowd.unit) {
+                const int2 e = crowd.unit[u];
+                r = e.x;
+                slice = e.y;
+                of = crowd_slices(g.start[r + 1] - g.start[r]);
+            }
+            rdf_cell(pos, g, a, r, slice, of, s_hist, hist, pending);
+        }
+    }
+    rdf_flush(a, s_hist, hist);
+}
+
+// The same pairs where cells hold a few atoms each: a thread per sorted position, its atom
+// against the later ones of its cell and those of the 13 neighbours above.  A cell with more
+// than kRdfCrowded candidates, too long a chain for a thread (a droplet of 108,000 atoms in 64
+// times its volume 650 us instead of 380), goes to the crowd list.
+constexpr double kRdfSparse = 6.0;
+constexpr int kRdfCrowded = 112;
+
+__global__ void __launch_bounds__(kRdfBlock)
+k_rdf_sparse(const double4* __restrict__ pos, int64_t n, RdfGrid g, RdfArgs a, RdfCrowd crowd,
+             unsigned long long* hist) {
+    extern __shared__ unsigned s_hist[];
+    rdf_zero(a, s_hist);
+    const int64_t s = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    if (s < n) {
+        int r = 0, hi = g.ncells;  // the rank whose range holds s
+        while (hi - r > 1) {
+            const int mid = (r + hi) >> 1;
+            if (g.start[mid] <= s) r = mid;
+            else hi = mid;
+        }
+        const int cell = g.cell_of_rank[r];
+        const int cx = cell % g.nx, cy = (cell / g.nx) % g.ny, cz = cell / (g.nx * g.ny);
+        const auto range = [&](int q) {  // of neighbour q, 13 the cell itself
+            int jx = cx + (q % 3) - 1, jy = cy + ((q / 3) % 3) - 1, jz = cz + (q / 9) - 1;
+            jx = jx < 0 ? jx + g.nx : (jx >= g.nx ? jx - g.nx : jx);
+            jy = jy < 0 ? jy + g.ny : (jy >= g.ny ? jy - g.ny : jy);
+            jz = jz < 0 ? jz + g.nz : (jz >= g.nz ? jz - g.nz : jz);
+            const int rr = g.rank_of_cell[jx + g.nx * (jy + g.ny * jz)];
+            return make_int2(g.start[rr], g.start[rr + 1]);
+        };
+        int64_t total = 0;
+        for (int q = 13; q < 27; ++q) {
+            const int2 t = range(q);
+            total += t.y - t.x;
+        }
+        const double4 p = ldg4(pos + g.sorted[s]);
+        if (total > kRdfCrowded) {
+            const int2 own = range(13);
+            if (s - own.x < crowd_slices(own.y - own.x))
+                crowd.unit[atomicAdd(crowd.count, 1)] = make_int2(r, static_cast<int>(s - own.x));
+        } else if (rdf_selected(a, p.w)) {
+            const Fold3 f3 = fold3_of(a.box);
+            for (int q = 13; q < 27; ++q) {
+                const int2 in = range(q);
+                for (int t = q == 13 ? static_cast<int>(s) + 1 : in.x; t < in.y; ++t) {
+                    const double4 o = ldg4(pos + g.sorted[t]);
+                    double dx, dy, dz;
+                    min_image_pair(f3, p, o, p.w < o.w, dx, dy, dz);
+                    const double r2 = norm2_exact(dx, dy, dz);
+                    if (r2 < a.rmax2_hi && rdf_selected(a, o.w))
+                        rdf_count(a, s_hist, hist, rdf_bin_of(a, r2));
+                }
+            }
         }
     }
     rdf_flush(a, s_hist, hist);
@@ -505,6 +624,7 @@ int md_rdf_destroy(md_rdf* r) {
     r->hist.release();
     r->sorted.release();
     r->start.release();
+    r->crowd.release();
     r->grid.release();
     delete r;
     return MD_OK;
@@ -584,8 +704,28 @@ int rdf_frame_launch(md_rdf* r, md_system* sys, int64_t first, int64_t stride) {
             MDB_TRY(cell_sort(sys, r->grid, r->sorted.as<int>(), r->start.as<int>()));
             RdfGrid g{r->grid.nx, r->grid.ny, r->grid.nz, r->grid.ncells, r->grid.rank_of_cell,
                       r->grid.cell_of_rank, r->start.as<int>(), r->sorted.as<int>()};
-            k_rdf_cells<<<r->grid.ncells, 32 * kRdfWarps, shm, ctx->stream>>>(
-                sys->cur.pos, g, a, r->hist.as<unsigned long long>());
+            const double mean = static_cast<double>(n) / g.ncells;
+            RdfCrowd crowd{nullptr, nullptr};
+            int64_t slices = 1, blocks;
+            bool walk = true;
+            if (mean < kRdfSparse && g.ncells > 64 * ctx->sm_count) {
+                MDB_TRY(r->crowd.ensure(sizeof(int2) * static_cast<size_t>(n + n / kRdfTile + 2)));
+                crowd = RdfCrowd{r->crowd.as<int2>() + 1, r->crowd.as<int>()};
+                MDB_CUDA(cudaMemsetAsync(crowd.count, 0, sizeof(int), ctx->stream));
+                k_rdf_sparse<<<grid_for(n, kRdfBlock), kRdfBlock, shm, ctx->stream>>>(
+                    sys->cur.pos, n, g, a, crowd, r->hist.as<unsigned long long>());
+                ++ctx->launches;
+                blocks = 32 * ctx->sm_count;
+            } else {
+                slices = std::max<int64_t>(1, std::min<int64_t>(8 * ctx->sm_count / g.ncells,
+                                                                static_cast<int64_t>(14.0 * mean / 512)));
+                walk = a.use_shared && a.bins > 3.0 * mean * mean;
+                blocks = g.ncells * slices;
+                if (walk) blocks = std::min<int64_t>(blocks, 5 * ctx->sm_count);
+            }
+            auto kernel = walk ? k_rdf_cells<true> : k_rdf_cells<false>;
+            kernel<<<static_cast<unsigned>(blocks), 32 * kRdfWarps, shm, ctx->stream>>>(
+                sys->cur.pos, g, a, crowd, static_cast<int>(slices), r->hist.as<unsigned long long>());
         } else {
             // spans of a multiple of 32 atoms, enough of them for two blocks per SM
             const int64_t xblocks = grid_for(n, kRdfBlock);
