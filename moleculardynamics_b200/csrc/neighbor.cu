@@ -473,18 +473,26 @@ __device__ __forceinline__ void build_report(int local_max, int lane, int stride
 // pair set (forEachPair) applies the reference's exact test to the positions of
 // the build and is bit-identical to the reference's.
 // Rows list candidates in stencil order, atoms of a cell in sorted order.
-__device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ pos,
+// Candidates are staged in pairs, structure-of-arrays within a pair so that two
+// are tested with one packed FP32x2 instruction per step:
+// a[p] = (-x0, -x1, -y0, -y1), b[p] = (-z0, -z1, j0, j1).
+template <int CAND>
+struct CandidatePairs {
+    float4 a[kBuildWarps][CAND / 2];
+    float4 b[kBuildWarps][CAND / 2];
+};
+
+template <int CAND>
+__device__ __forceinline__ void verlet_cells_body(CandidatePairs<CAND>& staged,
+                                                  const double4* __restrict__ pos,
                                                   const int* __restrict__ start, const GridArgs& g,
                                                   double rl2, int* __restrict__ nbr,
                                                   int* __restrict__ count, int stride,
                                                   uint32_t* status, int* max_count, int groups,
                                                   unsigned block) {
-    // Candidates in pairs, structure-of-arrays within a pair so that two
-    // candidates are tested with one packed FP32x2 instruction per step:
-    // s_a[p] = (-x0, -x1, -y0, -y1), s_b[p] = (-z0, -z1, j0, j1).
-    __shared__ float4 s_a[kBuildWarps][kMaxCand / 2];
-    __shared__ float4 s_b[kBuildWarps][kMaxCand / 2];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float4* const s_a = staged.a[warp];
+    float4* const s_b = staged.b[warp];
     // `groups` warps share a crowded cell, each taking every groups-th run of 32 atoms
     const int wid = static_cast<int>(block) * kBuildWarps + warp;
     const int r = wid / groups, grp = wid % groups;
@@ -494,8 +502,8 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
     const float hi_thr = bc.hi_thr;
     const int a0 = start[r], a1 = start[r + 1];
     int local_max = 0;
-    for (int wb = 0; wb < total; wb += kMaxCand) {
-        const int wlen = min(kMaxCand, total - wb);
+    for (int wb = 0; wb < total; wb += CAND) {
+        const int wlen = min(CAND, total - wb);
         __syncwarp();
         // stage candidates [wb, wb + wlen)
         int ns = 0;
@@ -509,8 +517,8 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
             const unsigned m = __ballot_sync(0xffffffffu, keep);
             if (keep) {
                 const int tt = ns + __popc(m & ((1u << lane) - 1u)), pr = tt >> 1, h = tt & 1;
-                float* A = reinterpret_cast<float*>(&s_a[warp][pr]);
-                float* B = reinterpret_cast<float*>(&s_b[warp][pr]);
+                float* A = reinterpret_cast<float*>(&s_a[pr]);
+                float* B = reinterpret_cast<float*>(&s_b[pr]);
                 A[h] = -cx32;
                 A[2 + h] = -cy32;
                 B[h] = -cz32;
@@ -519,8 +527,8 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
             ns += __popc(m);
         }
         if ((ns & 1) && lane == 0) {  // pad the odd slot: infinitely far, no atom
-            float* A = reinterpret_cast<float*>(&s_a[warp][ns >> 1]);
-            float* B = reinterpret_cast<float*>(&s_b[warp][ns >> 1]);
+            float* A = reinterpret_cast<float*>(&s_a[ns >> 1]);
+            float* B = reinterpret_cast<float*>(&s_b[ns >> 1]);
             A[1] = A[3] = B[1] = 1e30f;
             B[3] = __int_as_float(-1);
         }
@@ -541,7 +549,7 @@ __device__ __forceinline__ void verlet_cells_body(const double4* __restrict__ po
             const int npairs = (ns + 1) >> 1;
 #pragma unroll 2
             for (int pr = 0; pr < npairs; ++pr) {
-                const float4 A = s_a[warp][pr], B = s_b[warp][pr];
+                const float4 A = s_a[pr], B = s_b[pr];
                 const float2 dx = __fadd2_rn(fx2, make_float2(A.x, A.y));
                 const float2 dy = __fadd2_rn(fy2, make_float2(A.z, A.w));
                 const float2 dz = __fadd2_rn(fz2, make_float2(B.x, B.y));
@@ -568,7 +576,8 @@ k_verlet_cells(const double4* __restrict__ pos, const int* __restrict__ start, G
                double rl2, int* __restrict__ nbr, int* __restrict__ count, int stride,
                uint32_t* status, int* max_count, const int* flag, int groups) {
     if (!gate(flag)) return;
-    verlet_cells_body(pos, start, g, rl2, nbr, count, stride, status, max_count, groups, blockIdx.x);
+    __shared__ CandidatePairs<kMaxCand> staged;
+    verlet_cells_body(staged, pos, start, g, rl2, nbr, count, stride, status, max_count, groups, blockIdx.x);
 }
 
 // The atoms ib .. ib + A of a cell against 32 candidates, one a lane: the hits in candidate
@@ -626,8 +635,18 @@ __device__ __forceinline__ void store_counts(const int (&c)[A], int ib, int a1, 
 // whole build: 254 us by lanes over atoms, 180 so (two atoms a warp 204, eight 220); at
 // density 0.3 (6.6 a cell) 213 and 231.
 constexpr int kSparseAtoms = 4;
+// Cells of more than kSparseCrowd atoms (a droplet, a slab, in a mostly empty box) take the lane
+// an atom after all, their candidates staged kSparseCand at a time so that the other warps keep
+// their blocks and L1.  186,624 liquid atoms in 27 times their volume, whole build: 329 us by
+// lanes over atoms alone, 351 by lanes over candidates alone, 241 so (a line of 16 atoms 276);
+// in 5.8 times their volume 227, 292 and 230.  With windows of 576 the gas of density 0.15
+// took 275 us instead of 202.
+constexpr int kSparseCrowd = 8;
+constexpr int kSparseCand = 128;
 
-__device__ __forceinline__ void verlet_sparse_body(const double4* __restrict__ pos,
+template <int CAND>
+__device__ __forceinline__ void verlet_sparse_body(CandidatePairs<CAND>& staged,
+                                                   const double4* __restrict__ pos,
                                                    const int* __restrict__ start, const GridArgs& g,
                                                    double rl2, int* __restrict__ nbr,
                                                    int* __restrict__ count, int stride,
@@ -640,6 +659,11 @@ __device__ __forceinline__ void verlet_sparse_body(const double4* __restrict__ p
     if (r >= g.ncells) return;
     const int a0 = start[r], a1 = start[r + 1];
     if (a0 + A * grp >= a1) return;
+    if (a1 - a0 > kSparseCrowd) {
+        verlet_cells_body(staged, pos, start, g, rl2, nbr, count, stride, status, max_count, groups,
+                          block);
+        return;
+    }
     const BuildCell bc = build_cell(g, start, rl2, r, lane);
     const unsigned below = (1u << lane) - 1u;
     int local_max = 0;
@@ -673,7 +697,8 @@ k_verlet_sparse(const double4* __restrict__ pos, const int* __restrict__ start, 
                 double rl2, int* __restrict__ nbr, int* __restrict__ count, int stride,
                 uint32_t* status, int* max_count, const int* flag, int groups) {
     if (!gate(flag)) return;
-    verlet_sparse_body(pos, start, g, rl2, nbr, count, stride, status, max_count, groups, blockIdx.x);
+    __shared__ CandidatePairs<kSparseCand> staged;
+    verlet_sparse_body(staged, pos, start, g, rl2, nbr, count, stride, status, max_count, groups, blockIdx.x);
 }
 
 // The same rows for systems too small to fill the GPU with a warp a cell (864 atoms are 27
@@ -1299,11 +1324,12 @@ k_batch_rebuild_cells(const RebuildRep* __restrict__ reps, const int4* __restric
     const int4 e = __ldg(blk + blockIdx.x);
     const RebuildRep& d = reps[e.x];
     if (!gate(d.flag)) return;
+    __shared__ CandidatePairs<kMaxCand> staged;
     if (d.sparse)
-        verlet_sparse_body(d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
+        verlet_sparse_body(staged, d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
                            d.max_count, d.groups, e.y);
     else
-        verlet_cells_body(d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
+        verlet_cells_body(staged, d.cur.pos, d.start, d.g, d.rl2, d.nbr, d.count, d.stride, d.status,
                           d.max_count, d.groups, e.y);
 }
 
