@@ -259,8 +259,9 @@ MD_API int md_lj_set_tile_threads(md_lj* lj, int tpa);
 /* Halo tiles of a Verlet list: built now from the current list and again at
  * every rebuild (on = 1), or dropped (0).  md_run_lj and md_batch_run turn them on
  * by themselves for mixed-precision systems of >= 65,536 atoms, and md_run_lj for
- * FP64 ones of >= 196,608, where the faster force kernel pays for building them.  Lists without a cell grid
- * (fewer than 3 cells per side) keep none.  No reference counterpart. */
+ * FP64 ones of >= 196,608 with 13 to 30 atoms a cell of the list, where the faster
+ * force kernel pays for building them.  Lists without a cell grid (fewer than 3
+ * cells per side) keep none.  No reference counterpart. */
 MD_API int md_verlet_set_halo(md_verlet* v, int on);
 /* How many of a list's halo tiles are staged in shared memory (the rest gather
  * through the int32 rows), out of how many (0, 0 without tiles).  Diagnostics;

@@ -1819,7 +1819,7 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
     // halo tiles, when the list keeps them (fused runs of large systems turn them on,
     // or md_verlet_set_halo)
     const bool halo = lj->halo && sys->n > 0 && v->halo_on && v->stride % 8 == 0 &&
-                      (mixed || (sys->wrapped && a.rc2 < 0x1p400));
+                      (mixed || (sys->wrapped && a.rc2 < 0x1p400 && verlet_halo_pays64(v, sys->n)));
     ctx_time_begin(ctx, MD_KERNEL_LJ_FORCE);
     const bool cubic = a.res[0] == a.res[1] && a.res[0] == a.res[2];
     if (halo && !mixed) {

@@ -311,6 +311,7 @@ struct md_verlet {
     // Halo tiles (mixed-precision force path): per block of kHaloAtoms sorted
     // atoms, runs of the cells around them and the rows as 16-bit halo slots.
     bool halo_on = false;
+    bool halo_asked = false;        // by the caller (md_verlet_set_halo), not by a run
     mdb::DevBuf halo_runs;          // blocks * kHaloRuns int2 (first atom, slot base)
     mdb::DevBuf halo_meta;          // blocks int2 (runs or -1 when not staged, atoms)
     mdb::DevBuf nbr16;              // n * stride halo slots
@@ -334,7 +335,17 @@ constexpr int64_t kHaloMinAtoms = 65536;
 // atoms 19 of 154 us against 65, at 1,048,576 atoms 125 of 523 us against 257 (a rebuild
 // every seven steps or so).
 constexpr int64_t kHaloMinAtoms64 = 196608;
+// ... and only where nearly every tile is staged, since a tile that is not costs the FP64
+// pass more than the gathered kernel: between these mean occupancies of the list's cells.
+// Below, 128 atoms span too many cells; above, a tile exceeds its slots.  40 steps, gathered
+// and over tiles (ms): 864,000 atoms at 6.9 atoms a cell 11.2 and 20.3, 10.1 14.7 and 15.7,
+// 11.7 15.4 and 16.3, 13.5 17.7 and 16.8, 15.7 18.1 and 17.0, 20.2 20.2 and 16.7, 26.4 25.1
+// and 21.3, 32 31.5 and 29.8, 39.4 36.7 and 44.7, 71 (a cutoff of 4 in the liquid) 63 and
+// 144; 256,000 atoms at 14.6 6.3 and 5.9, 24 8.5 and 7.1, 27.6 9.0 and 9.0, 32 11.1 and 11.2.
+constexpr double kHaloMinMean64 = 13.0, kHaloMaxMean64 = 30.0;
 inline int64_t halo_blocks(int64_t n) { return (n + kHaloAtoms - 1) / kHaloAtoms; }
+// Whether an FP64 pass gains from this list's tiles (or its caller asked for them).
+bool verlet_halo_pays64(const md_verlet* v, int64_t n);
 // Turns the halo tiles on for this list (built right away from the current list
 // unless the stream is capturing); false when they cannot be used.
 bool verlet_halo_ready(md_verlet* v, md_system* sys);

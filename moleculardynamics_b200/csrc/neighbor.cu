@@ -1553,9 +1553,15 @@ bool verlet_halo_ready(md_verlet* v, md_system* sys) {
     return true;
 }
 
+bool verlet_halo_pays64(const md_verlet* v, int64_t n) {
+    if (v->halo_asked) return true;
+    const double mean = static_cast<double>(n) / std::max(v->grid.ncells, 1);
+    return n >= kHaloMinAtoms64 && mean >= kHaloMinMean64 && mean <= kHaloMaxMean64;
+}
+
 void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj, bool batch) {
     const bool mixed = lj->precision == MD_PRECISION_MIXED;
-    if (lj->halo && (mixed ? sys->n >= kHaloMinAtoms : !batch && sys->n >= kHaloMinAtoms64))
+    if (lj->halo && (mixed ? sys->n >= kHaloMinAtoms : !batch && verlet_halo_pays64(v, sys->n)))
         verlet_halo_ready(v, sys);
 }
 
@@ -2009,13 +2015,14 @@ int md_verlet_set_capacity(md_verlet* v, int capacity, int fixed) {
 int md_verlet_set_halo(md_verlet* v, int on) {
     graph_epoch_bump();
     if (!v) return fail(MD_ERR_INVALID_ARGUMENT, "md_verlet_set_halo: NULL");
+    v->halo_asked = false;
     if (!on) {
         v->halo_on = false;
         return MD_OK;
     }
     if (!v->sys) return fail(MD_ERR_INVALID_ARGUMENT, "md_verlet_set_halo: list was never built");
     MDB_TRY(verlet_ready(v, v->sys, "md_verlet_set_halo"));
-    verlet_halo_ready(v, v->sys);  // a list without a cell grid keeps gathering
+    v->halo_asked = verlet_halo_ready(v, v->sys);  // a list without a cell grid keeps gathering
     return ctx_check_status(v->ctx);
 }
 
