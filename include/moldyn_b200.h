@@ -245,9 +245,12 @@ MD_API int md_lj_set_unroll(int unroll);
  * (moleculardynamics_b200/autotune.py); no reference counterpart. */
 MD_API int md_lj_set_launch(md_lj* lj, int tpa, int unroll);
 /* Read neighbours through the list's halo tiles when it keeps them (on = 1, the
- * default) or always gather them through the int32 rows (0).  A halo tile holds a block of 128 cell-sorted atoms and every atom of the
- * cells around them in shared memory; rows then also exist as 16-bit tile slots.
- * Forces are identical either way.  No reference counterpart. */
+ * default) or always gather them through the int32 rows (0).  A halo tile holds a
+ * block of 128 cell-sorted atoms and every atom of the cells around them in shared
+ * memory; rows then also exist as 16-bit tile slots.  FP64 forces are identical
+ * either way: the tiles serve the default two threads per atom, other launch shapes
+ * gather.  Mixed forces over tiles are those of two threads per atom, whatever the
+ * shape asked for.  No reference counterpart. */
 MD_API int md_lj_set_halo(md_lj* lj, int on);
 /* Shape of the mixed tile kernel: 0 (the default) one CTA per tile with two threads
  * per atom, the halo staged by the threads; 1 the same with the halo queued by bulk

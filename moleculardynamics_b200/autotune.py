@@ -21,6 +21,7 @@ import ctypes as C
 import json
 import math
 import os
+import re
 
 import moleculardynamics_b200 as md
 
@@ -49,14 +50,28 @@ def _store(path, table):
     os.replace(tmp, path)
 
 
-def problem_key(ctx, sys, lj, verlet_cutoff, skin):
+def _default_kernel(ctx, n, lj, verlet):
+    """What the default shape runs where that is not the plain two-thread pass: FP64 systems
+    below 64 and 256 atoms per SM take sixteen and four lanes an atom, and a list may keep
+    halo tiles."""
+    sms = re.search(r"\((\d+) SMs\)", ctx.device_name())
+    key = []
+    if sms and lj.precision == md.PRECISION_FP64 and n < 256 * int(sms.group(1)):
+        key.append("lanes16" if n < 64 * int(sms.group(1)) else "lanes4")
+    if verlet is not None and verlet.halo_tiles()[1] > 0:
+        key.append("tiles")
+    return key
+
+
+def problem_key(ctx, sys, lj, verlet_cutoff, skin, verlet=None):
     """Size bucket (powers of two) and density to two figures: launch shapes that
-    win on one system win on its neighbours."""
+    win on one system win on its neighbours where the default shape means the same kernel."""
     n = sys.n
     rho = n / sys.volume()
     return "|".join([ctx.device_name(), f"n2^{max(0, int(round(math.log2(max(n, 1)))))}",
                      f"rho{rho:.2g}", f"rc{lj.cutoff:g}", f"skin{skin:g}",
-                     f"trunc{lj.truncation}", f"prec{lj.precision}"])
+                     f"trunc{lj.truncation}", f"prec{lj.precision}"]
+                    + _default_kernel(ctx, n, lj, verlet))
 
 
 def time_force_kernel(ctx, sys, lj, verlet, repeats=5):
@@ -76,10 +91,12 @@ def time_force_kernel(ctx, sys, lj, verlet, repeats=5):
 
 def tune_force_kernel(sys, lj, verlet, skin, shapes=SHAPES, repeats=5, use_cache=True):
     """Applies and returns the fastest (tpa, unroll) for this problem; the dict of
-    timings is returned too (empty when the answer came from the cache)."""
+    timings is returned too (empty when the answer came from the cache).  Two threads an
+    atom read the list's halo tiles if it keeps them: for a system whose fused runs do, tune
+    after a first run or verlet.set_halo(True)."""
     ctx = sys.ctx
     path = cache_path()
-    key = problem_key(ctx, sys, lj, lj.cutoff, skin)
+    key = problem_key(ctx, sys, lj, lj.cutoff, skin, verlet)
     table = _load(path) if use_cache else {}
     if key in table:
         tpa, unroll = table[key]["shape"]

@@ -1798,6 +1798,8 @@ int lj_quantize_async(md_lj* lj, md_system* sys, const int* gate) {
     return MD_OK;
 }
 
+bool lj_halo64_shape(const md_lj* lj) { return (lj->tpa ? lj->tpa : g_lj_tpa) == 2; }
+
 int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q_gate,
                            bool q_current, const KickArgs* kick, bool* kicked) {
     if (kicked) *kicked = false;
@@ -1819,7 +1821,8 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
     // halo tiles, when the list keeps them (fused runs of large systems turn them on,
     // or md_verlet_set_halo)
     const bool halo = lj->halo && sys->n > 0 && v->halo_on && v->stride % 8 == 0 &&
-                      (mixed || (sys->wrapped && a.rc2 < 0x1p400 && verlet_halo_pays64(v, sys->n)));
+                      (mixed || (lj_halo64_shape(lj) && sys->wrapped && a.rc2 < 0x1p400 &&
+                                 verlet_halo_pays64(v, sys->n)));
     ctx_time_begin(ctx, MD_KERNEL_LJ_FORCE);
     const bool cubic = a.res[0] == a.res[1] && a.res[0] == a.res[2];
     if (halo && !mixed) {

@@ -344,6 +344,8 @@ constexpr int64_t kHaloMinAtoms64 = 196608;
 // 144; 256,000 atoms at 14.6 6.3 and 5.9, 24 8.5 and 7.1, 27.6 9.0 and 9.0, 32 11.1 and 11.2.
 constexpr double kHaloMinMean64 = 13.0, kHaloMaxMean64 = 30.0;
 inline int64_t halo_blocks(int64_t n) { return (n + kHaloAtoms - 1) / kHaloAtoms; }
+// The FP64 tile kernel sums as two threads an atom do; other shapes gather, in their order.
+bool lj_halo64_shape(const md_lj* lj);
 // Whether an FP64 pass gains from this list's tiles (or its caller asked for them).
 bool verlet_halo_pays64(const md_verlet* v, int64_t n);
 // Turns the halo tiles on for this list (built right away from the current list

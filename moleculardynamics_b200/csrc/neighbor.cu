@@ -1561,7 +1561,8 @@ bool verlet_halo_pays64(const md_verlet* v, int64_t n) {
 
 void verlet_halo_for_run(md_verlet* v, md_system* sys, const md_lj* lj, bool batch) {
     const bool mixed = lj->precision == MD_PRECISION_MIXED;
-    if (lj->halo && (mixed ? sys->n >= kHaloMinAtoms : !batch && verlet_halo_pays64(v, sys->n)))
+    if (lj->halo && (mixed ? sys->n >= kHaloMinAtoms
+                           : !batch && lj_halo64_shape(lj) && verlet_halo_pays64(v, sys->n)))
         verlet_halo_ready(v, sys);
 }
 
