@@ -868,8 +868,8 @@ __device__ __noinline__ ExactSums gathered_row_exact(LJArgs a, Box3 box,
 // overlap.  1,048,576-atom liquid, kick included: 606 us with two IEEE divisions a pair,
 // 525 us with the shared reciprocal, 397 us from tiles (two entries side by side, or their
 // loads ahead of the arithmetic of four, spill past 80 registers: 467 to 530 us).
-// Wrapped coordinates only.  A list with cells has three of them a side, so a pair near
-// half a box length is beyond the cutoff whichever way it folds.
+// Wrapped coordinates and cutoffs below half the box only: a pair near half a box length is
+// then beyond the cutoff whichever way it folds.
 constexpr int kHalo64Cap = 2304;  // slots: three blocks per SM; tiles with more gather
 
 template <bool LFS, bool KICK>
@@ -1820,9 +1820,10 @@ int lj_forces_verlet_async(md_lj* lj, md_system* sys, md_verlet* v, const int* q
     if (!q_current) MDB_TRY(lj_quantize_async(lj, sys, q_gate));
     // halo tiles, when the list keeps them (fused runs of large systems turn them on,
     // or md_verlet_set_halo)
+    const double half_box = 0.4999 * std::min({sys->box[0], sys->box[1], sys->box[2]});
     const bool halo = lj->halo && sys->n > 0 && v->halo_on && v->stride % 8 == 0 &&
-                      (mixed || (lj_halo64_shape(lj) && sys->wrapped && a.rc2 < 0x1p400 &&
-                                 verlet_halo_pays64(v, sys->n)));
+                      (mixed || (lj_halo64_shape(lj) && sys->wrapped && a.rc < half_box &&
+                                 a.rc2 < 0x1p400 && verlet_halo_pays64(v, sys->n)));
     ctx_time_begin(ctx, MD_KERNEL_LJ_FORCE);
     const bool cubic = a.res[0] == a.res[1] && a.res[0] == a.res[2];
     if (halo && !mixed) {
