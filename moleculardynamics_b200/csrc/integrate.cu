@@ -27,6 +27,7 @@ namespace {
 constexpr int kBlock = 256;
 
 // Where a fused run stands, on the device: a captured step cannot carry a step number.
+// Begins with the row index that a step in a batch has alone.
 struct RunCursor {
     int done;  // steps recorded (the next thermo row)
     int left;  // captured steps to go, counted down by each one's displacement check
@@ -320,7 +321,6 @@ __device__ __forceinline__ void nhc_post_body(NhcState* st, const double* ke_sum
     st->scale = nhc_half(st, 0.5 * st->dt, w, ke);
     st->ke = ke;
 }
-
 
 __global__ void k_nhc_post(NhcState* st, const double* ke_sum, Weights w) { nhc_post_body(st, ke_sum, w); }
 
@@ -631,18 +631,20 @@ int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj*
                          double* rows, int* idx, cudaGraph_t graph, int64_t* main_launches,
                          int64_t* body_launches, const cudaGraphConditionalHandle* loop) {
     md_context* ctx = sys->ctx;
-    NhcState* nhc = nhc_of(it);
+    RunCursor* run = loop ? reinterpret_cast<RunCursor*>(idx) : nullptr;
+    if (it->kind == 1 && !run)
+        return fail(MD_ERR_INVALID_ARGUMENT, "a captured Langevin step reads its number from a run's cursor");
     const int64_t l0 = ctx->launches;
     int rc = MD_OK;
     cudaGraphConditionalHandle h;
     if (cudaGraphConditionalHandleCreate(&h, graph, 0, cudaGraphCondAssignDefault) != cudaSuccess)
         return fail(MD_ERR_CUDA, "cudaGraphConditionalHandleCreate failed");
-    const StepHandles hs{h, loop ? *loop : 0, loop ? idx + 1 : nullptr};  // RunCursor::left
+    const StepHandles hs{h, run ? *loop : 0, run ? &run->left : nullptr};
     std::vector<cudaGraphNode_t> leaves;
     int4* q = nullptr;
     MDB_TRY(step_quantize_target(it, sys, lj, &q));  // allocated by the first, eager step
     rc = capture_into(ctx, graph, nullptr, 0, [&]() -> int {
-        return pre_force(it, sys, v, false, q, reinterpret_cast<const RunCursor*>(idx), &hs);
+        return pre_force(it, sys, v, false, q, run, &hs);
     }, &leaves);
     const int64_t l1 = ctx->launches;
     cudaGraphNode_t cond = nullptr;

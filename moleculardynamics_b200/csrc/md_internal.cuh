@@ -385,7 +385,8 @@ int nhc_apply_scale_async(md_integrator* it, md_system* sys);
 // when a rebuild is due; post_force).
 int vv_pre_async(md_integrator* it, md_system* sys, md_verlet* check, int* sticky);
 int vv_post_async(md_integrator* it, md_system* sys);
-// One fused step captured into `graph`; loop: the loop node whose body that is, or null.
+// One fused step captured into `graph`; loop: the loop node whose body that is, idx then the
+// run's cursor (md_run_lj), or null, idx the next row alone (a batch; no Langevin step).
 int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj* lj,
                          double* rows, int* idx, cudaGraph_t graph, int64_t* main_launches,
                          int64_t* body_launches, const cudaGraphConditionalHandle* loop);
