@@ -606,9 +606,19 @@ struct BatchForceRep {
 
 // The force pass of many systems in one launch: each block finds its system in
 // the block table and runs exactly the blocks a launch of that system alone
-// would, so every system's forces and sums equal its solo pass.
-template <int TPA, bool MIXED, bool LFS, int U, bool CUBIC, bool KICK>
-__global__ void __launch_bounds__(kBlock, UnrollBlocks<U, MIXED>::value)
+// would, so every system's forces and sums equal its solo pass.  The system's arguments come
+// from shared memory where the solo pass reads its parameters as operands, so FP64 terms
+// spill at the solo pass's two gathers in flight and four blocks: one gather and three blocks
+// (80 registers).  Eight replicas of 32,000 and 70,304 liquid atoms, 40 steps: truncated 16.7
+// ms with IEEE divisions, 17.8 with quotients, 13.6 so; shifted 17.2, 22.3 and 15.4; gas of
+// density 0.1 10.2, 9.2 and 9.1 (one gather alone 8.6, shifted liquid 17.0).
+template <bool MIXED>
+struct BatchShape {
+    static constexpr int unroll = MIXED ? 2 : 1, blocks = MIXED ? UnrollBlocks<2, true>::value : 3;
+};
+
+template <int TPA, bool MIXED, bool LFS, bool CUBIC, bool KICK>
+__global__ void __launch_bounds__(kBlock, BatchShape<MIXED>::blocks)
 k_lj_verlet_batch(const BatchForceRep* __restrict__ reps, const int4* __restrict__ blk) {
     // the system's arguments are read from shared memory as the solo kernel reads
     // its parameters, rather than held in registers
@@ -616,7 +626,7 @@ k_lj_verlet_batch(const BatchForceRep* __restrict__ reps, const int4* __restrict
     const int4 e = __ldg(blk + blockIdx.x);
     if (threadIdx.x == 0) d = reps[e.x];
     __syncthreads();
-    lj_verlet_body<TPA, MIXED, LFS, U, CUBIC, KICK>(
+    lj_verlet_body<TPA, MIXED, LFS, BatchShape<MIXED>::unroll, CUBIC, KICK>(
         static_cast<const typename PosOf<MIXED>::T*>(d.pos), d.pd, d.nbr, d.count, d.stride, d.n,
         d.box, d.a, d.fx, d.fy, d.fz, d.part, d.ticket, d.out, e.y, e.z, d.kick);
 }
@@ -1948,9 +1958,9 @@ namespace {
 
 template <int TPA, bool MIXED, bool LFS, bool CUBIC>
 void batch_force_t(BatchForce* b, cudaStream_t s) {
-    auto kernel = k_lj_verlet_batch<TPA, MIXED, LFS, 2, CUBIC, false>;
+    auto kernel = k_lj_verlet_batch<TPA, MIXED, LFS, CUBIC, false>;
     if constexpr (verlet_kicks(TPA, 2))
-        if (b->kick) kernel = k_lj_verlet_batch<TPA, MIXED, LFS, 2, CUBIC, true>;
+        if (b->kick) kernel = k_lj_verlet_batch<TPA, MIXED, LFS, CUBIC, true>;
     kernel<<<b->total, kBlock, 0, s>>>(b->reps.as<BatchForceRep>(), b->blk.as<int4>());
 }
 
