@@ -16,6 +16,7 @@
 // pass over the real-space list.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <new>
 #include <type_traits>
 #include <unordered_map>
@@ -51,7 +52,8 @@ struct RealArgs {
     double sig2, four_eps, tf_eps;
     int lj_lfs;             // O-O LJ with linear force shift at the cutoff
     double rc, uc, dudrc;
-    float quotient_r2;      // above this r^2 every dividend and quotient is finite
+    int quotient_r2;        // above this r^2 every dividend and quotient is finite: the bits
+                            // of an FP32 square, the high word of an FP64 one
 };
 
 // Terms of one pair inside the cutoff: force coefficient (F = s d), real-space energy and
@@ -108,8 +110,9 @@ __device__ __noinline__ RealTerms<T> real_terms_ieee(T r2, T cqq, bool coulomb, 
 template <class T>
 __device__ __forceinline__ RealTerms<T> real_pair(T r2, T cqq, bool coulomb, bool lj,
                                                   const RealArgs& a) {
-    bool fast = static_cast<float>(r2) > a.quotient_r2;
-    if constexpr (sizeof(T) == 8) fast = fast && !low_ones(r2);
+    bool fast;
+    if constexpr (sizeof(T) == 4) fast = __float_as_int(r2) > a.quotient_r2;
+    else fast = __double2hiint(r2) > a.quotient_r2 && !low_ones(r2);
     if (!fast) return real_terms_ieee<T>(r2, cqq, coulomb, lj, &a);
     T r;
     if constexpr (sizeof(T) == 4) r = __fsqrt_rn(r2);
@@ -865,8 +868,12 @@ RealArgs real_args_of(const md_ewald* ew, double alpha, bool mixed) {
     a.dudrc = -(24.0 * ew->epsilon_o * (2.0 * s6 * s6 - s6)) / ew->cutoff;
     // 48 eps (sigma^2 / r^2)^6 and that over r^2 below the largest numbers
     const double top = std::pow(a.sig2, 6.0) * std::max(2.0, 2.0 * a.tf_eps) / (mixed ? 1e37 : 1e307);
-    a.quotient_r2 = static_cast<float>(
-        std::max({1e-15, std::pow(top, 1.0 / 6.0), std::pow(top, 1.0 / 7.0)}));
+    const double line = std::max({1e-15, std::pow(top, 1.0 / 6.0), std::pow(top, 1.0 / 7.0)});
+    const float line32 = static_cast<float>(std::min(line, 3e38));
+    int64_t bits;
+    std::memcpy(&bits, &line, sizeof bits);
+    a.quotient_r2 = static_cast<int>(bits >> 32);
+    if (mixed) std::memcpy(&a.quotient_r2, &line32, sizeof line32);
     return a;
 }
 
