@@ -130,9 +130,9 @@ __device__ __forceinline__ int rdf_bin_of(const RdfArgs& a, double r2) {
 }
 
 // A block takes a cell (of width rMax or a little more): its atoms against those of itself
-// and 13 of its 26 neighbours, so that every pair of cells is met once.  A warp takes 32 candidates of the flattened
-// neighbour ranges at a time, one per lane, skips them if none lies within rMax of the
-// cell's box, and tests them against the cell's atoms (shared-memory broadcasts) in FP32
+// and 13 of its 26 neighbours, so that every pair of cells is met once.  A warp takes 32
+// candidates of the flattened neighbour ranges at a time, one per lane, skips them if none
+// lies within rMax of the cell's box, and tests them against the cell's atoms (shared-memory broadcasts) in FP32
 // units of rMax, widened by 1e-4 (their error is below 1e-6); hits, about one test in
 // eight, are queued and settled 32 at a time with the reference's displacement and bin,
 // so no lane idles through the FP64 part.

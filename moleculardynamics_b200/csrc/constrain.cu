@@ -144,8 +144,9 @@ __device__ __forceinline__ void shift_ends(Mol& r, int i, int j, const double (&
 // of dependent FP64 operations, three constraints one after another, so what counts is the
 // chain: its divisions (126 clocks each, two of the three in the chain) are quotients by
 // shared or precomputed reciprocals (divide() for masses or denominators outside their
-// range), and nothing in a constraint branches: the fold and the update select.  1,029 sites at tolerance 1e-12: 65 us with IEEE
-// divisions and 256-thread blocks, 40 us with quotients, 32 us without branches.
+// range), and nothing in a constraint branches: the fold and the update select.  1,029
+// sites at tolerance 1e-12: 65 us with IEEE divisions and 256-thread blocks, 40 us with
+// quotients, 32 us without branches.
 __device__ int shake_molecule(Mol& r, const Mol& ref, const double m[3], const RigidArgs& a,
                               const Fold3& f3) {
     double b[3][3], two_inv_mass[3];

@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(kRealBlock, MIXED ? 14 : 10)
 k_ewald_real(const double4* __restrict__ pos, const double* __restrict__ q,
              const int64_t* __restrict__ mol, const int* __restrict__ nbr,
              const int* __restrict__ count, int stride, int64_t n, Box3 box,
-             const __grid_constant__ RealArgs a, int mode, double* fxo, double* fyo, double* fzo, double* part, unsigned* ticket,
-             double* out) {
+             const __grid_constant__ RealArgs a, int mode, double* fxo, double* fyo, double* fzo,
+             double* part, unsigned* ticket, double* out) {
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     const int64_t i = t / TPA;
     const int g = static_cast<int>(t % TPA);

@@ -633,7 +633,8 @@ int capture_lj_step_into(md_integrator* it, md_system* sys, md_verlet* v, md_lj*
     md_context* ctx = sys->ctx;
     RunCursor* run = loop ? reinterpret_cast<RunCursor*>(idx) : nullptr;
     if (it->kind == 1 && !run)
-        return fail(MD_ERR_INVALID_ARGUMENT, "a captured Langevin step reads its number from a run's cursor");
+        return fail(MD_ERR_INVALID_ARGUMENT,
+                    "a captured Langevin step reads its number from a run's cursor");
     const int64_t l0 = ctx->launches;
     int rc = MD_OK;
     cudaGraphConditionalHandle h;

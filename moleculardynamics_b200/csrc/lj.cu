@@ -876,8 +876,9 @@ __device__ __noinline__ ExactSums gathered_row_exact(LJArgs a, Box3 box,
 // entry costs some 20 wavefronts a warp instead of 64.  The terms of an entry are formed
 // without a branch on the cutoff (a warp nearly always holds a pair inside it), so entries
 // overlap.  1,048,576-atom liquid, kick included: 606 us with two IEEE divisions a pair,
-// 525 us with the shared reciprocal, 397 us from tiles (two entries side by side, or their
-// loads ahead of the arithmetic of four, spill past 80 registers: 467 to 530 us).
+// 525 us with the shared reciprocal, 429 us from tiles (397 when first measured, where two
+// entries side by side, or their loads ahead of the arithmetic of four, which spill past 80
+// registers, took 467 to 530).
 // Wrapped coordinates and cutoffs below half the box only: a pair near half a box length is
 // then beyond the cutoff whichever way it folds.
 constexpr int kHalo64Cap = 2304;  // slots: three blocks per SM; tiles with more gather
