@@ -44,19 +44,19 @@ def test_replicas_equal_their_solo_runs(md, tpa, trunc):
 
 
 def test_pace(md):
-    """Eight liquids of 32,000 and 70,304 atoms: shifted within 1.18 times truncated (1.14
-    measured)."""
-    times = []
+    """Eight liquids of 32,000 and 70,304 atoms: shifted within 1.2 times truncated (1.14
+    measured), the two in turn."""
+    runs, times = [], ([], [])
     for trunc in (0, 1):
         keep = [replica(md, 20 + 6 * (k % 2), 0.8442, trunc) for k in range(8)]
         b = md.Batch()
         for r in keep:
             b.add(*r)
         b.run(20)
-        t = []
-        for _ in range(7):
+        runs.append((b, keep))
+    for _ in range(9):
+        for (b, _), t in zip(runs, times):
             a = time.perf_counter()
             b.run(40)
             t.append(time.perf_counter() - a)
-        times.append(min(t))
-    assert times[1] < 1.18 * times[0]
+    assert min(times[1]) < 1.2 * min(times[0])
