@@ -2,6 +2,7 @@
 thread an atom, a crowd among sparse cells, blocks that walk the cells, each against the
 oracle's all-pairs histogram, exactly; coordinates several box lengths away and subsets; and
 frames whose time must not depend on the number of cells alone."""
+import ctypes as C
 import time
 
 import numpy as np
@@ -50,6 +51,42 @@ def test_unwrapped_and_subsets(md, box, rmax, first, stride):
     rdf.accumulate(md.System.from_arrays(pos, box), first, stride)
     hist, _ = O.rdf([pos[first::stride]], box, rmax, 100)
     assert np.array_equal(rdf.histogram(), hist)
+
+
+@pytest.mark.parametrize("rmax,bins", [(2.7, 60), (3.5, 3000), (19.0, 100)])
+def test_frames_in_a_captured_block(md, rmax, bins):
+    """A droplet of water: the frames that md_water_rdf_run's graph takes (sparse cells, walked
+    cells, 27 cells) are those of separate calls on the same trajectory."""
+    half = np.radians(0.5 * 109.47)
+    body = np.array([[0, 0, 0], [np.sin(half), 0, np.cos(half)], [-np.sin(half), 0, np.cos(half)]])
+    grid = np.stack(np.meshgrid(*[np.arange(7)] * 3, indexing="ij"), -1).reshape(-1, 3) - 3.0
+    rng = np.random.default_rng(5)
+    turn = np.linalg.qr(rng.normal(size=(len(grid), 3, 3)))[0]
+    pos = (3.1 * grid[:, None] + np.einsum("mij,kj->mki", turn, body)).reshape(-1, 3)
+    m = len(grid)
+    vel = np.repeat(3.0 * rng.normal(size=(m, 3)), 3, axis=0)
+    dof, hist = md.RigidWater.degrees_of_freedom(m, True), []
+    for fused in (True, False):
+        s = md.System.from_arrays(pos, np.full(3, 60.0), vel=vel, mass=np.tile([15.9994, 1.008, 1.008], m),
+                                  charge=np.tile([-0.8476, 0.4238, 0.4238], m), mol=np.arange(3 * m) // 3)
+        rigid = md.RigidWater(1.0, 109.47, settle=True)
+        rigid.constrain_velocities(s)
+        it = md.ConstrainedVelocityVerlet(md.units.femtoseconds(1.0), rigid)
+        ff, rdf = md.SpceForceField(), md.Rdf(rmax, bins)
+        if fused:
+            t = C.c_double()
+            md._check(md.lib().md_water_rdf_run(it.handle, s.handle, ff.handle, rdf.handle, 298.0, dof,
+                                                20, 10, 40, 5, C.byref(t)))
+        else:
+            for _ in range(2):
+                it.run(s, ff, 10)
+                s.rescale_temperature(dof, 298.0)
+                rigid.constrain_velocities(s)
+            for _ in range(8):
+                it.run(s, ff, 5)
+                rdf.accumulate(s, 0, 3)
+        hist.append(rdf.histogram())
+    assert hist[0].sum() > 0 and np.array_equal(hist[0], hist[1])
 
 
 def frame_time(md, pos, box, rmax, bins):
